@@ -25,6 +25,7 @@ NUMERIC_SOURCES = [
     "numeric/factor_kernels.cu",
     "numeric/dense_kernels.cu",
     "numeric/pivot_kernels.cu",
+    "numeric/pivot_panel.cu",
     "numeric/solve_kernels.cu",
     "numeric/solve_dataflow.cu",
     "numeric/pinv_kernels.cu",
@@ -58,7 +59,7 @@ def build_analysis(force: bool = False) -> str:
 
 # Units that restate the reference's scalar in-front arithmetic: no fused multiply-add, so that their
 # values, and the pivots and inertia that depend on exact cancellation, match the reference's
-NO_CONTRACTION = {"factor_kernels.cu", "pivot_kernels.cu"}
+NO_CONTRACTION = {"factor_kernels.cu", "pivot_kernels.cu", "pivot_panel.cu"}
 
 
 def build_numeric(force: bool = False) -> str:

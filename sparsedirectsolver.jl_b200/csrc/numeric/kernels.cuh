@@ -292,6 +292,50 @@ cudaError_t launch_large_pivot_coop(int structure, const LargePivotArgs<T>& a, c
 template <typename T>
 int large_pivot_coop_capacity(int structure);   // co-resident CTAs of the cooperative kernel on this device
 
+// Wide LDLT / LU fronts in 32-column blocks (pivot_panel.cuh): a launch of clusters of C CTAs. Per CTA a list
+// of jobs, the same length within a cluster; a front's group is its leader (one CTA for PANEL_SINGLE, one
+// cluster for PANEL_LEAD) and helper CTAs for the updates.
+constexpr int PP_THREADS = 512;   // rows a leader CTA holds, one per thread
+constexpr int PP_MAXC = 16;       // most CTAs of a cluster
+constexpr int PP_NB = 32;         // columns of a block
+constexpr int PANEL_SINGLE_F = 384;   // tallest front led by one CTA
+enum PanelRole : int32_t { PANEL_IDLE = 0, PANEL_SINGLE, PANEL_LEAD, PANEL_HELP };
+struct PanelJob {
+    int32_t role;
+    int32_t fi;      // index in the launch's front list
+    int32_t rank;    // the CTA's rank in the front's group, leader first
+    int32_t gs;      // CTAs of the group
+};
+struct PanelGroups {
+    const PanelJob* jobs;
+    const int32_t* job_ptr;   // per CTA, grid + 1
+    unsigned int* bar;        // per listed front: group barrier counter, zeroed before the launch
+    int32_t* status;          // nonzero: a bounded group barrier gave up
+    int32_t csize;
+};
+// What the block leaves for T1 and T2, in the front's scratch
+template <typename T>
+struct PanelHdr {
+    int k0, k1, kend, ndisp;      // eliminated columns k0 .. k1 - 1 of the block k0 .. kend - 1
+    int moved, pairs;             // a row changed its place; the block has 2x2 pivots
+    int kind[PP_NB];
+    int rowmap[PP_NB];            // the row (as the block started) that is now row k0 + t
+    int ddst[PP_NB], dsrc[PP_NB]; // rows beyond k1 that hold another row: ddst holds dsrc (a block row)
+    T tdk[PP_NB];
+    T lt[PP_NB][PP_NB];           // lt[s][t]: multiplier of row k0 + t in column k0 + s (s < t)
+};
+
+// doubles of a front's scratch: D (2 w), local order, kinds, the header, the block's solved rows
+__host__ __device__ inline int64_t panel_scratch_len(int f, int w) {
+    return 2 * (int64_t)w + (w + 1) / 2 + (w + 7) / 8 + (int64_t)(sizeof(PanelHdr<double>) / 8 + 1) + (int64_t)PP_NB * f + 4;
+}
+
+template <typename T>
+cudaError_t launch_pivot_panel(int structure, const LargePivotArgs<T>& a, const PanelGroups& g, int grid, cudaStream_t st);
+template <typename T>
+int pivot_panel_clusters(int structure, int csize);   // co-resident clusters of csize CTAs on this device
+cudaError_t prepare_pivot_panel();
+
 // sampled outer product over a CSR pattern (the adjoint of a solve with respect to the values)
 template <typename I>
 struct OuterArgs {

@@ -1,0 +1,875 @@
+// Wide LDLT (Bunch-Kaufman) and LU (threshold) fronts of one-member plans, 32 columns at a time.
+//
+// A front's leader (one CTA, or one cluster whose CTAs share the rows) holds the current block of at most
+// 32 columns in registers, one row per thread, and runs the pivot steps there: per step one exchange of
+// the column's maxima and of the pivot row over distributed shared memory, one cluster barrier, and the
+// rank-1 (rank-2) update of the block's columns in registers. The rest of the front takes the whole block
+// at once: the block's rows are solved against its unit triangle (T1), then every entry takes the block's
+// products one after another (T2), by the leader and the front's helper CTAs.
+//
+// What bounds it: the chain of pivot steps, 2.6 us a column with everything (lap3d 40^3 "S": 14.4 ms over the
+// 5477 columns of the tree's wide fronts, level by level; the cooperative kernel's two group barriers a column
+// took 58.8 ms, and 71.3 against 14.1 ms for the 40^3 LU). The updates run at a few percent of the FP64 rate.
+//
+// Every entry receives the products of ldlt_front_steps / lu_front_steps (front_factor.cuh) in the same
+// order, each product and difference rounded on its own, and every pivot decision sees the same values, so
+// pivots, D and panels are those of the one-CTA kernel bit for bit.
+//
+// A pivot that needs a column outside the block (a Bunch-Kaufman partner, or the search over all diagonals
+// after a rejected choice) is taken only as a block's first one, where the whole front is up to date: a
+// later one ends the block early.
+#pragma once
+#include <stdint.h>
+
+#include "common.cuh"
+#include "front_factor.cuh"
+#include "kernels.cuh"
+#include "pivot.cuh"
+
+namespace sds {
+
+constexpr int PP_WARPS = PP_THREADS / 32;
+constexpr int PP_TR = 128, PP_TC = 64;   // rows and columns of an update tile: 4 x 4 entries per thread
+static_assert(PP_TR * PP_TC == 16 * PP_THREADS, "an update tile holds 16 entries per thread");
+
+template <typename T>
+struct PanelSmem {
+    T prow[PP_NB][PP_NB + 2];                              // the pivot rows as they were eliminated, entry e at
+                                                           // e + 1: entries (1, 2), (3, 4), ... are aligned pairs
+    unsigned hi[2][PP_MAXC * PP_WARPS];                    // per warp: an upper bound of the column's entries
+    unsigned long long lam[PP_MAXC * PP_WARPS];            // per warp: the column's largest entry above row w
+    unsigned long long mx[PP_MAXC * PP_WARPS];             // ... and of all rows (NaN wins)
+    int ridx[PP_MAXC * PP_WARPS];
+    unsigned long long sg[PP_MAXC * PP_WARPS], m1[PP_MAXC * PP_WARPS], m2[PP_MAXC * PP_WARPS];
+    T sc[4];                                               // F[r, r], F[k, r], F[r, k]
+    int plp;
+    int kind[PP_NB];
+    double tdk[PP_NB];
+    int sel[2];
+    int ok;
+    double red[PP_WARPS];
+    int redi[PP_WARPS];
+    PanelHdr<T> hdr;                                       // T1 / T2: the block's header
+    T Rs[PP_NB][PP_TR];
+    T Cs[PP_NB][PP_TC];
+};
+
+// --- keys: |v| as an integer in the order of the values; NaN above infinity -------------------------------------
+__device__ __forceinline__ unsigned long long pp_key(double v) {
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ unsigned long long pp_key(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+template <typename T>
+__device__ __forceinline__ double pp_val(unsigned long long k) {
+    if constexpr (sizeof(T) == 8) return __longlong_as_double((long long)k);
+    else return (double)__uint_as_float((unsigned)k);
+}
+template <typename T>
+__device__ __forceinline__ unsigned long long pp_inf() {
+    return sizeof(T) == 8 ? 0x7ff0000000000000ull : 0x7f800000ull;
+}
+template <typename T>
+__device__ __forceinline__ unsigned long long pp_warp_max(unsigned long long k) {
+    if constexpr (sizeof(T) == 8) {
+        const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
+        return ((unsigned long long)mh << 32) | ml;
+    } else {
+        return __reduce_max_sync(0xffffffffu, (unsigned)k);
+    }
+}
+// the part of a key that one 32-bit reduction takes, and a value no smaller than any with that part (NaN
+// for infinities and NaN)
+__device__ __forceinline__ unsigned pp_hi(double v) { return (unsigned)(pp_key(v) >> 32); }
+__device__ __forceinline__ unsigned pp_hi(float v) { return (unsigned)pp_key(v); }
+template <typename T>
+__device__ __forceinline__ double pp_bound(unsigned h) {
+    if constexpr (sizeof(T) == 8)
+        return __longlong_as_double((long long)((unsigned long long)(h >= 0x7ff00000u ? 0x7ff80000u : h + 1u) << 32));
+    else return h >= 0x7f800000u ? __longlong_as_double(0x7ff8000000000000ll) : (double)__uint_as_float(h);
+}
+// the largest key and, among equal ones, the smallest index; a zero key has no index (-1)
+template <typename T>
+__device__ __forceinline__ unsigned long long pp_warp_argmax(unsigned long long k, int& idx) {
+    const unsigned long long m = pp_warp_max<T>(k);
+    const unsigned i = __reduce_min_sync(0xffffffffu, k == m ? (unsigned)idx : 0xffffffffu);
+    idx = m == 0 ? -1 : (int)i;
+    return m;
+}
+
+// --- a front as its CTAs see it -----------------------------------------------------------------------------------
+template <typename T, bool GEN>
+struct PanelFront {
+    T* P;
+    T* U;
+    int f, w, c0;
+    double* dd;
+    double* ee;
+    int* lp;
+    signed char* kd;
+    PanelHdr<T>* hdr;
+    T* us;             // the block's rows right of it, solved and unscaled: us[t f + c]
+    int C, rank;       // the leader's CTAs and this CTA's rank among them
+    int gs, grank;     // the front's CTAs and this CTA's rank among them
+    unsigned int* bar;
+    unsigned int epoch;
+    int32_t* status;
+    int* ok;           // shared memory: the front's barriers have held so far
+    // F[i, j], i or j < w
+    __device__ T& at(int i, int j) const {
+        if (!GEN || (i >= j && j < w)) return P[i + (int64_t)j * f];
+        return U[j + (int64_t)i * f];
+    }
+    __device__ double get(int i, int j) const { return (double)at(i, j); }
+    __device__ int scan_rows() const { return f; }
+    __device__ double part_max(int, int, int) const { return 0.0; }
+};
+
+// one value into the leader's CTA q's copy of *p
+template <typename V>
+__device__ __forceinline__ void pp_put(V* p, int q, int rank, V v) {
+    if (q == rank) *p = v;
+    else pp_remote_store(p, q, v);
+}
+
+// the leader's CTAs meet; their writes before it (shared, distributed shared and global) are visible after
+template <typename T, bool GEN>
+__device__ __forceinline__ void pp_sync(const PanelFront<T, GEN>& F) {
+    if (F.C > 1) pp_cluster_barrier();
+    else __syncthreads();
+}
+
+// every CTA of the front meets; false once a bounded wait has given up (the same for the whole CTA)
+template <typename T, bool GEN>
+__device__ __forceinline__ bool pp_group_sync(PanelFront<T, GEN>& F) {
+    if (F.gs > F.C) pp_group_barrier(F.bar, F.epoch, F.gs, F.status, F.ok);
+    else pp_sync(F);
+    return *F.ok != 0;
+}
+
+template <typename T>
+__device__ __forceinline__ T pp_pick(const T (&a)[PP_NB], int x) {
+    T v = a[0];
+#pragma unroll
+    for (int e = 1; e < PP_NB; ++e)
+        if (e == x) v = a[e];
+    return v;
+}
+
+// The thread that holds row `pos` writes its registers to prow[t], its warp copies them to every other
+// leader CTA, 16 bytes a lane (a single lane's stores to each CTA in turn took 0.8 of a step's 2.7 us).
+// Whole warps call it.
+template <typename T, bool GEN>
+__device__ __forceinline__ void pp_publish(const PanelFront<T, GEN>& F, PanelSmem<T>& S, const T (&a)[PP_NB], int rp, int pos,
+                                           int t) {
+    const unsigned own = __ballot_sync(0xffffffffu, rp == pos);
+    if (own == 0) return;
+    const int lane = threadIdx.x & 31;
+    T* row = S.prow[t];
+    if (rp == pos) {
+        row[1] = a[0];
+#pragma unroll
+        for (int e = 1; e + 1 < PP_NB; e += 2) pp_store2(row + e + 1, a[e], a[e + 1]);
+        row[PP_NB] = a[PP_NB - 1];
+    }
+    __syncwarp();
+    if (F.C > 1) {
+        constexpr int CH = (PP_NB + 2) / 2;    // aligned pairs of the row
+        const int per = 32 / F.C, q = lane / per;
+        if (q != F.rank)
+            for (int c = lane % per; c < CH; c += per) pp_remote_store2(row + 2 * c, q, row[2 * c], row[2 * c + 1]);
+    }
+}
+
+// The reference's best_1x1 and what follows a rejected choice (bc, br), by one CTA over the whole, up to date
+// front: the acceptable diagonal of largest magnitude, first on ties, tried in that order
+template <typename T, bool GEN>
+__device__ void pp_search(const PanelFront<T, GEN>& F, PanelSmem<T>& S, int k, int pivot, double u, double eps, int bc,
+                          int br, int& c_out, int& r_out) {
+    const CtaTeam tm{(int)threadIdx.x, PP_THREADS, S.red, S.redi};
+    r_out = -1;
+    double la = -1.0;      // the last candidate tried; -1: none yet
+    int lj = -1;
+    while (true) {
+        double a = -1.0;
+        int j = -1;
+        for (int i = k + tm.rank; i < F.w; i += tm.size) {
+            const double x = fabs(F.get(i, i));
+            if (!(x >= eps)) continue;
+            if (lj >= 0 && !(x < la || (x == la && i > lj))) continue;
+            if (x > a) { a = x; j = i; }
+        }
+        tm.reduce_argmax(a, j);
+        __syncthreads();
+        if (j < 0) break;
+        if (threshold_ok(F, j, k, u, a, tm)) { c_out = j; return; }
+        __syncthreads();
+        la = a;
+        lj = j;
+    }
+    if (pivot == PIVOT_DIAGONAL) {
+        const double a0 = fabs(F.get(k, k));
+        double a = -1.0;
+        int j = -1;
+        for (int i = k + 1 + tm.rank; i < F.w; i += tm.size) {
+            const double x = fabs(F.get(i, i));
+            if (x > a) { a = x; j = i; }
+        }
+        tm.reduce_argmax(a, j);
+        const int big = (j >= 0 && a > a0) ? j : k;
+        c_out = fabs(F.get(big, big)) >= eps ? big : k;
+        return;
+    }
+    if (br >= 0 && nonsingular_2x2_w(F, k, br, eps)) r_out = br;
+    c_out = bc;
+}
+
+struct PanelPivot {
+    int pivot, lu_pivot;
+    double u, eps;
+    const int8_t* psign;
+    const int32_t* perm;
+};
+
+// The pivot steps of the block that starts at column k0, by the leader's CTAs. Returns k1, the first column
+// that is left; st[] collects the statistics (every thread holds the same).
+template <typename T, int STRUCT>
+__device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelPivot& pv, int k0, int64_t* st) {
+    constexpr bool GEN = STRUCT == STRUCT_G;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int f = F.f, w = F.w, C = F.C;
+    const int nb = min(PP_NB, w - k0), kend = k0 + nb;
+    // rows k0 .. f - 1 in one contiguous, warp-aligned chunk per CTA
+    const int chunk = ((f - k0 + C - 1) / C + 31) & ~31;
+    const int nw = chunk >> 5, nparts = C * nw;
+    const int orig = tid < chunk && k0 + F.rank * chunk + tid < f ? k0 + F.rank * chunk + tid : -1;
+    int rp = orig;                      // the row's place; a finished row keeps its own (<= k)
+    T a[PP_NB];                         // the row's entries of columns k, k + 1, ... and, behind them, its
+                                        // multipliers: one rotation per eliminated column
+    int mylp = 0;
+    const double alpha = (1.0 + sqrt(17.0)) / 8.0;
+    auto load = [&]() {
+#pragma unroll
+        for (int e = 0; e < PP_NB; ++e) a[e] = (orig >= 0 && e < nb) ? F.at(orig, k0 + e) : T(0);
+        mylp = (orig >= 0 && orig < w) ? F.lp[orig] : 0;
+    };
+    load();
+    if (F.rank == 0 && tid == 0) F.hdr->ndisp = F.hdr->moved = 0;
+    int par = 0, j = 0;
+    while (j < nb) {
+        const int k = k0 + j;
+        // a bound of the column below row k, and row k itself, to every leader CTA
+        if (warp < nw) {
+            const unsigned h = __reduce_max_sync(0xffffffffu, rp > k ? pp_hi(a[0]) : 0u);
+            if (lane < C) pp_put(&S.hi[par][F.rank * nw + warp], lane, F.rank, h);
+            pp_publish(F, S, a, rp, k, j);
+        }
+        pp_sync(F);
+        unsigned h = 0;
+        for (int i = lane; i < nparts; i += 32) h = max(h, S.hi[par][i]);
+        const double bound = pp_bound<T>(__reduce_max_sync(0xffffffffu, h));
+        par ^= 1;
+        const double akk = fabs((double)S.prow[j][1]);
+        // The bound alone accepts most pivots (every test grows with the maxima). Else the exact maxima:
+        // lambda = max over the rows k < i < w with its first row r, mall = max over all rows i > k (NaN wins).
+        bool fast;
+        if (GEN) fast = !pv.lu_pivot || (akk >= pv.u * bound && akk >= pv.u * akk);
+        else if (pv.pivot == PIVOT_NONE) fast = true;
+        else fast = akk >= pv.eps && akk >= pv.u * bound && (pv.pivot == PIVOT_DIAGONAL || akk >= alpha * bound);
+        double lambda = 0.0, mall = 0.0;
+        int r = -1;
+        if (!fast) {
+            if (warp < nw) {
+                const unsigned long long key = rp > k ? pp_key(a[0]) : 0ull;
+                const unsigned long long mkey = pp_warp_max<T>(key);
+                int ri = rp;
+                const unsigned long long lkey =
+                    pp_warp_argmax<T>(rp > k && rp < w && key <= pp_inf<T>() ? key : 0ull, ri);
+                if (lane < C) {
+                    const int at = F.rank * nw + warp;
+                    pp_put(&S.lam[at], lane, F.rank, lkey);
+                    pp_put(&S.mx[at], lane, F.rank, mkey);
+                    pp_put(&S.ridx[at], lane, F.rank, ri);
+                }
+            }
+            pp_sync(F);
+            unsigned long long lk = 0, mk = 0;
+            r = 0x7fffffff;
+            for (int i = lane; i < nparts; i += 32) {
+                const unsigned long long l = S.lam[i], m = S.mx[i];
+                const int ri = S.ridx[i];
+                if (l > lk || (l == lk && l != 0 && ri < r)) { lk = l; r = ri; }
+                if (m > mk) mk = m;
+            }
+            lk = pp_warp_argmax<T>(lk, r);
+            lambda = pp_val<T>(lk);
+            mall = pp_val<T>(pp_warp_max<T>(mk));
+        }
+        int c = k, r2 = -1;
+        if (GEN) {
+            if (!fast && !(akk >= pv.u * jmax(mall, akk)) && r >= 0 && lambda > akk) c = r;
+            if (c != k) {   // row interchange: rows change places, their data stay
+                pp_sync(F);
+                if (rp == k) rp = c;
+                else if (rp == c) rp = k;
+                if (warp < nw) pp_publish(F, S, a, rp, k, j);
+                pp_sync(F);
+            }
+        } else if (!fast) {
+            bool acc;
+            int bc = k, br = -1;
+            if (pv.pivot == PIVOT_DIAGONAL || r < 0 || akk >= alpha * lambda) {
+                acc = akk >= pv.eps && akk >= pv.u * mall;
+            } else {
+                if (r >= kend && j > 0) break;   // the partner's column is not up to date
+                // column r: its maxima, those of column k without row r, and the corner entries
+                T v = T(0);
+                if (rp >= k) v = r < kend ? pp_pick(a, r - k) : F.at(orig, r);
+                if (warp < nw) {
+                    const unsigned long long kv = rp >= k && rp != r ? pp_key(v) : 0ull;
+                    const unsigned long long s1 = pp_warp_max<T>(rp < w ? kv : 0ull);
+                    const unsigned long long s2 = pp_warp_max<T>(rp != k ? kv : 0ull);
+                    const unsigned long long s3 = pp_warp_max<T>(rp > k && rp != r ? pp_key(a[0]) : 0ull);
+                    if (lane < C) {
+                        const int at = F.rank * nw + warp;
+                        pp_put(&S.sg[at], lane, F.rank, s1);
+                        pp_put(&S.m2[at], lane, F.rank, s2);
+                        pp_put(&S.m1[at], lane, F.rank, s3);
+                    }
+                    if (rp == r)
+                        for (int q = 0; q < C; ++q) {
+                            pp_put(&S.sc[0], q, F.rank, v);
+                            pp_put(&S.sc[2], q, F.rank, a[0]);
+                        }
+                    if (rp == k)
+                        for (int q = 0; q < C; ++q) pp_put(&S.sc[1], q, F.rank, v);
+                }
+                pp_sync(F);
+                unsigned long long s1 = 0, s2 = 0, s3 = 0;
+                for (int i = lane; i < nparts; i += 32) {
+                    if (S.sg[i] > s1) s1 = S.sg[i];
+                    if (S.m2[i] > s2) s2 = S.m2[i];
+                    if (S.m1[i] > s3) s3 = S.m1[i];
+                }
+                const double sigma = pp_val<T>(pp_warp_max<T>(s1)), m2 = pp_val<T>(pp_warp_max<T>(s2)),
+                             m1 = pp_val<T>(pp_warp_max<T>(s3));
+                const double fkk = (double)S.prow[j][1], frr = (double)S.sc[0], fkr = (double)S.sc[1],
+                             frk = (double)S.sc[2];
+                if (akk * sigma >= alpha * lambda * lambda) {
+                    acc = akk >= pv.eps && akk >= pv.u * mall;
+                } else if (fabs(frr) >= alpha * sigma) {
+                    bc = r;
+                    acc = fabs(frr) >= pv.eps && fabs(frr) >= pv.u * jmax(m2, fabs(fkr));
+                } else {
+                    br = r;
+                    const double det = fkk * frr - fkr * frk;
+                    const double big = jmax(jmax(fabs(fkk), fabs(frk)), fabs(frr));
+                    acc = det != 0.0 && isfinite(det) && big >= pv.eps;
+                    if (acc) {
+                        const double e11 = fabs(frr / det), e12 = fabs(fkr / det), e21 = fabs(frk / det),
+                                     e22 = fabs(fkk / det);
+                        acc = pv.u * (e11 * m1 + e21 * m2) <= 1.0 && pv.u * (e12 * m1 + e22 * m2) <= 1.0;
+                    }
+                }
+            }
+            c = bc;
+            r2 = br;
+            if (!acc) {
+                if (j > 0) break;                // the search needs the whole front up to date
+                if (F.rank == 0) {
+                    int cs = k, rs = -1;
+                    pp_search(F, S, k, pv.pivot, pv.u, pv.eps, bc, br, cs, rs);
+                    __syncthreads();
+                    if (tid == 0)
+                        for (int q = 0; q < C; ++q) {
+                            pp_put(&S.sel[0], q, 0, cs);
+                            pp_put(&S.sel[1], q, 0, rs);
+                        }
+                }
+                pp_sync(F);
+                c = S.sel[0];
+                r2 = S.sel[1];
+            }
+            const int p = r2 < 0 ? k : k + 1, q = r2 < 0 ? c : r2;
+            if (p != q || r2 >= 0) {
+                pp_sync(F);                      // everyone has read what the exchanges below overwrite
+                if (p != q && q < kend) {        // inside the block: columns in registers, rows by place
+                    if (rp >= k) {
+                        const int y = q - k;
+                        const T vp = p == k ? a[0] : a[1], vq = pp_pick(a, y);
+                        if (p == k) a[0] = vq;
+                        else a[1] = vq;
+#pragma unroll
+                        for (int e = 1; e < PP_NB; ++e)
+                            if (e == y) a[e] = vp;
+                    }
+                    if (rp == p) rp = q;
+                    else if (rp == q) rp = p;
+                } else if (p != q) {             // outside it (j = 0): the interchange in memory
+                    const int gt = F.rank * PP_THREADS + tid, GT = C * PP_THREADS;
+                    for (int i = gt; i < f; i += GT) {
+                        if (i == p || i == q) continue;
+                        const T t = F.at(i, p);
+                        F.at(i, p) = F.at(i, q);
+                        F.at(i, q) = t;
+                    }
+                    for (int i = gt; i < w; i += GT) {
+                        if (i == p || i == q) continue;
+                        const T t = F.at(p, i);
+                        F.at(p, i) = F.at(q, i);
+                        F.at(q, i) = t;
+                    }
+                    if (gt == 0) {
+                        T t = F.at(p, p);
+                        F.at(p, p) = F.at(q, q);
+                        F.at(q, q) = t;
+                        t = F.at(p, q);
+                        F.at(p, q) = F.at(q, p);
+                        F.at(q, p) = t;
+                        const int tl = F.lp[p];
+                        F.lp[p] = F.lp[q];
+                        F.lp[q] = tl;
+                    }
+                    pp_sync(F);
+                    load();
+                }
+                if (warp < nw) {
+                    pp_publish(F, S, a, rp, k, j);
+                    if (r2 >= 0) pp_publish(F, S, a, rp, k + 1, j + 1);
+                }
+                pp_sync(F);
+            }
+        }
+        const bool lead = F.rank == 0 && tid == 0;
+        if (GEN || r2 < 0) {
+            double dk = (double)S.prow[j][1];
+            int kk = KIND_1X1;
+            if (!(fabs(dk) >= pv.eps) || dk == 0.0) {
+                if (dk == 0.0) st[ST_NZERO]++;
+                int lpk = 0;
+                if (!GEN) {   // the column this row is of
+                    if (rp == k)
+                        for (int q = 0; q < C; ++q) pp_put(&S.plp, q, F.rank, mylp);
+                    pp_sync(F);
+                    lpk = S.plp;
+                }
+                const int req = !GEN && pv.psign ? (int)pv.psign[pv.perm[F.c0 + lpk]] : 0;
+                dk = perturb_sign_of(dk, req) * pv.eps;
+                kk = KIND_PERTURBED;
+                st[ST_NPERT]++;
+                if (dk == 0.0 && st[ST_INFO] == 0) st[ST_INFO] = (GEN ? k : lpk) + 1;
+            }
+            if (!GEN) {
+                if (dk > 0) st[ST_NPOS]++;
+                else if (dk < 0) st[ST_NNEG]++;
+            }
+            if (lead) {
+                F.dd[k] = dk;
+                if (!GEN) F.ee[k] = 0.0;
+                F.kd[k] = (signed char)kk;
+            }
+            if (tid == 0) {
+                S.kind[j] = kk;
+                S.tdk[j] = dk;
+            }
+            if (rp > k) {
+                const T l = GEN ? a[0] / T(dk) : T((double)a[0] / dk);
+                const int left = nb - j;   // columns k .. kend - 1
+                const T* row = S.prow[j] + 1;
+#pragma unroll
+                for (int g = 0; g < PP_NB; g += 8) {
+                    T u[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2)
+                        if (g + e + 2 < PP_NB) pp_load2(row + g + e + 1, u[e], u[e + 1]);
+                        else u[e] = row[g + e + 1 < PP_NB ? g + e + 1 : 0], u[e + 1] = T(0);
+                    if (g + 8 < left) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (g + e + 1 < PP_NB) a[g + e] = a[g + e + 1] - l * u[e];
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (g + e + 1 < PP_NB) {
+                                const T t = a[g + e + 1] - l * u[e];
+                                a[g + e] = g + e + 1 < left ? t : a[g + e + 1];
+                            }
+                    }
+                }
+                a[PP_NB - 1] = l;
+            }
+            j += 1;
+        } else {
+            const double fa = (double)S.prow[j][1], fb = (double)S.prow[j + 1][1], fc = (double)S.prow[j + 1][2];
+            const double det = fa * fc - fb * fb;
+            const double e11 = fc / det, e12 = -fb / det, e21 = -fb / det, e22 = fa / det;
+            st[ST_N2X2]++;
+            if (det < 0) { st[ST_NPOS]++; st[ST_NNEG]++; }
+            else if (fa > 0) st[ST_NPOS] += 2;
+            else st[ST_NNEG] += 2;
+            if (lead) {
+                F.dd[k] = fa; F.dd[k + 1] = fc; F.ee[k] = fb; F.ee[k + 1] = 0.0;
+                F.kd[k] = KIND_2X2_FIRST; F.kd[k + 1] = KIND_2X2_SECOND;
+            }
+            if (tid == 0) {
+                S.kind[j] = KIND_2X2_FIRST;
+                S.kind[j + 1] = KIND_2X2_SECOND;
+                S.tdk[j] = S.tdk[j + 1] = 1.0;
+            }
+            if (rp > k + 1) {
+                const double x1 = (double)a[0], x2 = (double)a[1];
+                const T l1 = T(x1 * e11 + x2 * e21), l2 = T(x1 * e12 + x2 * e22);
+                const int left = nb - j;
+#pragma unroll
+                for (int e = 0; e < PP_NB - 2; ++e) {
+                    const T t = a[e + 2] - (l1 * S.prow[j][e + 3] + l2 * S.prow[j + 1][e + 3]);
+                    a[e] = e + 2 < left ? t : a[e + 2];
+                }
+                a[PP_NB - 2] = l1;
+                a[PP_NB - 1] = l2;
+            }
+            j += 2;
+        }
+    }
+    const int nbd = j, k1 = k0 + nbd;
+    // the registers back to the columns' order, then out to the rows' places
+    if (orig >= 0 && rp >= k1) {
+        for (int t = nbd; t < PP_NB; ++t) {
+            const T a0 = a[0];
+#pragma unroll
+            for (int e = 0; e + 1 < PP_NB; ++e) a[e] = a[e + 1];
+            a[PP_NB - 1] = a0;
+        }
+#pragma unroll
+        for (int e = 0; e < PP_NB; ++e)
+            if (e < nb) F.P[rp + (int64_t)(k0 + e) * f] = a[e];
+        if (rp != orig) {
+            const int d = atomicAdd(&F.hdr->ndisp, 1);
+            F.hdr->ddst[d] = rp;
+            F.hdr->dsrc[d] = orig;
+        }
+    } else if (orig >= 0) {
+        F.hdr->rowmap[rp - k0] = orig;
+    }
+    if (orig >= 0 && rp != orig) F.hdr->moved = 1;
+    if (orig >= 0 && rp < w) F.lp[rp] = mylp;
+    if (F.rank == 0) {
+        __syncthreads();   // S.kind and S.tdk of the last step
+        for (int q = tid; q < PP_NB * PP_NB; q += PP_THREADS) {
+            const int t = q % PP_NB, s = q / PP_NB;      // row t, column s
+            T l = T(0);
+            if (s < t && t < nbd) {
+                const int rot = S.kind[t] == KIND_2X2_SECOND ? t - 1 : t;   // the row's rotations when it was taken
+                if (s < rot) l = S.prow[t][1 + PP_NB - rot + s];
+                F.P[(k0 + t) + (int64_t)(k0 + s) * f] = l;
+            }
+            F.hdr->lt[s][t] = l;
+            if (GEN && s > t && s < nb) F.U[(k0 + s) + (int64_t)(k0 + t) * f] = S.prow[t][1 + s - t] / T(S.tdk[t]);
+        }
+        if (tid < nbd) {
+            F.hdr->kind[tid] = S.kind[tid];
+            F.hdr->tdk[tid] = T(S.tdk[tid]);
+        }
+        if (tid == 0) {
+            int pairs = 0;
+            for (int t = 0; !GEN && t < nbd; ++t) pairs |= S.kind[t] == KIND_2X2_FIRST;
+            F.hdr->pairs = pairs;
+            F.hdr->k0 = k0;
+            F.hdr->k1 = k1;
+            F.hdr->kend = kend;
+        }
+    }
+    return k1;
+}
+
+// T1: the block's rows right of the block, solved against its unit triangle (unscaled, into F.us); the rows'
+// interchanges in the columns left of the block
+template <typename T, int STRUCT>
+__device__ void pp_rows(const PanelFront<T, STRUCT == STRUCT_G>& F, const PanelHdr<T>& H) {
+    constexpr bool GEN = STRUCT == STRUCT_G;
+    const int f = F.f, nbd = H.k1 - H.k0;
+    const int lane = threadIdx.x & 31, gt = F.grank * PP_THREADS + threadIdx.x, GT = F.gs * PP_THREADS;
+    const int cfirst = GEN ? H.k1 : H.kend, clast = GEN ? f : F.w;
+    // Four lanes per column, row 4 i + sub in a lane's g[i]: the solve is a chain of nbd broadcasts, 1 us for a
+    // warp, where one lane per column took 3; eight columns a warp, the warps spread over the group's CTAs
+    // (sixteen in one CTA took 16 us).
+    constexpr int NG = PP_NB / 4;
+    const int sub = lane & 3;
+    for (int c0 = cfirst + ((threadIdx.x >> 5) * F.gs + F.grank) * 8; c0 < clast; c0 += F.gs * PP_WARPS * 8) {
+        const int c = c0 + (lane >> 2);
+        const bool live = c < clast;
+        T g[NG];
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            const int t = 4 * i + sub;
+            g[i] = live && t < nbd ? F.at(H.moved ? H.rowmap[t] : H.k0 + t, c) : T(0);
+        }
+        T u0 = T(0);   // the first of a 2x2 pair's two rows
+        for (int s = 0; s < nbd; s += 4) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (s + q >= nbd) break;
+                const T u = __shfl_sync(0xffffffffu, g[0], (lane & ~3) + q);
+                if (live && sub == q) F.us[(int64_t)(s + q) * f + c] = u;
+                const T* l = &H.lt[s + q][s + sub];
+                const int kd = GEN || !H.pairs ? KIND_1X1 : H.kind[s + q];
+                if (kd == KIND_2X2_FIRST) {
+                    u0 = u;
+                } else if (kd == KIND_2X2_SECOND) {
+                    const T* l0 = &H.lt[s + q - 1][s + sub];
+#pragma unroll
+                    for (int i = 0; i < NG; ++i)
+                        if (s + 4 * i < nbd && (i > 0 || sub > q)) g[i] -= l0[4 * i] * u0 + l[4 * i] * u;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < NG; ++i)
+                        if (s + 4 * i < nbd && (i > 0 || sub > q)) g[i] -= l[4 * i] * u;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i + 1 < NG; ++i) g[i] = g[i + 1];
+        }
+    }
+    if (!H.moved) return;
+    for (int c = gt; c < H.k0; c += GT) {
+        T* col = F.P + (int64_t)c * f;
+        T b[2 * PP_NB];
+        for (int t = 0; t < nbd; ++t) b[t] = col[H.rowmap[t]];
+        for (int d = 0; d < H.ndisp; ++d) b[PP_NB + d] = col[H.dsrc[d]];
+        for (int t = 0; t < nbd; ++t) col[H.k0 + t] = b[t];
+        for (int d = 0; d < H.ndisp; ++d) col[H.ddst[d]] = b[PP_NB + d];
+    }
+}
+
+// One update tile: entries (row0 + i, col0 + c) of `C` (leading dimension f), each minus the block's
+// products R[row] Cc[col] in the order of its columns. R and Cc are read at R[row + t rld] and
+// Cc[col + t cld]. Entry (row, col) is live when row >= col + low. src(row, col): where its value comes from.
+template <typename T, int STRUCT, int RI, class SRC>
+__device__ __forceinline__ void pp_tile(PanelSmem<T>& S, const PanelHdr<T>& H, T* Cp, int f, int row0, int col0, int nr,
+                                        int nc, int low, const T* R, int64_t rld, const T* Cc, int64_t cld, SRC src) {
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5, nbd = H.k1 - H.k0;
+    T c[RI][4];
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = tx + 32 * i, cc = 4 * ty + q;
+            c[i][q] = r < nr && cc < nc && row0 + r >= col0 + cc + low ? *src(row0 + r, col0 + cc) : T(0);
+        }
+    constexpr int TR = 32 * RI;
+#pragma unroll
+    for (int x = 0; x < PP_NB * TR / PP_THREADS; ++x) {
+        const int q = tid + x * PP_THREADS, t = q / TR, r = q % TR;
+        S.Rs[t][r] = t < nbd && r < nr ? R[row0 + r + (int64_t)t * rld] : T(0);
+    }
+#pragma unroll
+    for (int x = 0; x < PP_NB * PP_TC / PP_THREADS; ++x) {
+        const int q = tid + x * PP_THREADS, t = q / PP_TC, r = q % PP_TC;
+        S.Cs[t][r] = t < nbd && r < nc ? Cc[col0 + r + (int64_t)t * cld] : T(0);
+    }
+    __syncthreads();
+    if (STRUCT != STRUCT_S || !H.pairs) {
+#pragma unroll 4
+        for (int t = 0; t < PP_NB; ++t) {   // beyond nbd: zeros
+            T ra[RI], ca[4];
+#pragma unroll
+            for (int i = 0; i < RI; ++i) ra[i] = S.Rs[t][tx + 32 * i];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ca[q] = S.Cs[t][4 * ty + q];
+#pragma unroll
+            for (int i = 0; i < RI; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) c[i][q] -= ra[i] * ca[q];
+        }
+    }
+    for (int t = STRUCT != STRUCT_S || !H.pairs ? nbd : 0; t < nbd;) {
+        T ra[RI], ca[4];
+#pragma unroll
+        for (int i = 0; i < RI; ++i) ra[i] = S.Rs[t][tx + 32 * i];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ca[q] = S.Cs[t][4 * ty + q];
+        if (STRUCT == STRUCT_S && H.kind[t] == KIND_2X2_FIRST) {
+            T rb[RI], cb[4];
+#pragma unroll
+            for (int i = 0; i < RI; ++i) rb[i] = S.Rs[t + 1][tx + 32 * i];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) cb[q] = S.Cs[t + 1][4 * ty + q];
+#pragma unroll
+            for (int i = 0; i < RI; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) c[i][q] -= ra[i] * ca[q] + rb[i] * cb[q];
+            t += 2;
+        } else {
+#pragma unroll
+            for (int i = 0; i < RI; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) c[i][q] -= ra[i] * ca[q];
+            t += 1;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = tx + 32 * i, cc = 4 * ty + q;
+            if (r < nr && cc < nc && row0 + r >= col0 + cc + low) Cp[row0 + r + (int64_t)(col0 + cc) * f] = c[i][q];
+        }
+    __syncthreads();
+}
+
+// T2: the block's products into the rest of the front. "S": columns kend .. w - 1, rows k1 .. f - 1. "G": the
+// same columns (k1 .. w - 1) on and below the diagonal in the L panel, and rows k1 .. w - 1 right of the
+// diagonal in the U^T panel (there a tile's rows are the matrix' columns).
+template <typename T, int STRUCT, int RI>
+__device__ void pp_update_tiles(const PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelHdr<T>& H) {
+    constexpr bool GEN = STRUCT == STRUCT_G;
+    const int f = F.f, w = F.w, k1 = H.k1, cf = GEN ? k1 : H.kend;
+    constexpr int TR = 32 * RI;
+    const int ntr = (f - k1 + TR - 1) / TR, ntc = (w - cf + PP_TC - 1) / PP_TC;
+    const int nt = ntr * ntc, all = GEN ? 2 * nt : nt;
+    const T* Lb = F.P + (int64_t)H.k0 * f;
+    auto row_of = [&](int i) {
+        int s = i;
+        for (int d = 0; d < H.ndisp; ++d)
+            if (H.ddst[d] == i) s = H.dsrc[d];
+        return s;
+    };
+    for (int q = F.grank; q < all; q += F.gs) {
+        const int qq = q < nt ? q : q - nt;
+        const int row0 = k1 + (qq % ntr) * TR, col0 = cf + (qq / ntr) * PP_TC;
+        const int nr = min(TR, f - row0), nc = min(PP_TC, w - col0);
+        if (GEN && row0 + nr - 1 < col0) continue;   // above the diagonal
+        if (q < nt) {
+            pp_tile<T, STRUCT, RI>(S, H, F.P, f, row0, col0, nr, nc, GEN ? 0 : -(1 << 29), Lb, f, F.us, f,
+                               [&](int i, int c) -> const T* {
+                                   const int s = row_of(i);
+                                   return s == i ? F.P + i + (int64_t)c * f : &F.at(s, c);
+                               });
+        } else if constexpr (GEN) {
+            pp_tile<T, STRUCT, RI>(S, H, F.U, f, row0, col0, nr, nc, 1, F.us, f, Lb, f,
+                               [&](int c, int i) -> const T* { return F.U + c + (int64_t)row_of(i) * f; });
+        }
+    }
+}
+
+template <typename T, int STRUCT>
+__device__ void pp_update(const PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelHdr<T>& H) {
+    const int cf = STRUCT == STRUCT_G ? H.k1 : H.kend;
+    if (cf >= F.w) return;
+    // 128-row tiles while every CTA has two of them, 64-row tiles below that: half the time of the last round
+    const int nt = ((F.f - H.k1 + PP_TR - 1) / PP_TR) * ((F.w - cf + PP_TC - 1) / PP_TC);
+    if (nt >= 2 * F.gs) pp_update_tiles<T, STRUCT, 4>(F, S, H);
+    else pp_update_tiles<T, STRUCT, 2>(F, S, H);
+}
+
+// "G": the block's rows, scaled, into the U^T panel (after T2: its tiles may read the rows' old values)
+template <typename T>
+__device__ void pp_urows(const PanelFront<T, true>& F, const PanelHdr<T>& H, int part, int nparts) {
+    const int nbd = H.k1 - H.k0, n = F.f - H.k1;
+    const int64_t gt = (int64_t)part * PP_THREADS + threadIdx.x, GT = (int64_t)nparts * PP_THREADS;
+    for (int64_t q = gt; q < (int64_t)n * nbd; q += GT) {
+        const int t = (int)(q / n), c = H.k1 + (int)(q % n);
+        F.U[c + (int64_t)(H.k0 + t) * F.f] = F.us[(int64_t)t * F.f + c] / H.tdk[t];
+    }
+}
+
+// One front, by every CTA of its group
+template <typename T, int STRUCT>
+__device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelSmem<T>& S, int C, unsigned int* bar,
+                         int32_t* status) {
+    constexpr bool GEN = STRUCT == STRUCT_G;
+    const int s = A.list[job.fi];
+    const DFront fd = A.fronts[s];
+    PanelFront<T, GEN> F;
+    F.P = A.factor + fd.panel;
+    F.U = GEN ? A.ufactor + fd.panel : nullptr;
+    F.f = fd.f;
+    F.w = fd.w;
+    F.c0 = fd.c0;
+    const int f = fd.f, w = fd.w;
+    double* scr = A.scratch + A.scr_off[job.fi];
+    F.dd = scr;
+    F.ee = scr + w;
+    F.lp = reinterpret_cast<int*>(F.ee + w);
+    F.kd = reinterpret_cast<signed char*>(F.ee + w + (w + 1) / 2);
+    double* h = F.ee + w + (w + 1) / 2 + (w + 7) / 8;
+    F.hdr = reinterpret_cast<PanelHdr<T>*>(h);
+    F.us = reinterpret_cast<T*>(h + sizeof(PanelHdr<double>) / 8 + 1);
+    F.C = job.role == PANEL_SINGLE ? 1 : C;
+    F.rank = job.rank < F.C ? job.rank : 0;
+    F.gs = job.gs;
+    F.grank = job.rank;
+    F.bar = bar + job.fi;
+    F.epoch = 0;
+    F.status = status;
+    F.ok = &S.ok;
+    if (threadIdx.x == 0) S.ok = 1;
+    __syncthreads();
+    const bool leads = job.rank < F.C;
+    const int tid = threadIdx.x, gt = F.grank * PP_THREADS + tid, GT = F.gs * PP_THREADS;
+    const PanelPivot pv{A.pivot, A.lu_pivot, A.u, A.eps, A.psign, A.perm};
+    if (STRUCT == STRUCT_S)
+        for (int64_t q = gt; q < (int64_t)w * w; q += GT) {
+            const int i = (int)(q % w), j = (int)(q / w);
+            if (i > j) F.P[j + (int64_t)i * f] = F.P[i + (int64_t)j * f];
+        }
+    for (int q = gt; q < w; q += GT) F.lp[q] = q;
+    bool ok = pp_group_sync(F);
+    int64_t st[NSTAT] = {0, 0, 0, 0, 0, 0};
+    PanelHdr<T>& H = S.hdr;
+    // A barrier that gave up (a status word, no fault): helpers leave, the leader's CTAs go through the
+    // blocks together without the shared phases, so that they still meet at every cluster barrier
+    for (int k = 0, first = 1; k < w; first = 0) {
+        if constexpr (GEN) {   // the previous block's rows: the helpers while the leader factors, or everyone
+            const int helpers = F.gs - F.C;
+            if (!first && ok && helpers == 0) pp_urows<T>(F, H, F.grank, F.gs);
+            else if (!first && ok && !leads) pp_urows<T>(F, H, F.grank - F.C, helpers);
+        }
+        int k1 = 0;
+        if (leads) k1 = pp_block<T, STRUCT>(F, S, pv, k, st);
+        if (ok) ok = pp_group_sync(F);
+        if (!ok && !leads) return;
+        if (ok) {
+            const int* src = reinterpret_cast<const int*>(F.hdr);
+            int* dst = reinterpret_cast<int*>(&H);
+            for (int q = tid; q < (int)(sizeof(PanelHdr<T>) / 4); q += PP_THREADS) dst[q] = src[q];
+            __syncthreads();
+            k1 = H.k1;
+            pp_rows<T, STRUCT>(F, H);
+            ok = pp_group_sync(F);
+            if (!ok && !leads) return;
+        }
+        k = k1;
+        if (k < w && ok) {
+            pp_update<T, STRUCT>(F, S, H);
+            ok = pp_group_sync(F);
+            if (!ok && !leads) return;
+        }
+    }
+    if (!ok) return;
+    if constexpr (GEN) pp_urows<T>(F, H, F.grank, F.gs);
+    for (int64_t q = gt; q < (int64_t)w * w; q += GT) {
+        const int i = (int)(q % w), j = (int)(q / w);
+        if (i == j) {
+            F.P[i + (int64_t)j * f] = T(1);
+            if (GEN) F.U[i + (int64_t)j * f] = T(1);
+        } else if (i < j && !GEN) {
+            F.P[i + (int64_t)j * f] = T(0);
+        }
+    }
+    const int64_t n = A.n;
+    for (int q = gt; q < w; q += GT) {
+        const int64_t g = fd.c0 + q;
+        A.piv[g] = fd.c0 + F.lp[q] + 1;
+        A.kind[g] = F.kd[q];
+        A.d[g] = F.dd[q];
+        A.d[n + g] = STRUCT == STRUCT_S ? F.ee[q] : 0.0;
+    }
+    if (F.grank == 0 && tid == 0) {
+        int64_t* So = A.stats + (int64_t)s * NSTAT;
+        for (int q = 0; q < NSTAT; ++q) So[q] = st[q];
+        A.finfo[s] = (int32_t)st[ST_INFO];
+    }
+}
+
+}  // namespace sds

@@ -138,6 +138,79 @@ struct Arena {
     }
 };
 
+// Jobs of one level's wide LDLT / LU fronts for the panel kernel (pivot_panel.cuh) on `ncl` clusters of C
+// CTAs. A front of at most PANEL_SINGLE_F rows takes one CTA: its steps then meet at a CTA barrier instead
+// of a cluster barrier, and the level's small fronts run side by side. Every other front is led by a
+// cluster; clusters that are left over help with the updates of the fronts with the most of them. More
+// fronts than CTAs (clusters) queue up, the largest first on the least loaded one.
+std::vector<std::vector<PanelJob>> panel_jobs(const std::vector<std::pair<int, int>>& fw, int C, int ncl, bool gen) {
+    struct Item { int i; double work; };
+    std::vector<Item> cl, sg;
+    for (int i = 0; i < (int)fw.size(); ++i) {
+        const double f = fw[i].first, w = fw[i].second;
+        // a step's fixed cost (about 1200 row updates) and the updates
+        const Item it{i, w * (1200.0 + f) + f * w * w / 64.0};
+        (fw[i].first <= PANEL_SINGLE_F ? sg : cl).push_back(it);
+    }
+    auto desc = [](const Item& a, const Item& b) { return a.work > b.work; };
+    std::stable_sort(cl.begin(), cl.end(), desc);
+    std::stable_sort(sg.begin(), sg.end(), desc);
+    const int nlead = std::min((int)cl.size(), ncl);
+    int nsc = std::min(((int)sg.size() + C - 1) / C, ncl - nlead);
+    int spare = ncl - nlead - nsc;
+    std::vector<std::vector<PanelJob>> jobs((size_t)(nlead + nsc) * C);
+    std::vector<double> load(nlead, 0.0);
+    std::vector<int> lead_of(cl.size(), 0), first(nlead, -1);
+    for (size_t q = 0; q < cl.size(); ++q) {
+        const int c = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        lead_of[q] = c;
+        load[c] += cl[q].work;
+        if (first[c] < 0) first[c] = (int)q;
+        for (int r = 0; r < C; ++r) jobs[c * C + r].push_back({PANEL_LEAD, cl[q].i, r, C});
+    }
+    // helpers: one cluster at a time to the front whose update tiles per CTA are the most
+    std::vector<int> helpers(nlead, 0);
+    auto tiles = [&](int c) {
+        const int f = fw[cl[first[c]].i].first, w = fw[cl[first[c]].i].second;
+        return (double)((f - 32 + 127) / 128) * ((std::max(w - 32, 0) + 63) / 64) * (gen ? 1.2 : 1.0);
+    };
+    for (; spare > 0; --spare) {
+        int best = -1;
+        double most = 1.0;
+        for (int c = 0; c < nlead; ++c) {
+            const double t = tiles(c) / ((1 + helpers[c]) * C);
+            if (t > most) { most = t; best = c; }
+        }
+        if (best < 0) break;
+        helpers[best]++;
+    }
+    for (int c = 0; c < nlead; ++c) {
+        const int gs = (1 + helpers[c]) * C;
+        for (int r = 0; r < C; ++r) jobs[c * C + r][0].gs = gs;
+        for (int h = 0; h < helpers[c]; ++h)
+            for (int r = 0; r < C; ++r) {
+                jobs.push_back({});
+                jobs.back().push_back({PANEL_HELP, cl[first[c]].i, (1 + h) * C + r, gs});
+            }
+    }
+    // the small fronts: on clusters of their own, or behind the led fronts when there are none
+    const int s0 = nsc > 0 ? nlead * C : 0, sn = (nsc > 0 ? nsc : nlead) * C;
+    std::vector<double> sload(sn, 0.0);
+    for (int q = 0; nsc == 0 && q < sn; ++q) sload[q] = load[q / C];
+    // led fronts first in every list: a cluster's CTAs run the same number of jobs
+    for (const Item& it : sg) {
+        const int c = (int)(std::min_element(sload.begin(), sload.end()) - sload.begin());
+        sload[c] += it.work;
+        jobs[s0 + c].push_back({PANEL_SINGLE, it.i, 0, 1});
+    }
+    for (size_t b = 0; b < jobs.size(); b += C) {
+        size_t len = 0;
+        for (int r = 0; r < C; ++r) len = std::max(len, jobs[b + r].size());
+        for (int r = 0; r < C; ++r) jobs[b + r].resize(len, PanelJob{PANEL_IDLE, 0, 0, 1});
+    }
+    return jobs;
+}
+
 }  // namespace
 
 Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts, cudaStream_t st) {
@@ -849,7 +922,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                     const DFront& F = P->fronts[s];
                     lists.push_back(s);
                     scr_off.push_back(so);
-                    so += pivot_scratch_len(F.f, F.w);
+                    so += std::max(pivot_scratch_len(F.f, F.w), panel_scratch_len(F.f, F.w));
                 }
                 P->scr_len = std::max(P->scr_len, so);
                 P->prog.push_back(pl);
@@ -1475,12 +1548,44 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         // cooperative pivot launches (single-member plans): a group of co-resident CTAs per wide front,
         // sized by the front's update work f w^2, at least one CTA and at most the update items of its
         // first step (row chunks x column groups; twice that for the U^T part of "G")
+        std::vector<PanelJob> pjobs;
+        std::vector<int32_t> pjob_ptr;
         std::vector<int32_t> coop_first;
-        if (P->nbatch == 1) {
+        if (P->nbatch == 1 && P->structure != STRUCT_SPD) {
+            if (prepare_pivot_panel() != cudaSuccess)
+                throw BuildError(SDSB200_CUDA_ERROR, "panel kernel attribute setup failed");
             const int cap = P->elsize == 8 ? large_pivot_coop_capacity<double>(P->structure)
                                            : large_pivot_coop_capacity<float>(P->structure);
+            int ncl[2] = {-1, -1};   // co-resident clusters of 8 and of 16 CTAs
             for (ProgLaunch& L : P->prog) {
-                if (L.kind != L_PIVOT_FRONT || L.count <= 0 || 2 * L.count > cap) continue;
+                if (L.kind != L_PIVOT_FRONT || L.count <= 0) continue;
+                // the panel kernel while a cluster holds every row, one per thread; the cooperative kernel
+                // beyond (8192 rows)
+                std::vector<std::pair<int, int>> fw;
+                int fmax = 0;
+                for (int i = 0; i < L.count; ++i) {
+                    const DFront& F = P->fronts[lists[L.list + i]];
+                    fw.push_back({F.f, F.w});
+                    fmax = std::max(fmax, F.f);
+                }
+                const int big = fmax > 8 * PP_THREADS, C = big ? 16 : 8;
+                if (ncl[big] < 0)
+                    ncl[big] = P->elsize == 8 ? pivot_panel_clusters<double>(P->structure, C)
+                                              : pivot_panel_clusters<float>(P->structure, C);
+                if (fmax <= C * PP_THREADS && ncl[big] > 0) {
+                    const auto jobs = panel_jobs(fw, C, ncl[big], gen);
+                    L.panel = (int32_t)pjob_ptr.size();
+                    L.panel_csize = C;
+                    L.coop_grid = (int32_t)jobs.size();
+                    for (const auto& v : jobs) {
+                        pjob_ptr.push_back((int32_t)pjobs.size());
+                        pjobs.insert(pjobs.end(), v.begin(), v.end());
+                    }
+                    pjob_ptr.push_back((int32_t)pjobs.size());
+                    P->coop_bar_len = std::max(P->coop_bar_len, L.count);
+                    continue;
+                }
+                if (2 * L.count > cap) continue;
                 double total = 0;
                 for (int i = 0; i < L.count; ++i) {
                     const DFront& F = P->fronts[lists[L.list + i]];
@@ -1504,6 +1609,8 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
             }
         }
         P->d_coop_first = upload(P, coop_first, st);
+        P->d_panel_jobs = upload(P, pjobs, st);
+        P->d_panel_ptr = upload(P, pjob_ptr, st);
         if (P->coop_bar_len) P->d_coop_bar = dalloc<unsigned int>(P, P->coop_bar_len);
         P->maps.ea = upload(P, ea, st);
         P->maps.eacol = upload(P, eacol, st);

@@ -28,7 +28,9 @@ struct ProgLaunch {
     double flops;      // algorithmic flops of the launch (reference convention for the fronts)
     double bytes;      // algorithmic device-memory bytes of the launch
     int32_t coop = -1;      // pivot: offset of the group prefix in coop_first (-1: one CTA per front)
-    int32_t coop_grid = 0;  // pivot: CTAs of the cooperative launch
+    int32_t coop_grid = 0;  // pivot: CTAs of the cooperative or panel launch
+    int32_t panel = -1;     // pivot: the panel kernel's job starts, in panel_ptr (-1: another kernel)
+    int32_t panel_csize = 0;
     int32_t exact = 0;      // gemm: the contribution-block update of an LDLT / LU front, which the FP64
                             // form sums in the oracle's order (1: LDLT, 2: LU)
     int32_t side = 0;       // runs on the plan's side stream (the solve's inverses, off the factorization's
@@ -94,6 +96,8 @@ struct Plan {
     int64_t* d_scr_off = nullptr;
     CholStepTask* d_steptasks = nullptr; // tasks of the large-Cholesky step launches
     int32_t* d_coop_first = nullptr;   // group prefixes of the cooperative pivot launches
+    PanelJob* d_panel_jobs = nullptr;  // the panel kernel's jobs and their starts per CTA
+    int32_t* d_panel_ptr = nullptr;
     unsigned int* d_coop_bar = nullptr; // their group barrier counters
     int32_t coop_bar_len = 0;
     int64_t* d_woff = nullptr;
