@@ -11,33 +11,77 @@
 
 namespace sds {
 
+// addresses of p and of the mbarrier in the cluster's CTA q
+__device__ __forceinline__ void pp_remote(const void* p, int q, unsigned& ra) {
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(q));
+}
+// asynchronous stores into CTA q's shared memory; their bytes count into its mbarrier
 template <typename V>
-__device__ __forceinline__ void pp_remote_store(V* p, int q, V v) {
-    unsigned la = (unsigned)__cvta_generic_to_shared(p), ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(q));
+__device__ __forceinline__ void pp_x_store(V* p, int q, V v, unsigned long long* mbar) {
+    unsigned ra, rm;
+    pp_remote(p, q, ra);
+    pp_remote(mbar, q, rm);
     if constexpr (sizeof(V) == 8) {
         unsigned long long b;
         memcpy(&b, &v, 8);
-        asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(ra), "l"(b) : "memory");
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(ra), "l"(b), "r"(rm)
+                     : "memory");
     } else {
         static_assert(sizeof(V) == 4, "4 or 8 bytes");
         unsigned b;
         memcpy(&b, &v, 4);
-        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(ra), "r"(b) : "memory");
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(ra), "r"(b), "r"(rm)
+                     : "memory");
     }
 }
+__device__ __forceinline__ void pp_x_store2(double* p, int q, double x, double y, unsigned long long* mbar) {
+    unsigned ra, rm;
+    pp_remote(p, q, ra);
+    pp_remote(mbar, q, rm);
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(ra), "d"(x), "d"(y),
+                 "r"(rm)
+                 : "memory");
+}
+__device__ __forceinline__ void pp_x_store2(float* p, int q, float x, float y, unsigned long long* mbar) {
+    unsigned ra, rm;
+    pp_remote(p, q, ra);
+    pp_remote(mbar, q, rm);
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(ra), "f"(x), "f"(y),
+                 "r"(rm)
+                 : "memory");
+}
+__device__ __forceinline__ void pp_x_arm(unsigned long long* mbar, int bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(mbar)),
+                 "r"(bytes)
+                 : "memory");
+}
+// a wait of some seconds at most, then the status word (which later waits do not outlast)
+__device__ __forceinline__ void pp_x_wait(unsigned long long* mbar, int parity, int32_t* status) {
+    const unsigned m = (unsigned)__cvta_generic_to_shared(mbar);
+    for (unsigned spins = 0;; ++spins) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(m), "r"(parity)
+            : "memory");
+        if (done) return;
+        if ((spins & 1023) == 1023 && *(volatile int32_t*)status != 0) return;
+        if (spins > (1u << 24)) {
+            atomicExch(status, 1);
+            return;
+        }
+    }
+}
+__device__ __forceinline__ void pp_x_init(unsigned long long* mbar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(mbar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+// the first n threads of the CTA
+__device__ __forceinline__ void pp_warps_barrier(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
 
-// two values at an even (pair-aligned) place
-__device__ __forceinline__ void pp_remote_store2(double* p, int q, double x, double y) {
-    unsigned la = (unsigned)__cvta_generic_to_shared(p), ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(q));
-    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(ra), "d"(x), "d"(y) : "memory");
-}
-__device__ __forceinline__ void pp_remote_store2(float* p, int q, float x, float y) {
-    unsigned la = (unsigned)__cvta_generic_to_shared(p), ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(q));
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ra), "f"(x), "f"(y) : "memory");
-}
 __device__ __forceinline__ void pp_store2(double* p, double x, double y) { *reinterpret_cast<double2*>(p) = make_double2(x, y); }
 __device__ __forceinline__ void pp_store2(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
 __device__ __forceinline__ void pp_load2(const double* p, double& x, double& y) {
@@ -93,9 +137,15 @@ template <typename T, int STRUCT>
 __global__ void __launch_bounds__(PP_THREADS, 1) pivot_panel_kernel(LargePivotArgs<T> A, PanelGroups G) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PanelSmem<T>& S = *reinterpret_cast<PanelSmem<T>*>(smem_raw);
+    if (threadIdx.x == 0) {
+        pp_x_init(&S.mbar[0]);
+        pp_x_init(&S.mbar[1]);
+    }
+    pp_cluster_barrier();
+    unsigned xn = 0;
     for (int q = G.job_ptr[blockIdx.x]; q < G.job_ptr[blockIdx.x + 1]; ++q) {
         const PanelJob job = G.jobs[q];
-        if (job.role != PANEL_IDLE) pp_front<T, STRUCT>(A, job, S, G.csize, G.bar, G.status);
+        if (job.role != PANEL_IDLE) pp_front<T, STRUCT>(A, job, S, G.csize, G.bar, G.status, xn);
         // the cluster's CTAs start their next job, or leave, together: none writes into another's shared
         // memory before or after its front
         pp_cluster_barrier();

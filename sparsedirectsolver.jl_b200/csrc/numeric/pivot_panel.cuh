@@ -7,10 +7,6 @@
 // at once: the block's rows are solved against its unit triangle (T1), then every entry takes the block's
 // products one after another (T2), by the leader and the front's helper CTAs.
 //
-// What bounds it: the chain of pivot steps, 2.6 us a column with everything (lap3d 40^3 "S": 14.4 ms over the
-// 5477 columns of the tree's wide fronts, level by level; the cooperative kernel's two group barriers a column
-// took 58.8 ms, and 71.3 against 14.1 ms for the 40^3 LU). The updates run at a few percent of the FP64 rate.
-//
 // Every entry receives the products of ldlt_front_steps / lu_front_steps (front_factor.cuh) in the same
 // order, each product and difference rounded on its own, and every pivot decision sees the same values, so
 // pivots, D and panels are those of the one-CTA kernel bit for bit.
@@ -36,22 +32,27 @@ template <typename T>
 struct PanelSmem {
     T prow[PP_NB][PP_NB + 2];                              // the pivot rows as they were eliminated, entry e at
                                                            // e + 1: entries (1, 2), (3, 4), ... are aligned pairs
+    unsigned long long mbar[2];                            // the leader's exchanges, by turns
     unsigned hi[2][PP_MAXC * PP_WARPS];                    // per warp: an upper bound of the column's entries
     unsigned long long lam[PP_MAXC * PP_WARPS];            // per warp: the column's largest entry above row w
     unsigned long long mx[PP_MAXC * PP_WARPS];             // ... and of all rows (NaN wins)
     int ridx[PP_MAXC * PP_WARPS];
     unsigned long long sg[PP_MAXC * PP_WARPS], m1[PP_MAXC * PP_WARPS], m2[PP_MAXC * PP_WARPS];
     T sc[4];                                               // F[r, r], F[k, r], F[r, k]
-    int plp;
+    int plp, nbd, ok;
+    int sel[2];
     int kind[PP_NB];
     double tdk[PP_NB];
-    int sel[2];
-    int ok;
     double red[PP_WARPS];
     int redi[PP_WARPS];
     PanelHdr<T> hdr;                                       // T1 / T2: the block's header
-    T Rs[PP_NB][PP_TR];
-    T Cs[PP_NB][PP_TC];
+    union {
+        T L[PP_NB][PP_THREADS];                            // the block: the rows' multipliers
+        struct {
+            T Rs[PP_NB][PP_TR];                            // T2: the operands of a tile
+            T Cs[PP_NB][PP_TC];
+        };
+    };
 };
 
 // --- keys: |v| as an integer in the order of the values; NaN above infinity -------------------------------------
@@ -111,6 +112,7 @@ struct PanelFront {
     T* us;             // the block's rows right of it, solved and unscaled: us[t f + c]
     int C, rank;       // the leader's CTAs and this CTA's rank among them
     int gs, grank;     // the front's CTAs and this CTA's rank among them
+    unsigned xn;       // exchanges of the leader's CTAs so far (the same in each)
     unsigned int* bar;
     unsigned int epoch;
     int32_t* status;
@@ -124,13 +126,6 @@ struct PanelFront {
     __device__ int scan_rows() const { return f; }
     __device__ double part_max(int, int, int) const { return 0.0; }
 };
-
-// one value into the leader's CTA q's copy of *p
-template <typename V>
-__device__ __forceinline__ void pp_put(V* p, int q, int rank, V v) {
-    if (q == rank) *p = v;
-    else pp_remote_store(p, q, v);
-}
 
 // the leader's CTAs meet; their writes before it (shared, distributed shared and global) are visible after
 template <typename T, bool GEN>
@@ -156,37 +151,111 @@ __device__ __forceinline__ T pp_pick(const T (&a)[PP_NB], int x) {
     return v;
 }
 
-// The thread that holds row `pos` writes its registers to prow[t], its warp copies them to every other
-// leader CTA, 16 bytes a lane (a single lane's stores to each CTA in turn took 0.8 of a step's 2.7 us).
-// Whole warps call it.
+// --- exchanges of the leader's CTAs ---------------------------------------------------------------------------------
+// Every leader CTA sends what the others need with asynchronous stores that count into the receiver's
+// mbarrier, and waits for its own: 0.2 us for maxima and pivot row where stores and a cluster barrier took 0.7.
+// Two mbarriers take turns: a CTA sends for the turn after next only when every CTA has finished this one.
+// Only the warps that hold rows take part. One CTA alone meets at a barrier of those warps instead.
 template <typename T, bool GEN>
-__device__ __forceinline__ void pp_publish(const PanelFront<T, GEN>& F, PanelSmem<T>& S, const T (&a)[PP_NB], int rp, int pos,
-                                           int t) {
-    const unsigned own = __ballot_sync(0xffffffffu, rp == pos);
-    if (own == 0) return;
-    const int lane = threadIdx.x & 31;
-    T* row = S.prow[t];
-    if (rp == pos) {
-        row[1] = a[0];
+struct PanelX {
+    PanelFront<T, GEN>& F;
+    PanelSmem<T>& S;
+    int nw, b;
+    __device__ PanelX(PanelFront<T, GEN>& F_, PanelSmem<T>& S_, int nw_) : F(F_), S(S_), nw(nw_), b(0) {}
+    // opens the next exchange, of `bytes` bytes into each CTA
+    __device__ __forceinline__ void open(int bytes) {
+        b = F.xn & 1;
+        if (F.C > 1 && threadIdx.x == 0) pp_x_arm(&S.mbar[b], bytes);
+    }
+    template <typename V>
+    __device__ __forceinline__ void put(V* p, int q, V v) const {   // into CTA q's copy of *p
+        if (F.C > 1) pp_x_store(p, q, v, &S.mbar[b]);
+        else *p = v;
+    }
+    __device__ __forceinline__ void close() {
+        if (F.C > 1) pp_x_wait(&S.mbar[b], (F.xn >> 1) & 1, F.status);
+        else pp_warps_barrier(nw * 32);
+        F.xn++;
+    }
+    // the warps meet: what they read before may be overwritten after, and (fence) what they wrote to global
+    // memory is visible
+    __device__ __forceinline__ void meet(bool fence = false) {
+        if (fence) __threadfence();
+        __syncwarp();
+        if (fence) __threadfence();
+        if (F.C > 1) {
+            open(F.C * nw * 4);
+            const int lane = threadIdx.x & 31;
+            if (lane < F.C) put(&S.hi[b][F.rank * nw + (threadIdx.x >> 5)], lane, 0u);
+            close();
+        } else {
+            pp_warps_barrier(nw * 32);
+        }
+        if (fence) __threadfence();
+    }
+    // bytes of a pivot row with `left` live entries, as whole pairs
+    __device__ static int row_bytes(int left) { return (left + 2) / 2 * 2 * (int)sizeof(T); }
+    // The thread that holds row `pos` writes its `left` live entries to prow[t], and its warp sends them to
+    // every CTA, a pair per store. Whole warps call it, inside an exchange.
+    __device__ __forceinline__ void row(const T (&a)[PP_NB], int rp, int pos, int t, int left) const {
+        if (__ballot_sync(0xffffffffu, rp == pos) == 0) return;
+        T* row = S.prow[t];
+        if (rp == pos) {
+            row[1] = a[0];
 #pragma unroll
-        for (int e = 1; e + 1 < PP_NB; e += 2) pp_store2(row + e + 1, a[e], a[e + 1]);
-        row[PP_NB] = a[PP_NB - 1];
+            for (int g = 0; g < PP_NB; g += 8)
+                if (g + 1 < left) {
+#pragma unroll
+                    for (int e = g + 1; e < g + 9 && e + 1 < PP_NB; e += 2) pp_store2(row + e + 1, a[e], a[e + 1]);
+                }
+            row[PP_NB] = a[PP_NB - 1];
+        }
+        __syncwarp();
+        if (F.C > 1) {
+            const int lane = threadIdx.x & 31, per = 32 / F.C, q = lane / per, ch = (left + 2) / 2;
+            for (int c = lane % per; c < ch; c += per) pp_x_store2(row + 2 * c, q, row[2 * c], row[2 * c + 1], &S.mbar[b]);
+        }
     }
-    __syncwarp();
-    if (F.C > 1) {
-        constexpr int CH = (PP_NB + 2) / 2;    // aligned pairs of the row
-        const int per = 32 / F.C, q = lane / per;
-        if (q != F.rank)
-            for (int c = lane % per; c < CH; c += per) pp_remote_store2(row + 2 * c, q, row[2 * c], row[2 * c + 1]);
+};
+
+// the warps of a CTA that hold rows, as a team (pivot.cuh)
+struct PanelTeam {
+    int rank, size;
+    double* red;
+    int* redi;
+    __device__ double reduce_jmax(double v) const {
+        v = warp_jmax(v);
+        pp_warps_barrier(size);
+        if ((rank & 31) == 0) red[rank >> 5] = v;
+        pp_warps_barrier(size);
+        double r = red[0];
+        for (int w = 1; w < (size >> 5); ++w) r = jmax(r, red[w]);
+        return r;
     }
-}
+    __device__ void reduce_argmax(double& v, int& idx) const {
+        warp_argmax(v, idx);
+        pp_warps_barrier(size);
+        if ((rank & 31) == 0) {
+            red[rank >> 5] = v;
+            redi[rank >> 5] = idx;
+        }
+        pp_warps_barrier(size);
+        v = red[0];
+        idx = redi[0];
+        for (int w = 1; w < (size >> 5); ++w)
+            if (red[w] > v || (red[w] == v && redi[w] >= 0 && (idx < 0 || redi[w] < idx))) {
+                v = red[w];
+                idx = redi[w];
+            }
+    }
+};
 
 // The reference's best_1x1 and what follows a rejected choice (bc, br), by one CTA over the whole, up to date
 // front: the acceptable diagonal of largest magnitude, first on ties, tried in that order
 template <typename T, bool GEN>
-__device__ void pp_search(const PanelFront<T, GEN>& F, PanelSmem<T>& S, int k, int pivot, double u, double eps, int bc,
+__device__ void pp_search(const PanelFront<T, GEN>& F, PanelSmem<T>& S, int nw, int k, int pivot, double u, double eps, int bc,
                           int br, int& c_out, int& r_out) {
-    const CtaTeam tm{(int)threadIdx.x, PP_THREADS, S.red, S.redi};
+    const PanelTeam tm{(int)threadIdx.x, nw * 32, S.red, S.redi};
     r_out = -1;
     double la = -1.0;      // the last candidate tried; -1: none yet
     int lj = -1;
@@ -200,10 +269,8 @@ __device__ void pp_search(const PanelFront<T, GEN>& F, PanelSmem<T>& S, int k, i
             if (x > a) { a = x; j = i; }
         }
         tm.reduce_argmax(a, j);
-        __syncthreads();
         if (j < 0) break;
         if (threshold_ok(F, j, k, u, a, tm)) { c_out = j; return; }
-        __syncthreads();
         la = a;
         lj = j;
     }
@@ -232,7 +299,11 @@ struct PanelPivot {
 };
 
 // The pivot steps of the block that starts at column k0, by the leader's CTAs. Returns k1, the first column
-// that is left; st[] collects the statistics (every thread holds the same).
+// that is left; st[] collects the statistics (every thread of the warps that hold rows has the same).
+//
+// A step is a chain of latencies, not of work: the maxima and the pivot row to the other CTAs, the decision,
+// a division, the update of up to 31 columns. Two thousand rows in eight CTAs take 1 us a column against 11
+// through group barriers in global memory.
 template <typename T, int STRUCT>
 __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelPivot& pv, int k0, int64_t* st) {
     constexpr bool GEN = STRUCT == STRUCT_G;
@@ -244,8 +315,8 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
     const int nw = chunk >> 5, nparts = C * nw;
     const int orig = tid < chunk && k0 + F.rank * chunk + tid < f ? k0 + F.rank * chunk + tid : -1;
     int rp = orig;                      // the row's place; a finished row keeps its own (<= k)
-    T a[PP_NB];                         // the row's entries of columns k, k + 1, ... and, behind them, its
-                                        // multipliers: one rotation per eliminated column
+    T a[PP_NB];                         // the row's entries of columns k, k + 1, ...: the columns move down by one
+                                        // with every eliminated one, so that no index depends on k
     int mylp = 0;
     const double alpha = (1.0 + sqrt(17.0)) / 8.0;
     auto load = [&]() {
@@ -255,317 +326,295 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
     };
     load();
     if (F.rank == 0 && tid == 0) F.hdr->ndisp = F.hdr->moved = 0;
-    int par = 0, j = 0;
-    while (j < nb) {
-        const int k = k0 + j;
-        // a bound of the column below row k, and row k itself, to every leader CTA
-        if (warp < nw) {
-            const unsigned h = __reduce_max_sync(0xffffffffu, rp > k ? pp_hi(a[0]) : 0u);
-            if (lane < C) pp_put(&S.hi[par][F.rank * nw + warp], lane, F.rank, h);
-            pp_publish(F, S, a, rp, k, j);
-        }
-        pp_sync(F);
-        unsigned h = 0;
-        for (int i = lane; i < nparts; i += 32) h = max(h, S.hi[par][i]);
-        const double bound = pp_bound<T>(__reduce_max_sync(0xffffffffu, h));
-        par ^= 1;
-        const double akk = fabs((double)S.prow[j][1]);
-        // The bound alone accepts most pivots (every test grows with the maxima). Else the exact maxima:
-        // lambda = max over the rows k < i < w with its first row r, mall = max over all rows i > k (NaN wins).
-        bool fast;
-        if (GEN) fast = !pv.lu_pivot || (akk >= pv.u * bound && akk >= pv.u * akk);
-        else if (pv.pivot == PIVOT_NONE) fast = true;
-        else fast = akk >= pv.eps && akk >= pv.u * bound && (pv.pivot == PIVOT_DIAGONAL || akk >= alpha * bound);
-        double lambda = 0.0, mall = 0.0;
-        int r = -1;
-        if (!fast) {
-            if (warp < nw) {
+    if (warp < nw) {
+        PanelX<T, GEN> X(F, S, nw);
+        int j = 0;
+        while (j < nb) {
+            const int k = k0 + j, left = nb - j;   // columns k .. kend - 1
+            // a bound of the column below row k, and row k itself, to every leader CTA
+            X.open(nparts * 4 + X.row_bytes(left));
+            unsigned h = __reduce_max_sync(0xffffffffu, rp > k ? pp_hi(a[0]) : 0u);
+            if (lane < C) X.put(&S.hi[X.b][F.rank * nw + warp], lane, h);
+            X.row(a, rp, k, j, left);
+            X.close();
+            h = 0;
+            for (int i = lane; i < nparts; i += 32) h = max(h, S.hi[X.b][i]);
+            const double bound = pp_bound<T>(__reduce_max_sync(0xffffffffu, h));
+            const double akk = fabs((double)S.prow[j][1]);
+            // The bound alone accepts most pivots (every test grows with the maxima). Else the exact maxima:
+            // lambda = max over the rows k < i < w with its first row r, mall = max over all rows i > k (NaN wins).
+            bool fast;
+            if (GEN) fast = !pv.lu_pivot || (akk >= pv.u * bound && akk >= pv.u * akk);
+            else if (pv.pivot == PIVOT_NONE) fast = true;
+            else fast = akk >= pv.eps && akk >= pv.u * bound && (pv.pivot == PIVOT_DIAGONAL || akk >= alpha * bound);
+            int c = k, r2 = -1;
+            if (!fast) {
                 const unsigned long long key = rp > k ? pp_key(a[0]) : 0ull;
                 const unsigned long long mkey = pp_warp_max<T>(key);
                 int ri = rp;
                 const unsigned long long lkey =
                     pp_warp_argmax<T>(rp > k && rp < w && key <= pp_inf<T>() ? key : 0ull, ri);
+                X.open(nparts * 20);
                 if (lane < C) {
                     const int at = F.rank * nw + warp;
-                    pp_put(&S.lam[at], lane, F.rank, lkey);
-                    pp_put(&S.mx[at], lane, F.rank, mkey);
-                    pp_put(&S.ridx[at], lane, F.rank, ri);
+                    X.put(&S.lam[at], lane, lkey);
+                    X.put(&S.mx[at], lane, mkey);
+                    X.put(&S.ridx[at], lane, ri);
                 }
-            }
-            pp_sync(F);
-            unsigned long long lk = 0, mk = 0;
-            r = 0x7fffffff;
-            for (int i = lane; i < nparts; i += 32) {
-                const unsigned long long l = S.lam[i], m = S.mx[i];
-                const int ri = S.ridx[i];
-                if (l > lk || (l == lk && l != 0 && ri < r)) { lk = l; r = ri; }
-                if (m > mk) mk = m;
-            }
-            lk = pp_warp_argmax<T>(lk, r);
-            lambda = pp_val<T>(lk);
-            mall = pp_val<T>(pp_warp_max<T>(mk));
-        }
-        int c = k, r2 = -1;
-        if (GEN) {
-            if (!fast && !(akk >= pv.u * jmax(mall, akk)) && r >= 0 && lambda > akk) c = r;
-            if (c != k) {   // row interchange: rows change places, their data stay
-                pp_sync(F);
-                if (rp == k) rp = c;
-                else if (rp == c) rp = k;
-                if (warp < nw) pp_publish(F, S, a, rp, k, j);
-                pp_sync(F);
-            }
-        } else if (!fast) {
-            bool acc;
-            int bc = k, br = -1;
-            if (pv.pivot == PIVOT_DIAGONAL || r < 0 || akk >= alpha * lambda) {
-                acc = akk >= pv.eps && akk >= pv.u * mall;
-            } else {
-                if (r >= kend && j > 0) break;   // the partner's column is not up to date
-                // column r: its maxima, those of column k without row r, and the corner entries
-                T v = T(0);
-                if (rp >= k) v = r < kend ? pp_pick(a, r - k) : F.at(orig, r);
-                if (warp < nw) {
-                    const unsigned long long kv = rp >= k && rp != r ? pp_key(v) : 0ull;
-                    const unsigned long long s1 = pp_warp_max<T>(rp < w ? kv : 0ull);
-                    const unsigned long long s2 = pp_warp_max<T>(rp != k ? kv : 0ull);
-                    const unsigned long long s3 = pp_warp_max<T>(rp > k && rp != r ? pp_key(a[0]) : 0ull);
-                    if (lane < C) {
-                        const int at = F.rank * nw + warp;
-                        pp_put(&S.sg[at], lane, F.rank, s1);
-                        pp_put(&S.m2[at], lane, F.rank, s2);
-                        pp_put(&S.m1[at], lane, F.rank, s3);
-                    }
-                    if (rp == r)
-                        for (int q = 0; q < C; ++q) {
-                            pp_put(&S.sc[0], q, F.rank, v);
-                            pp_put(&S.sc[2], q, F.rank, a[0]);
-                        }
-                    if (rp == k)
-                        for (int q = 0; q < C; ++q) pp_put(&S.sc[1], q, F.rank, v);
-                }
-                pp_sync(F);
-                unsigned long long s1 = 0, s2 = 0, s3 = 0;
+                X.close();
+                unsigned long long lk = 0, mk = 0;
+                int r = 0x7fffffff;
                 for (int i = lane; i < nparts; i += 32) {
-                    if (S.sg[i] > s1) s1 = S.sg[i];
-                    if (S.m2[i] > s2) s2 = S.m2[i];
-                    if (S.m1[i] > s3) s3 = S.m1[i];
+                    const unsigned long long l = S.lam[i], m = S.mx[i];
+                    const int x = S.ridx[i];
+                    if (l > lk || (l == lk && l != 0 && x < r)) { lk = l; r = x; }
+                    if (m > mk) mk = m;
                 }
-                const double sigma = pp_val<T>(pp_warp_max<T>(s1)), m2 = pp_val<T>(pp_warp_max<T>(s2)),
-                             m1 = pp_val<T>(pp_warp_max<T>(s3));
-                const double fkk = (double)S.prow[j][1], frr = (double)S.sc[0], fkr = (double)S.sc[1],
-                             frk = (double)S.sc[2];
-                if (akk * sigma >= alpha * lambda * lambda) {
-                    acc = akk >= pv.eps && akk >= pv.u * mall;
-                } else if (fabs(frr) >= alpha * sigma) {
-                    bc = r;
-                    acc = fabs(frr) >= pv.eps && fabs(frr) >= pv.u * jmax(m2, fabs(fkr));
+                lk = pp_warp_argmax<T>(lk, r);
+                const double lambda = pp_val<T>(lk), mall = pp_val<T>(pp_warp_max<T>(mk));
+                if (GEN) {
+                    if (!(akk >= pv.u * jmax(mall, akk)) && r >= 0 && lambda > akk) c = r;
                 } else {
-                    br = r;
-                    const double det = fkk * frr - fkr * frk;
-                    const double big = jmax(jmax(fabs(fkk), fabs(frk)), fabs(frr));
-                    acc = det != 0.0 && isfinite(det) && big >= pv.eps;
-                    if (acc) {
-                        const double e11 = fabs(frr / det), e12 = fabs(fkr / det), e21 = fabs(frk / det),
-                                     e22 = fabs(fkk / det);
-                        acc = pv.u * (e11 * m1 + e21 * m2) <= 1.0 && pv.u * (e12 * m1 + e22 * m2) <= 1.0;
+                    bool acc;
+                    int bc = k, br = -1;
+                    if (pv.pivot == PIVOT_DIAGONAL || r < 0 || akk >= alpha * lambda) {
+                        acc = akk >= pv.eps && akk >= pv.u * mall;
+                    } else {
+                        if (r >= kend && j > 0) break;   // the partner's column is not up to date
+                        // column r: its maxima, those of column k without row r, and the corner entries
+                        T v = T(0);
+                        if (rp >= k) v = r < kend ? pp_pick(a, r - k) : F.at(orig, r);
+                        const unsigned long long kv = rp >= k && rp != r ? pp_key(v) : 0ull;
+                        unsigned long long s1 = pp_warp_max<T>(rp < w ? kv : 0ull);
+                        unsigned long long s2 = pp_warp_max<T>(rp != k ? kv : 0ull);
+                        unsigned long long s3 = pp_warp_max<T>(rp > k && rp != r ? pp_key(a[0]) : 0ull);
+                        X.open(nparts * 24 + 3 * (int)sizeof(T));
+                        if (lane < C) {
+                            const int at = F.rank * nw + warp;
+                            X.put(&S.sg[at], lane, s1);
+                            X.put(&S.m2[at], lane, s2);
+                            X.put(&S.m1[at], lane, s3);
+                        }
+                        if (rp == r)
+                            for (int q = 0; q < C; ++q) {
+                                X.put(&S.sc[0], q, v);
+                                X.put(&S.sc[2], q, a[0]);
+                            }
+                        if (rp == k)
+                            for (int q = 0; q < C; ++q) X.put(&S.sc[1], q, v);
+                        X.close();
+                        s1 = s2 = s3 = 0;
+                        for (int i = lane; i < nparts; i += 32) {
+                            if (S.sg[i] > s1) s1 = S.sg[i];
+                            if (S.m2[i] > s2) s2 = S.m2[i];
+                            if (S.m1[i] > s3) s3 = S.m1[i];
+                        }
+                        const double sigma = pp_val<T>(pp_warp_max<T>(s1)), m2 = pp_val<T>(pp_warp_max<T>(s2)),
+                                     m1 = pp_val<T>(pp_warp_max<T>(s3));
+                        const double fkk = (double)S.prow[j][1], frr = (double)S.sc[0], fkr = (double)S.sc[1],
+                                     frk = (double)S.sc[2];
+                        if (akk * sigma >= alpha * lambda * lambda) {
+                            acc = akk >= pv.eps && akk >= pv.u * mall;
+                        } else if (fabs(frr) >= alpha * sigma) {
+                            bc = r;
+                            acc = fabs(frr) >= pv.eps && fabs(frr) >= pv.u * jmax(m2, fabs(fkr));
+                        } else {
+                            br = r;
+                            const double det = fkk * frr - fkr * frk;
+                            const double big = jmax(jmax(fabs(fkk), fabs(frk)), fabs(frr));
+                            acc = det != 0.0 && isfinite(det) && big >= pv.eps;
+                            if (acc) {
+                                const double e11 = fabs(frr / det), e12 = fabs(fkr / det), e21 = fabs(frk / det),
+                                             e22 = fabs(fkk / det);
+                                acc = pv.u * (e11 * m1 + e21 * m2) <= 1.0 && pv.u * (e12 * m1 + e22 * m2) <= 1.0;
+                            }
+                        }
+                    }
+                    c = bc;
+                    r2 = br;
+                    if (!acc) {
+                        if (j > 0) break;                // the search needs the whole front up to date
+                        X.open(8);
+                        if (F.rank == 0) {
+                            int cs = k, rs = -1;
+                            pp_search(F, S, nw, k, pv.pivot, pv.u, pv.eps, bc, br, cs, rs);
+                            if (tid == 0)
+                                for (int q = 0; q < C; ++q) {
+                                    X.put(&S.sel[0], q, cs);
+                                    X.put(&S.sel[1], q, rs);
+                                }
+                        }
+                        X.close();
+                        c = S.sel[0];
+                        r2 = S.sel[1];
                     }
                 }
+                const int p = r2 < 0 ? k : k + 1, q = r2 < 0 ? c : r2;
+                if (p != q || r2 >= 0) {
+                    X.meet();                            // everyone has read what the exchange below overwrites
+                    if (p != q && q < kend) {            // "S" inside the block: columns in registers; rows by place
+                        if (!GEN && rp >= k) {
+                            const int y = q - k;
+                            const T vp = p == k ? a[0] : a[1], vq = pp_pick(a, y);
+                            if (p == k) a[0] = vq;
+                            else a[1] = vq;
+#pragma unroll
+                            for (int e = 1; e < PP_NB; ++e)
+                                if (e == y) a[e] = vp;
+                        }
+                        if (rp == p) rp = q;
+                        else if (rp == q) rp = p;
+                    } else if (p != q && GEN) {          // row interchange: rows change places, their data stay
+                        if (rp == p) rp = q;
+                        else if (rp == q) rp = p;
+                    } else if (p != q) {                 // outside it (j = 0): the interchange in memory
+                        const int gt = F.rank * nw * 32 + tid, GT = C * nw * 32;
+                        for (int i = gt; i < f; i += GT) {
+                            if (i == p || i == q) continue;
+                            const T t = F.at(i, p);
+                            F.at(i, p) = F.at(i, q);
+                            F.at(i, q) = t;
+                        }
+                        for (int i = gt; i < w; i += GT) {
+                            if (i == p || i == q) continue;
+                            const T t = F.at(p, i);
+                            F.at(p, i) = F.at(q, i);
+                            F.at(q, i) = t;
+                        }
+                        if (gt == 0) {
+                            T t = F.at(p, p);
+                            F.at(p, p) = F.at(q, q);
+                            F.at(q, q) = t;
+                            t = F.at(p, q);
+                            F.at(p, q) = F.at(q, p);
+                            F.at(q, p) = t;
+                            const int tl = F.lp[p];
+                            F.lp[p] = F.lp[q];
+                            F.lp[q] = tl;
+                        }
+                        X.meet(true);
+                        load();
+                    }
+                    X.open((r2 >= 0 ? 2 : 1) * X.row_bytes(left));
+                    X.row(a, rp, k, j, left);
+                    if (r2 >= 0) X.row(a, rp, k + 1, j + 1, left);
+                    X.close();
+                }
             }
-            c = bc;
-            r2 = br;
-            if (!acc) {
-                if (j > 0) break;                // the search needs the whole front up to date
-                if (F.rank == 0) {
-                    int cs = k, rs = -1;
-                    pp_search(F, S, k, pv.pivot, pv.u, pv.eps, bc, br, cs, rs);
-                    __syncthreads();
-                    if (tid == 0)
-                        for (int q = 0; q < C; ++q) {
-                            pp_put(&S.sel[0], q, 0, cs);
-                            pp_put(&S.sel[1], q, 0, rs);
+            const bool lead = F.rank == 0 && tid == 0;
+            if (GEN || r2 < 0) {
+                double dk = (double)S.prow[j][1];
+                int kk = KIND_1X1;
+                if (!(fabs(dk) >= pv.eps) || dk == 0.0) {
+                    if (dk == 0.0) st[ST_NZERO]++;
+                    int lpk = 0;
+                    if (!GEN) {   // the column this row is of
+                        X.open(4);
+                        if (rp == k)
+                            for (int q = 0; q < C; ++q) X.put(&S.plp, q, mylp);
+                        X.close();
+                        lpk = S.plp;
+                    }
+                    const int req = !GEN && pv.psign ? (int)pv.psign[pv.perm[F.c0 + lpk]] : 0;
+                    dk = perturb_sign_of(dk, req) * pv.eps;
+                    kk = KIND_PERTURBED;
+                    st[ST_NPERT]++;
+                    if (dk == 0.0 && st[ST_INFO] == 0) st[ST_INFO] = (GEN ? k : lpk) + 1;
+                }
+                if (!GEN) {
+                    if (dk > 0) st[ST_NPOS]++;
+                    else if (dk < 0) st[ST_NNEG]++;
+                }
+                if (lead) {
+                    F.dd[k] = dk;
+                    if (!GEN) F.ee[k] = 0.0;
+                    F.kd[k] = (signed char)kk;
+                }
+                if (tid == 0) {
+                    S.kind[j] = kk;
+                    S.tdk[j] = dk;
+                }
+                if (rp > k) {
+                    const T l = GEN ? a[0] / T(dk) : T((double)a[0] / dk);
+                    S.L[j][tid] = l;
+                    const T* row = S.prow[j] + 1;
+                    // columns at and beyond `left` hold nothing any more, whatever lands in them
+#pragma unroll
+                    for (int g = 0; g < PP_NB; g += 8)
+                        if (g + 1 < left) {
+#pragma unroll
+                            for (int e = g; e < g + 8; e += 2) {
+                                T u0, u1 = T(0);
+                                if (e + 2 < PP_NB) pp_load2(row + e + 1, u0, u1);
+                                else u0 = row[e + 1];
+                                a[e] = a[e + 1] - l * u0;
+                                if (e + 2 < PP_NB) a[e + 1] = a[e + 2] - l * u1;
+                            }
                         }
                 }
-                pp_sync(F);
-                c = S.sel[0];
-                r2 = S.sel[1];
-            }
-            const int p = r2 < 0 ? k : k + 1, q = r2 < 0 ? c : r2;
-            if (p != q || r2 >= 0) {
-                pp_sync(F);                      // everyone has read what the exchanges below overwrite
-                if (p != q && q < kend) {        // inside the block: columns in registers, rows by place
-                    if (rp >= k) {
-                        const int y = q - k;
-                        const T vp = p == k ? a[0] : a[1], vq = pp_pick(a, y);
-                        if (p == k) a[0] = vq;
-                        else a[1] = vq;
+                j += 1;
+            } else {
+                const double fa = (double)S.prow[j][1], fb = (double)S.prow[j + 1][1], fc = (double)S.prow[j + 1][2];
+                const double det = fa * fc - fb * fb;
+                const double e11 = fc / det, e12 = -fb / det, e21 = -fb / det, e22 = fa / det;
+                st[ST_N2X2]++;
+                if (det < 0) { st[ST_NPOS]++; st[ST_NNEG]++; }
+                else if (fa > 0) st[ST_NPOS] += 2;
+                else st[ST_NNEG] += 2;
+                if (lead) {
+                    F.dd[k] = fa; F.dd[k + 1] = fc; F.ee[k] = fb; F.ee[k + 1] = 0.0;
+                    F.kd[k] = KIND_2X2_FIRST; F.kd[k + 1] = KIND_2X2_SECOND;
+                }
+                if (tid == 0) {
+                    S.kind[j] = KIND_2X2_FIRST;
+                    S.kind[j + 1] = KIND_2X2_SECOND;
+                    S.tdk[j] = S.tdk[j + 1] = 1.0;
+                }
+                if (rp == k + 1) S.L[j][tid] = T(0);
+                if (rp > k + 1) {
+                    const double x1 = (double)a[0], x2 = (double)a[1];
+                    const T l1 = T(x1 * e11 + x2 * e21), l2 = T(x1 * e12 + x2 * e22);
+                    S.L[j][tid] = l1;
+                    S.L[j + 1][tid] = l2;
 #pragma unroll
-                        for (int e = 1; e < PP_NB; ++e)
-                            if (e == y) a[e] = vp;
-                    }
-                    if (rp == p) rp = q;
-                    else if (rp == q) rp = p;
-                } else if (p != q) {             // outside it (j = 0): the interchange in memory
-                    const int gt = F.rank * PP_THREADS + tid, GT = C * PP_THREADS;
-                    for (int i = gt; i < f; i += GT) {
-                        if (i == p || i == q) continue;
-                        const T t = F.at(i, p);
-                        F.at(i, p) = F.at(i, q);
-                        F.at(i, q) = t;
-                    }
-                    for (int i = gt; i < w; i += GT) {
-                        if (i == p || i == q) continue;
-                        const T t = F.at(p, i);
-                        F.at(p, i) = F.at(q, i);
-                        F.at(q, i) = t;
-                    }
-                    if (gt == 0) {
-                        T t = F.at(p, p);
-                        F.at(p, p) = F.at(q, q);
-                        F.at(q, q) = t;
-                        t = F.at(p, q);
-                        F.at(p, q) = F.at(q, p);
-                        F.at(q, p) = t;
-                        const int tl = F.lp[p];
-                        F.lp[p] = F.lp[q];
-                        F.lp[q] = tl;
-                    }
-                    pp_sync(F);
-                    load();
+                    for (int e = 0; e < PP_NB - 2; ++e)
+                        if (e + 2 < left) a[e] = a[e + 2] - (l1 * S.prow[j][e + 3] + l2 * S.prow[j + 1][e + 3]);
                 }
-                if (warp < nw) {
-                    pp_publish(F, S, a, rp, k, j);
-                    if (r2 >= 0) pp_publish(F, S, a, rp, k + 1, j + 1);
-                }
-                pp_sync(F);
+                j += 2;
             }
         }
-        const bool lead = F.rank == 0 && tid == 0;
-        if (GEN || r2 < 0) {
-            double dk = (double)S.prow[j][1];
-            int kk = KIND_1X1;
-            if (!(fabs(dk) >= pv.eps) || dk == 0.0) {
-                if (dk == 0.0) st[ST_NZERO]++;
-                int lpk = 0;
-                if (!GEN) {   // the column this row is of
-                    if (rp == k)
-                        for (int q = 0; q < C; ++q) pp_put(&S.plp, q, F.rank, mylp);
-                    pp_sync(F);
-                    lpk = S.plp;
-                }
-                const int req = !GEN && pv.psign ? (int)pv.psign[pv.perm[F.c0 + lpk]] : 0;
-                dk = perturb_sign_of(dk, req) * pv.eps;
-                kk = KIND_PERTURBED;
-                st[ST_NPERT]++;
-                if (dk == 0.0 && st[ST_INFO] == 0) st[ST_INFO] = (GEN ? k : lpk) + 1;
-            }
-            if (!GEN) {
-                if (dk > 0) st[ST_NPOS]++;
-                else if (dk < 0) st[ST_NNEG]++;
-            }
-            if (lead) {
-                F.dd[k] = dk;
-                if (!GEN) F.ee[k] = 0.0;
-                F.kd[k] = (signed char)kk;
-            }
-            if (tid == 0) {
-                S.kind[j] = kk;
-                S.tdk[j] = dk;
-            }
-            if (rp > k) {
-                const T l = GEN ? a[0] / T(dk) : T((double)a[0] / dk);
-                const int left = nb - j;   // columns k .. kend - 1
-                const T* row = S.prow[j] + 1;
-#pragma unroll
-                for (int g = 0; g < PP_NB; g += 8) {
-                    T u[8];
-#pragma unroll
-                    for (int e = 0; e < 8; e += 2)
-                        if (g + e + 2 < PP_NB) pp_load2(row + g + e + 1, u[e], u[e + 1]);
-                        else u[e] = row[g + e + 1 < PP_NB ? g + e + 1 : 0], u[e + 1] = T(0);
-                    if (g + 8 < left) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (g + e + 1 < PP_NB) a[g + e] = a[g + e + 1] - l * u[e];
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (g + e + 1 < PP_NB) {
-                                const T t = a[g + e + 1] - l * u[e];
-                                a[g + e] = g + e + 1 < left ? t : a[g + e + 1];
-                            }
-                    }
-                }
-                a[PP_NB - 1] = l;
-            }
-            j += 1;
-        } else {
-            const double fa = (double)S.prow[j][1], fb = (double)S.prow[j + 1][1], fc = (double)S.prow[j + 1][2];
-            const double det = fa * fc - fb * fb;
-            const double e11 = fc / det, e12 = -fb / det, e21 = -fb / det, e22 = fa / det;
-            st[ST_N2X2]++;
-            if (det < 0) { st[ST_NPOS]++; st[ST_NNEG]++; }
-            else if (fa > 0) st[ST_NPOS] += 2;
-            else st[ST_NNEG] += 2;
-            if (lead) {
-                F.dd[k] = fa; F.dd[k + 1] = fc; F.ee[k] = fb; F.ee[k + 1] = 0.0;
-                F.kd[k] = KIND_2X2_FIRST; F.kd[k + 1] = KIND_2X2_SECOND;
-            }
-            if (tid == 0) {
-                S.kind[j] = KIND_2X2_FIRST;
-                S.kind[j + 1] = KIND_2X2_SECOND;
-                S.tdk[j] = S.tdk[j + 1] = 1.0;
-            }
-            if (rp > k + 1) {
-                const double x1 = (double)a[0], x2 = (double)a[1];
-                const T l1 = T(x1 * e11 + x2 * e21), l2 = T(x1 * e12 + x2 * e22);
-                const int left = nb - j;
-#pragma unroll
-                for (int e = 0; e < PP_NB - 2; ++e) {
-                    const T t = a[e + 2] - (l1 * S.prow[j][e + 3] + l2 * S.prow[j + 1][e + 3]);
-                    a[e] = e + 2 < left ? t : a[e + 2];
-                }
-                a[PP_NB - 2] = l1;
-                a[PP_NB - 1] = l2;
-            }
-            j += 2;
-        }
+        if (tid == 0) S.nbd = j;
     }
-    const int nbd = j, k1 = k0 + nbd;
-    // the registers back to the columns' order, then out to the rows' places
+    __syncthreads();
+    const int nbd = S.nbd, k1 = k0 + nbd;
+    // the multipliers and what is left of the columns out to the rows' places
     if (orig >= 0 && rp >= k1) {
-        for (int t = nbd; t < PP_NB; ++t) {
-            const T a0 = a[0];
-#pragma unroll
-            for (int e = 0; e + 1 < PP_NB; ++e) a[e] = a[e + 1];
-            a[PP_NB - 1] = a0;
-        }
+        for (int e = 0; e < nbd; ++e) F.P[rp + (int64_t)(k0 + e) * f] = S.L[e][tid];
 #pragma unroll
         for (int e = 0; e < PP_NB; ++e)
-            if (e < nb) F.P[rp + (int64_t)(k0 + e) * f] = a[e];
+            if (nbd + e < nb) F.P[rp + (int64_t)(k1 + e) * f] = a[e];
         if (rp != orig) {
             const int d = atomicAdd(&F.hdr->ndisp, 1);
             F.hdr->ddst[d] = rp;
             F.hdr->dsrc[d] = orig;
         }
     } else if (orig >= 0) {
-        F.hdr->rowmap[rp - k0] = orig;
+        const int t = rp - k0;
+        F.hdr->rowmap[t] = orig;
+        for (int s = 0; s < t; ++s) {
+            const T l = S.L[s][tid];
+            F.P[rp + (int64_t)(k0 + s) * f] = l;
+            F.hdr->lt[s][t] = l;
+        }
     }
     if (orig >= 0 && rp != orig) F.hdr->moved = 1;
     if (orig >= 0 && rp < w) F.lp[rp] = mylp;
     if (F.rank == 0) {
-        __syncthreads();   // S.kind and S.tdk of the last step
-        for (int q = tid; q < PP_NB * PP_NB; q += PP_THREADS) {
-            const int t = q % PP_NB, s = q / PP_NB;      // row t, column s
-            T l = T(0);
-            if (s < t && t < nbd) {
-                const int rot = S.kind[t] == KIND_2X2_SECOND ? t - 1 : t;   // the row's rotations when it was taken
-                if (s < rot) l = S.prow[t][1 + PP_NB - rot + s];
-                F.P[(k0 + t) + (int64_t)(k0 + s) * f] = l;
+        if (GEN)
+            for (int q = tid; q < nbd * nb; q += PP_THREADS) {
+                const int t = q / nb, s = q % nb;        // row t, column s
+                if (s > t) F.U[(k0 + s) + (int64_t)(k0 + t) * f] = S.prow[t][1 + s - t] / T(S.tdk[t]);
             }
-            F.hdr->lt[s][t] = l;
-            if (GEN && s > t && s < nb) F.U[(k0 + s) + (int64_t)(k0 + t) * f] = S.prow[t][1 + s - t] / T(S.tdk[t]);
-        }
         if (tid < nbd) {
             F.hdr->kind[tid] = S.kind[tid];
             F.hdr->tdk[tid] = T(S.tdk[tid]);
@@ -776,7 +825,7 @@ __device__ void pp_urows(const PanelFront<T, true>& F, const PanelHdr<T>& H, int
 // One front, by every CTA of its group
 template <typename T, int STRUCT>
 __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelSmem<T>& S, int C, unsigned int* bar,
-                         int32_t* status) {
+                         int32_t* status, unsigned& xn) {
     constexpr bool GEN = STRUCT == STRUCT_G;
     const int s = A.list[job.fi];
     const DFront fd = A.fronts[s];
@@ -799,6 +848,7 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
     F.rank = job.rank < F.C ? job.rank : 0;
     F.gs = job.gs;
     F.grank = job.rank;
+    F.xn = xn;
     F.bar = bar + job.fi;
     F.epoch = 0;
     F.status = status;
@@ -846,6 +896,7 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
             if (!ok && !leads) return;
         }
     }
+    if (F.C > 1) xn = F.xn;   // one CTA alone uses no mbarrier
     if (!ok) return;
     if constexpr (GEN) pp_urows<T>(F, H, F.grank, F.gs);
     for (int64_t q = gt; q < (int64_t)w * w; q += GT) {
