@@ -32,6 +32,27 @@ struct DFront {
     int32_t rc_begin;  // this front's row-chunk starts among its parent's rows: rchunk[rc_begin + k], k <= K
 };
 
+// A shared-memory front as its kernel reads it, in launch order: one load instead of the list entry and the
+// front's descriptor; its children with a contribution block (kids), their rows among the front's (sri, child
+// after child), and the extend-add as items (front column p, kid, kid column t) ordered by p mod 8, p, kid: a
+// warp owns whole columns, so its additions need no barrier between children and keep their order.
+struct SFront {
+    int64_t panel, cb;
+    int32_t s, f, w, c0;
+    int32_t am_begin, am_end;
+    int32_t kid_begin, nkid;
+    int32_t sri_begin, nsri;   // also the items' range
+    int32_t ep_begin;          // 9 starts of the items with p mod 8 = 0 .. 7, relative to sri_begin
+    int32_t pad;
+};
+struct SKid {
+    int64_t cb;
+    int32_t mc, sri;           // order of its contribution block; its rows' start, relative to the front's
+};
+constexpr int SF_KIDS = 64;    // kids and items that the kernel stages in shared memory (the rest from global)
+constexpr int SF_ITEMS = 768;
+constexpr int SF_MAX_KIDS = 65535;   // an item packs p (8 bits), the kid (16) and t (8)
+
 // Rows of a front column that the large-front assembly builds at a time in shared memory (per warp)
 constexpr int ASM_ROWS = 256;
 

@@ -33,22 +33,83 @@
 
 namespace sds {
 
+// The in-front Cholesky of a front of at most 32 RPL rows by eight warps, in registers: warp q holds the
+// columns p = q (mod 8), lane the rows lane + 32 i. Per column one exchange: the owner scales it by the
+// reciprocal square root and puts it in shared memory (two buffers, one barrier), and every warp updates its
+// later columns. A column costs 0.2 us, against 0.35 with the front in shared memory and three barriers.
+// Returns 0, or 1 + the column whose pivot fails.
+template <typename T, int RPL>
+__device__ __forceinline__ int spd_front_regs(T (&a)[4 * RPL][RPL], int w, double eps, T* lcol, volatile int* fail) {
+    constexpr int CPW = 4 * RPL, R = 32 * RPL;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < CPW; ++c)
+        for (int q = 0; q < 8; ++q) {
+            const int k = 8 * c + q;
+            if (k >= w) return 0;
+            const int i0 = (8 * c) >> 5;   // the row chunk of row k
+            T* l = lcol + (k & 1) * R;
+            double d = 0.0;
+            if (warp == q) {
+                const double ajj = (double)__shfl_sync(0xffffffffu, a[c][i0], k & 31);
+                if (ajj > eps || (eps > 0 && ajj >= 0)) {
+                    d = fmax(ajj, eps);
+                    const T r = T(rsqrt(d));
+#pragma unroll
+                    for (int i = 0; i < RPL; ++i) {
+                        a[c][i] *= r;      // row k itself is set below; rows above are never read
+                        l[lane + 32 * i] = a[c][i];
+                    }
+                } else if (lane == 0) {
+                    *fail = k + 1;
+                }
+            }
+            __syncthreads();
+            if (*fail) return *fail;
+            T li[RPL];
+#pragma unroll
+            for (int i = 0; i < RPL; ++i) li[i] = l[lane + 32 * i];
+#pragma unroll
+            for (int c2 = c; c2 < CPW; ++c2) {
+                const int p = 8 * c2 + warp;
+                if (p > k) {
+                    const T lp = l[p];
+#pragma unroll
+                    for (int i = 0; i < RPL; ++i) a[c2][i] = fma(-li[i], lp, a[c2][i]);
+                }
+            }
+            if (warp == q && lane == (k & 31)) a[c][i0] = T(sqrt(d));
+        }
+    return 0;
+}
+
 // One front by the whole CTA, in shared memory (smem_raw holds at least small_front_smem(f)). The CTA's
-// threads all call it; it ends with the front's outputs written to global memory.
-template <typename T, int STRUCT>
-__device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int s, const int member,
+// threads all call it; it ends with the front's outputs written to global memory. RPL > 0: a Cholesky front
+// of at most 32 RPL rows, factored in registers by 256 threads.
+//
+// The bottom levels are launches of a few dependent loads per front, so the loads that do not depend on one
+// another go out together: the record; then the kids, rows, items and entries of A; then every contribution.
+// (Children one after another, each behind its descriptor, its rows and a barrier: lap2d 16^2 218 us a
+// factorization, now 140; lap2d 64^2 1048, now 612; 256 uneven FP32 systems 2530, now 1680. Three launches in
+// four are still latency: 5 us each.)
+template <typename T, int STRUCT, int RPL>
+__device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int at, const int member,
                                             unsigned char* smem_raw) {
-    const DFront fd = A.maps.fronts[s];
+    const SFront fd = A.sf[at];
+    const int s = fd.s;
     const int f = fd.f, w = fd.w, m = f - w;
     const int ld = f | 1;
     T* F = reinterpret_cast<T*>(smem_raw);
     size_t off = ((size_t)ld * f * sizeof(T) + 15) & ~size_t(15);
-    double* dd = reinterpret_cast<double*>(smem_raw + off);  // w
+    SKid* skid = reinterpret_cast<SKid*>(smem_raw + off);    // SF_KIDS
+    uint32_t* sitem = reinterpret_cast<uint32_t*>(skid + SF_KIDS);   // SF_ITEMS
+    uint8_t* ssri = reinterpret_cast<uint8_t*>(sitem + SF_ITEMS);    // SF_ITEMS
+    double* dd = reinterpret_cast<double*>(ssri + SF_ITEMS); // w
     double* ee = dd + w;                                     // w
     double* lvec = ee + w;                                   // 2 f (multipliers)
     int* lp = reinterpret_cast<int*>(lvec + 2 * f);          // w
-    int* ri = lp + w;                                        // relind of the current child (<= f)
-    int* ctl = ri + f;                                       // control words
+    // control words; with the front in registers behind the two column buffers (at dd)
+    int* ctl = RPL > 0 ? reinterpret_cast<int*>(reinterpret_cast<T*>(dd) + 64 * RPL) : lp + f;
     signed char* kd = reinterpret_cast<signed char*>(ctl + 16);
 
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
@@ -56,37 +117,125 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int s, 
     T* factor = A.factor + (int64_t)member * A.factor_len;
     T* cbar = A.cb + (int64_t)member * A.cb_len;
 
+    // this thread's first entry of A, on its way while the front is cleared
+    int k = fd.am_begin + tid, code = 0, before = 0;
+    double v0 = 0.0;
+    if (k < fd.am_end) {
+        code = A.maps.am_loc[k];
+        before = k > fd.am_begin ? A.maps.am_loc[k - 1] : 0;
+        v0 = nz[A.maps.am_src[k]];
+    }
+    const bool skids = fd.nkid <= SF_KIDS, sits = fd.nsri <= SF_ITEMS;
+    if (skids && tid < fd.nkid) skid[tid] = A.kids[fd.kid_begin + tid];
+    if (sits)
+        for (int q = tid; q < fd.nsri; q += nt) {
+            sitem[q] = A.items[fd.sri_begin + q];
+            ssri[q] = A.sri[fd.sri_begin + q];
+        }
+    const SKid* kids = skids ? skid : A.kids + fd.kid_begin;
+    const uint32_t* items = sits ? sitem : A.items + fd.sri_begin;
+    const uint8_t* sri = sits ? ssri : A.sri + fd.sri_begin;
     for (int q = tid; q < ld * f; q += nt) F[q] = T(0);
     if (tid < 16) ctl[tid] = 0;
     __syncthreads();
     // assembly of A: each run of equal destinations is summed by one thread, in entry order
-    for (int k = fd.am_begin + tid; k < fd.am_end; k += nt) {
-        int code = A.maps.am_loc[k];
-        if (k > fd.am_begin && A.maps.am_loc[k - 1] == code) continue;
+    for (; k < fd.am_end; k += nt) {
+        if (k != fd.am_begin + tid) {
+            code = A.maps.am_loc[k];
+            before = A.maps.am_loc[k - 1];
+            v0 = nz[A.maps.am_src[k]];
+        }
+        if (before == code) continue;
         T acc = T(0);
-        for (int q = k; q < fd.am_end && A.maps.am_loc[q] == code; ++q) acc += T(nz[A.maps.am_src[q]]);
+        acc += T(v0);
+        for (int q = k + 1; q < fd.am_end && A.maps.am_loc[q] == code; ++q) acc += T(nz[A.maps.am_src[q]]);
         int loc = (code > 0 ? code : -code) - 1;
         int i = loc % f, j = loc / f;
         if (code > 0) F[i + j * ld] += acc;
         else F[j + i * ld] += acc;
     }
-    __syncthreads();
-    // extend-add, children in order
-    for (int q = fd.ch_begin; q < fd.ch_end; ++q) {
-        const int c = A.maps.child_list[q];
-        const DFront cd = A.maps.fronts[c];
-        const int mc = cd.f - cd.w;
-        if (mc <= 0 || cd.cb < 0) continue;
-        for (int t = tid; t < mc; t += nt) ri[t] = A.maps.relind[cd.ri_begin + t];
-        __syncthreads();
-        const T* C = cbar + cd.cb;
-        for (int jj = warp; jj < mc; jj += nwarps) {
-            const int pj = ri[jj];
-            const int i0 = STRUCT == STRUCT_G ? 0 : jj;
-            batched_add<8, T>(i0 + lane, 32, mc, [&](int ii) { return (double)C[ii + (int64_t)jj * mc]; },
-                              [&](int ii) -> T* { return F + ri[ii] + pj * ld; });
+    // extend-add: a warp's columns, item after item, the first 64 rows of SF_U items loaded before the first
+    // addition (and the first of all before the barrier behind the entries of A)
+    constexpr int SF_U = 4;
+    T v[SF_U][2];
+    int n[SF_U], q0[SF_U], p[SF_U];
+    const T* col[SF_U];
+    const uint8_t* ri[SF_U];
+    int g = warp, e = A.ep[fd.ep_begin + g], e1 = A.ep[fd.ep_begin + g + 1];
+    auto load = [&]() {
+#pragma unroll
+        for (int u = 0; u < SF_U; ++u) {
+            n[u] = 0;
+            if (e + u >= e1) continue;
+            const uint32_t it = items[e + u];
+            const SKid kid = kids[(it >> 8) & 0xffffu];
+            const int t = it & 0xffu;
+            p[u] = it >> 24;
+            q0[u] = STRUCT == STRUCT_G ? 0 : t;
+            n[u] = kid.mc;
+            col[u] = cbar + kid.cb + (int64_t)t * kid.mc;
+            ri[u] = sri + kid.sri;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int q = q0[u] + lane + 32 * x;
+                v[u][x] = q < n[u] ? col[u][q] : T(0);
+            }
         }
-        __syncthreads();
+    };
+    load();
+    __syncthreads();
+    while (true) {
+#pragma unroll
+        for (int u = 0; u < SF_U; ++u) {
+            if (n[u] == 0) continue;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int q = q0[u] + lane + 32 * x;
+                if (q < n[u]) F[ri[u][q] + p[u] * ld] += v[u][x];
+            }
+            for (int q = q0[u] + lane + 64; q < n[u]; q += 32) F[ri[u][q] + p[u] * ld] += col[u][q];
+            __syncwarp();
+        }
+        e += SF_U;
+        while (e >= e1 && (g += nwarps) < 8) {
+            e = A.ep[fd.ep_begin + g];
+            e1 = A.ep[fd.ep_begin + g + 1];
+        }
+        if (e >= e1) break;
+        load();
+    }
+    __syncthreads();
+    if constexpr (RPL > 0) {
+        constexpr int CPW = 4 * RPL;
+        T a[CPW][RPL];
+#pragma unroll
+        for (int c = 0; c < CPW; ++c)
+#pragma unroll
+            for (int i = 0; i < RPL; ++i) {
+                const int p = 8 * c + warp, r = lane + 32 * i;
+                a[c][i] = (p < f && r < f && r >= p) ? F[r + p * ld] : T(0);
+            }
+        const int status = spd_front_regs<T, RPL>(a, w, A.eps, reinterpret_cast<T*>(dd), ctl);
+        T* P = factor + fd.panel;
+        const bool cbw = fd.cb >= 0 && m > 0 && status == 0;
+        T* C = cbar + fd.cb;
+#pragma unroll
+        for (int c = 0; c < CPW; ++c)
+#pragma unroll
+            for (int i = 0; i < RPL; ++i) {
+                const int p = 8 * c + warp, r = lane + 32 * i;
+                if (p < w) {
+                    if (r < f) P[r + (int64_t)p * f] = r < p ? T(0) : a[c][i];
+                } else if (cbw && p < f && r < f && r >= p) {
+                    C[(r - w) + (int64_t)(p - w) * m] = a[c][i];
+                }
+            }
+        if (tid == 0) {
+            int64_t* S = A.stats + ((int64_t)member * A.ns + s) * NSTAT;
+            for (int q = 0; q < NSTAT; ++q) S[q] = q == ST_NPOS ? (status ? status - 1 : w) : q == ST_INFO ? status : 0;
+            A.finfo[(int64_t)member * A.ns + s] = status;
+        }
+        return;
     }
     if (STRUCT == STRUCT_S) {  // the pivoting reads both triangles of the fully-summed block
         for (int q = tid; q < w * w; q += nt) {
@@ -192,15 +341,15 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int s, 
     }
 }
 
-template <typename T, int STRUCT>
+template <typename T, int STRUCT, int RPL>
 __global__ void __launch_bounds__(256) small_front_kernel(SmallArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
-    small_front<T, STRUCT>(A, A.list[blockIdx.x], member, smem_raw);
+    small_front<T, STRUCT, RPL>(A, blockIdx.x, member, smem_raw);
 }
 
 // Fused subtrees: one CTA factors a whole subtree of shared-memory fronts, front after front in the
-// subtree's postorder (A.list[A.sub_ptr[b] .. A.sub_ptr[b + 1]) for CTA b), in one launch for every
+// subtree's postorder (A.sf[A.sub_ptr[b] .. A.sub_ptr[b + 1]) for CTA b), in one launch for every
 // subtree of its size class instead of one launch per level. A child's contribution block goes to
 // global memory (the subtree's stack region of the arena, hot in L2) and its parent, later in the same
 // CTA, reads it back after the barrier between the two fronts, which makes the CTA's global writes
@@ -208,13 +357,13 @@ __global__ void __launch_bounds__(256) small_front_kernel(SmallArgs<T> A) {
 // the level launches'. Replaces the reference's regime-A kernels (subtree_cholesky_kernel!
 // src/numeric/subtree.jl:274-316, subtree_ldlt_kernel! src/numeric/ldlt.jl:1133-1228,
 // subtree_lu_kernel! src/numeric/lu.jl:424-493).
-template <typename T, int STRUCT>
+template <typename T, int STRUCT, int RPL>
 __global__ void __launch_bounds__(256) subtree_kernel(SmallArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
     const int q0 = A.sub_ptr[blockIdx.x], q1 = A.sub_ptr[blockIdx.x + 1];
     for (int q = q0; q < q1; ++q) {
-        small_front<T, STRUCT>(A, A.list[q], member, smem_raw);
+        small_front<T, STRUCT, RPL>(A, q, member, smem_raw);
         __syncthreads();   // the front's shared memory is read out before the next front zeroes it
     }
 }
@@ -320,8 +469,9 @@ __global__ void __launch_bounds__(256) warp_front_kernel(SmallArgs<T> A) {
 size_t small_front_smem(int fmax, int elsize) {
     size_t ld = fmax | 1;
     size_t b = (ld * fmax * elsize + 15) & ~size_t(15);
+    b += sizeof(SKid) * SF_KIDS + 5 * SF_ITEMS;   // the staged kids, items and rows
     b += sizeof(double) * (2 * fmax + 2 * fmax);  // dd, ee (w <= f), lvec (2 f)
-    b += sizeof(int) * (fmax + fmax + 16);        // lp, ri, ctl
+    b += sizeof(int) * (fmax + 16);               // lp, ctl
     b += fmax + 16;                               // kind
     return (b + 15) & ~size_t(15);
 }
@@ -339,20 +489,22 @@ cudaError_t launch_small(int structure, const SmallArgs<T>& a, int count, int nm
         return cudaGetLastError();
     }
     size_t smem = small_front_smem(fmax, sizeof(T));
-    int threads = fmax <= 48 ? 128 : 256;
+    const bool regs = structure == STRUCT_SPD && fmax <= 96;
+    int threads = regs || fmax > 48 ? 256 : 128;
     dim3 grid(count, nmembers);
+    auto go = [&](auto kern, auto sub_kern) {
+        if (sub) sub_kern<<<grid, threads, smem, st>>>(a);
+        else kern<<<grid, threads, smem, st>>>(a);
+    };
     switch (structure) {
         case STRUCT_SPD:
-            if (sub) subtree_kernel<T, STRUCT_SPD><<<grid, threads, smem, st>>>(a);
-            else small_front_kernel<T, STRUCT_SPD><<<grid, threads, smem, st>>>(a);
+            if (fmax <= 32) go(small_front_kernel<T, STRUCT_SPD, 1>, subtree_kernel<T, STRUCT_SPD, 1>);
+            else if (fmax <= 64) go(small_front_kernel<T, STRUCT_SPD, 2>, subtree_kernel<T, STRUCT_SPD, 2>);
+            else if (regs) go(small_front_kernel<T, STRUCT_SPD, 3>, subtree_kernel<T, STRUCT_SPD, 3>);
+            else go(small_front_kernel<T, STRUCT_SPD, 0>, subtree_kernel<T, STRUCT_SPD, 0>);
             break;
-        case STRUCT_S:
-            if (sub) subtree_kernel<T, STRUCT_S><<<grid, threads, smem, st>>>(a);
-            else small_front_kernel<T, STRUCT_S><<<grid, threads, smem, st>>>(a);
-            break;
-        default:
-            if (sub) subtree_kernel<T, STRUCT_G><<<grid, threads, smem, st>>>(a);
-            else small_front_kernel<T, STRUCT_G><<<grid, threads, smem, st>>>(a);
+        case STRUCT_S: go(small_front_kernel<T, STRUCT_S, 0>, subtree_kernel<T, STRUCT_S, 0>); break;
+        default: go(small_front_kernel<T, STRUCT_G, 0>, subtree_kernel<T, STRUCT_G, 0>);
     }
     return cudaGetLastError();
 }
@@ -368,18 +520,30 @@ cudaError_t prepare_factor_kernels(int max_smem) {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
     };
-    set((const void*)small_front_kernel<double, STRUCT_SPD>);
-    set((const void*)small_front_kernel<double, STRUCT_S>);
-    set((const void*)small_front_kernel<double, STRUCT_G>);
-    set((const void*)small_front_kernel<float, STRUCT_SPD>);
-    set((const void*)small_front_kernel<float, STRUCT_S>);
-    set((const void*)small_front_kernel<float, STRUCT_G>);
-    set((const void*)subtree_kernel<double, STRUCT_SPD>);
-    set((const void*)subtree_kernel<double, STRUCT_S>);
-    set((const void*)subtree_kernel<double, STRUCT_G>);
-    set((const void*)subtree_kernel<float, STRUCT_SPD>);
-    set((const void*)subtree_kernel<float, STRUCT_S>);
-    set((const void*)subtree_kernel<float, STRUCT_G>);
+    set((const void*)small_front_kernel<double, STRUCT_SPD, 0>);
+    set((const void*)small_front_kernel<double, STRUCT_SPD, 1>);
+    set((const void*)small_front_kernel<double, STRUCT_SPD, 2>);
+    set((const void*)small_front_kernel<double, STRUCT_SPD, 3>);
+    set((const void*)small_front_kernel<double, STRUCT_S, 0>);
+    set((const void*)small_front_kernel<double, STRUCT_G, 0>);
+    set((const void*)small_front_kernel<float, STRUCT_SPD, 0>);
+    set((const void*)small_front_kernel<float, STRUCT_SPD, 1>);
+    set((const void*)small_front_kernel<float, STRUCT_SPD, 2>);
+    set((const void*)small_front_kernel<float, STRUCT_SPD, 3>);
+    set((const void*)small_front_kernel<float, STRUCT_S, 0>);
+    set((const void*)small_front_kernel<float, STRUCT_G, 0>);
+    set((const void*)subtree_kernel<double, STRUCT_SPD, 0>);
+    set((const void*)subtree_kernel<double, STRUCT_SPD, 1>);
+    set((const void*)subtree_kernel<double, STRUCT_SPD, 2>);
+    set((const void*)subtree_kernel<double, STRUCT_SPD, 3>);
+    set((const void*)subtree_kernel<double, STRUCT_S, 0>);
+    set((const void*)subtree_kernel<double, STRUCT_G, 0>);
+    set((const void*)subtree_kernel<float, STRUCT_SPD, 0>);
+    set((const void*)subtree_kernel<float, STRUCT_SPD, 1>);
+    set((const void*)subtree_kernel<float, STRUCT_SPD, 2>);
+    set((const void*)subtree_kernel<float, STRUCT_SPD, 3>);
+    set((const void*)subtree_kernel<float, STRUCT_S, 0>);
+    set((const void*)subtree_kernel<float, STRUCT_G, 0>);
     set((const void*)warp_front_kernel<double>);
     set((const void*)warp_front_kernel<float>);
     return e;

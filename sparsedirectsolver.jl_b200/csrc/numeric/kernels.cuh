@@ -11,8 +11,13 @@ template <typename T>
 struct SmallArgs {
     DeviceMaps maps;
     int32_t count;           // fronts of the launch (the warp-per-front kernel)
-    const int32_t* list;     // fronts of this launch
-    const int32_t* sub_ptr;  // fused subtrees: subtree b is list[sub_ptr[b] .. sub_ptr[b + 1]) (NULL: one
+    const int32_t* list;     // fronts of this launch (the warp-per-front kernel)
+    const SFront* sf;        // the same fronts' records, with their kids, rows and items
+    const SKid* kids;
+    const uint8_t* sri;
+    const uint32_t* items;
+    const int32_t* ep;
+    const int32_t* sub_ptr;  // fused subtrees: subtree b is sf[sub_ptr[b] .. sub_ptr[b + 1]) (NULL: one
                              // front per CTA)
     const int32_t* members;  // active batch members (NULL: 0..nmembers-1)
     const double* nzval;

@@ -7,6 +7,11 @@
 // at once: the block's rows are solved against its unit triangle (T1), then every entry takes the block's
 // products one after another (T2), by the leader and the front's helper CTAs.
 //
+// What bounds it: the chain of pivot steps, 2.2 us a column with everything (lap3d 40^3 "S": 12.0 ms over the
+// 5477 columns of the tree's wide fronts, level by level; 40^3 LU 12.2 ms; with plain remote stores and a
+// cluster barrier per step 14.4 and 14.1 ms; the cooperative kernel's two group barriers a column in global
+// memory 58.8 and 71.3 ms). The updates run at a few percent of the FP64 rate.
+//
 // Every entry receives the products of ldlt_front_steps / lu_front_steps (front_factor.cuh) in the same
 // order, each product and difference rounded on its own, and every pivot decision sees the same values, so
 // pivots, D and panels are those of the one-CTA kernel bit for bit.
@@ -153,7 +158,8 @@ __device__ __forceinline__ T pp_pick(const T (&a)[PP_NB], int x) {
 
 // --- exchanges of the leader's CTAs ---------------------------------------------------------------------------------
 // Every leader CTA sends what the others need with asynchronous stores that count into the receiver's
-// mbarrier, and waits for its own: 0.2 us for maxima and pivot row where stores and a cluster barrier took 0.7.
+// mbarrier, and waits for its own. (Stores, then a cluster barrier: 0.25 us for the barrier alone, 0.7 us with
+// the maxima and the row, whose completion the barrier's release waits for.)
 // Two mbarriers take turns: a CTA sends for the turn after next only when every CTA has finished this one.
 // Only the warps that hold rows take part. One CTA alone meets at a barrier of those warps instead.
 template <typename T, bool GEN>
@@ -302,8 +308,7 @@ struct PanelPivot {
 // that is left; st[] collects the statistics (every thread of the warps that hold rows has the same).
 //
 // A step is a chain of latencies, not of work: the maxima and the pivot row to the other CTAs, the decision,
-// a division, the update of up to 31 columns. Two thousand rows in eight CTAs take 1 us a column against 11
-// through group barriers in global memory.
+// a division, the update of up to 31 columns.
 template <typename T, int STRUCT>
 __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelPivot& pv, int k0, int64_t* st) {
     constexpr bool GEN = STRUCT == STRUCT_G;

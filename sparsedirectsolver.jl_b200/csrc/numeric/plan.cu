@@ -357,9 +357,10 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         // tiled fronts solved through inverse panels (single-system plans; batches use block chains)
         const bool pinv_mode = tune_chains == 0 && P->nbatch == 1;
         P->fsmall_max = classes.back();
-        auto class_of = [&](int f) {
+        // 0: a large front
+        auto class_of = [&](const DFront& F) {
             for (int c : classes)
-                if (f <= c) return c;
+                if (F.f <= c && F.ch_end - F.ch_begin <= SF_MAX_KIDS) return c;
             return 0;
         };
 
@@ -377,7 +378,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 std::vector<int64_t> cp(ns, 0);
                 for (int64_t s = 0; s < ns; ++s) {   // children precede parents
                     const DFront& F = P->fronts[s];
-                    cp[s] += 1 + (class_of(F.f) ? 0 : (F.w + CHOL_NB - 1) / CHOL_NB);
+                    cp[s] += 1 + (class_of(F) ? 0 : (F.w + CHOL_NB - 1) / CHOL_NB);
                     if (F.parent >= 0) cp[F.parent] = std::max(cp[F.parent], cp[s]);
                 }
                 for (int64_t s = ns - 1; s >= 0; --s) {
@@ -428,7 +429,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 const DFront& F = P->fronts[s];
                 const int64_t m = F.f - F.w;
                 cbsz[s] = (F.parent >= 0 && m > 0) ? ((m * m + 31) & ~int64_t(31)) : 0;
-                bool e = s != P->schur_front && class_of(F.f) != 0;
+                bool e = s != P->schur_front && class_of(F) != 0;
                 for (int q = F.ch_begin; q < F.ch_end; ++q) {
                     const int c = (int)(child_list[q] - 1);
                     kids[s].push_back(c);
@@ -476,7 +477,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                     base.pop_back();
                     sub_of[x] = (int)subs.size();
                     t.order.push_back(x);
-                    t.cls = std::max(t.cls, class_of(P->fronts[x].f));
+                    t.cls = std::max(t.cls, class_of(P->fronts[x]));
                     if (x != (int)s && cbsz[x] > 0) {
                         t.off.push_back(top);
                         top += cbsz[x];
@@ -531,7 +532,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         for (int64_t s = 0; s < ns; ++s) {
             DFront& F = P->fronts[s];
             F.eacol_begin = (int32_t)eacol.size();
-            if (class_of(F.f) != 0 && s != P->schur_front) continue;
+            if (class_of(F) != 0 && s != P->schur_front) continue;
             std::vector<std::vector<std::pair<int, int>>> per(F.f);
             const int nchunk = (F.f + ASM_ROWS - 1) / ASM_ROWS;
             for (int q = F.ch_begin; q < F.ch_end; ++q) {
@@ -563,6 +564,46 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
             eacol.push_back((int32_t)(ea.size() / 2));
         }
 
+        // records of the shared-memory fronts in launch order (SFront, common.cuh)
+        std::vector<SFront> sfronts;
+        std::vector<SKid> skids;
+        std::vector<uint8_t> ssri;
+        std::vector<uint32_t> sitems;
+        std::vector<int32_t> sep;
+        auto add_sfront = [&](int s) {
+            const DFront& F = P->fronts[s];
+            SFront r{};
+            r.panel = F.panel; r.cb = F.cb; r.s = s; r.f = F.f; r.w = F.w; r.c0 = F.c0;
+            r.am_begin = F.am_begin; r.am_end = F.am_end;
+            r.kid_begin = to_i32((int64_t)skids.size(), "kids");
+            r.sri_begin = to_i32((int64_t)ssri.size(), "kid rows");
+            r.ep_begin = to_i32((int64_t)sep.size(), "item starts");
+            std::vector<std::pair<uint32_t, uint32_t>> it;   // (p mod 8, p, kid) and the item
+            for (int q = F.ch_begin; q < F.ch_end; ++q) {
+                const int c = (int)child_list[q] - 1;
+                if (c < 0 || c >= ns) throw BuildError(SDSB200_INVALID_VALUE, "child_list is inconsistent with snparent");
+                const DFront& Cf = P->fronts[c];
+                const int mc = Cf.f - Cf.w;
+                if (mc <= 0 || Cf.cb < 0) continue;
+                const uint32_t kid = (uint32_t)r.nkid++;
+                skids.push_back({Cf.cb, mc, (int32_t)(ssri.size() - r.sri_begin)});
+                for (int t = 0; t < mc; ++t) {
+                    const int p = (int)relind[Cf.ri_begin + t] - 1;
+                    if (p < 0 || p >= F.f) throw BuildError(SDSB200_INVALID_VALUE, "relind out of range");
+                    ssri.push_back((uint8_t)p);
+                    it.push_back({((uint32_t)(p & 7) << 24) | ((uint32_t)p << 16) | kid, ((uint32_t)p << 24) | (kid << 8) | (uint32_t)t});
+                }
+            }
+            r.nsri = (int32_t)it.size();
+            std::sort(it.begin(), it.end());   // the kid and p fix t
+            int32_t e = 0;
+            for (uint32_t g = 0; g < 9; ++g) {
+                while (e < (int32_t)it.size() && (it[e].first >> 24) < g) ++e;
+                sep.push_back(e);
+            }
+            for (auto& x : it) sitems.push_back(x.second);
+            sfronts.push_back(r);
+        };
         // launch program of the factorization
         std::vector<int32_t> lists;
         std::vector<CholStepTask> steptasks;
@@ -629,9 +670,11 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 }
                 lists.push_back(at);
                 double tri = (P->structure == STRUCT_G) ? 1.0 : 0.5;
+                pl.sf = (int64_t)sfronts.size();
                 for (int t : kv.second)
                     for (int s : subs[t].order) {
                         lists.push_back(s);
+                        add_sfront(s);
                         const DFront& F = P->fronts[s];
                         double f = F.f, w = F.w, m = F.f - F.w;
                         for (int k = 0; k < F.w; ++k) pl.flops += (f - k) * (f - k);
@@ -656,7 +699,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
             std::vector<int> large;
             for (int s : P->level_fronts[L]) {
                 if (fstream[s] != sg || sub_of[s] >= 0) continue;
-                int c = s == P->schur_front ? 0 : class_of(P->fronts[s].f);
+                int c = s == P->schur_front ? 0 : class_of(P->fronts[s]);
                 if (c) small[c].push_back(s);
                 else large.push_back(s);
             }
@@ -678,6 +721,8 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 pl.kind = L_SMALL; pl.level = L; pl.count = (int)kv.second.size(); pl.cls = kv.first;
                 pl.list = (int64_t)lists.size();
                 lists.insert(lists.end(), kv.second.begin(), kv.second.end());
+                pl.sf = (int64_t)sfronts.size();
+                for (int s : kv.second) add_sfront(s);
                 for (int s : kv.second) {
                     const DFront& F = P->fronts[s];
                     double f = F.f, w = F.w, m = F.f - F.w;
@@ -1609,6 +1654,11 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
             }
         }
         P->d_coop_first = upload(P, coop_first, st);
+        P->d_sfronts = upload(P, sfronts, st);
+        P->d_skids = upload(P, skids, st);
+        P->d_ssri = upload(P, ssri, st);
+        P->d_sitems = upload(P, sitems, st);
+        P->d_sep = upload(P, sep, st);
         P->d_panel_jobs = upload(P, pjobs, st);
         P->d_panel_ptr = upload(P, pjob_ptr, st);
         if (P->coop_bar_len) P->d_coop_bar = dalloc<unsigned int>(P, P->coop_bar_len);

@@ -29,6 +29,7 @@ struct ProgLaunch {
     double bytes;      // algorithmic device-memory bytes of the launch
     int32_t coop = -1;      // pivot: offset of the group prefix in coop_first (-1: one CTA per front)
     int32_t coop_grid = 0;  // pivot: CTAs of the cooperative or panel launch
+    int64_t sf = 0;         // small: first record of the launch's fronts
     int32_t panel = -1;     // pivot: the panel kernel's job starts, in panel_ptr (-1: another kernel)
     int32_t panel_csize = 0;
     int32_t exact = 0;      // gemm: the contribution-block update of an LDLT / LU front, which the FP64
@@ -96,6 +97,11 @@ struct Plan {
     int64_t* d_scr_off = nullptr;
     CholStepTask* d_steptasks = nullptr; // tasks of the large-Cholesky step launches
     int32_t* d_coop_first = nullptr;   // group prefixes of the cooperative pivot launches
+    SFront* d_sfronts = nullptr;       // records of the shared-memory fronts (common.cuh)
+    SKid* d_skids = nullptr;
+    uint8_t* d_ssri = nullptr;
+    uint32_t* d_sitems = nullptr;
+    int32_t* d_sep = nullptr;
     PanelJob* d_panel_jobs = nullptr;  // the panel kernel's jobs and their starts per CTA
     int32_t* d_panel_ptr = nullptr;
     unsigned int* d_coop_bar = nullptr; // their group barrier counters
