@@ -357,10 +357,27 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         // tiled fronts solved through inverse panels (single-system plans; batches use block chains)
         const bool pinv_mode = tune_chains == 0 && P->nbatch == 1;
         P->fsmall_max = classes.back();
+        // The line between the shared-memory kernel (one CTA per front) and the large-front path (several
+        // launches, many CTAs), without tuning: 64 rows. Factorizations at 160 / 96 / 64 / 32 rows, us: lap2d
+        // 64^2 612 / 560 / 450 / 572, lap3d 40^3 "S" 17886 / 15535 / 15201 / 15357, 40^3 LU 20519 / 17489 / 16937 /
+        // 17040, lap3d 48^3 8915 / 8811 / 8918 / 9056. Cholesky fronts of up to 96 rows stay there where a
+        // launch has a CTA's front for every SM: 256 uneven systems 1681 / 1679 / 1766 / 1875, uniform batch
+        // 96^2 x 256 7094 / 5642 / 5717 / 6332. LDLT and LU batches keep every front that fits: their large
+        // fronts run on one CTA each.
+        constexpr int FSMALL_DEFAULT = 64, FSMALL_MANY = 96, FSMALL_MANY_FRONTS = 148;
+        std::vector<int64_t> level_many(P->nlevels, 0);
+        for (const DFront& F : P->fronts)
+            if (F.f > FSMALL_DEFAULT && F.f <= FSMALL_MANY) level_many[F.level] += P->nbatch;
+        const bool spd = P->structure == STRUCT_SPD;
+        auto fsmall_of = [&](const DFront& F) {
+            if (tune_fsmall || (!spd && P->nbatch > 1)) return classes.back();
+            return spd && level_many[F.level] >= FSMALL_MANY_FRONTS ? FSMALL_MANY : FSMALL_DEFAULT;
+        };
         // 0: a large front
         auto class_of = [&](const DFront& F) {
+            if (F.f > fsmall_of(F) || F.ch_end - F.ch_begin > SF_MAX_KIDS) return 0;
             for (int c : classes)
-                if (F.f <= c && F.ch_end - F.ch_begin <= SF_MAX_KIDS) return c;
+                if (F.f <= c) return c;
             return 0;
         };
 

@@ -21,7 +21,7 @@ from __future__ import annotations
 
 from .capi import tuning as make_tuning
 
-CANDIDATES = tuple((fs, wd, ch, 0, 0, sub) for fs in (0, 128, 96) for wd in (0, 64) for ch in (0, 1)
+CANDIDATES = tuple((fs, wd, ch, 0, 0, sub) for fs in (0, 160, 96) for wd in (0, 64) for ch in (0, 1)
                    for sub in (0, 4))
 
 _cache: dict = {}
