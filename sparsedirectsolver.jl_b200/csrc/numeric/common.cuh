@@ -116,6 +116,7 @@ struct PinvTile {
     int32_t neg;
     int32_t nsplit, split, slot, cnt;
 };
+constexpr double PINV_GROUP_US = 300.0;   // factorization time that a group of inverse launches covers
 constexpr int PINV_KSPLIT = 256;   // longest inner dimension of one CTA's part
 
 constexpr int FSTREAM_DEFAULT = 4;   // factorization streams of a single-system Cholesky plan

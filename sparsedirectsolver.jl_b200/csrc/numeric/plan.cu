@@ -1253,27 +1253,48 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 std::vector<PinvTile> pt;
                 auto bw_of = [](int w, int b) { return std::min(DF_BLK, w - DF_BLK * b); };
                 int64_t pwork = 0;
-                // batch "level" -1: the stream's fused subtrees
-                for (int L = -1; L < P->nlevels; ++L)
-                  for (int sg = 0; sg < P->nfstreams; ++sg) {
-                    std::vector<int> lf;
+                // Consecutive levels of a stream share their side launches (batch "level" -1: the stream's
+                // fused subtrees): a level's own dozen launches of a few fronts keep the side stream busy
+                // longer than the level takes, and it then ends long after the factorization. A group covers
+                // PINV_GROUP_US of estimated factorization time, so that the wide fronts at the top still get
+                // theirs at once and little is left at the end. Factorizations with a group per level / 100 / 300 /
+                // 1200 us, us: lap2d 300^2 2751 / 1929 / 1865 / 1860, lap3d 48^3 FP64 8874 / 7683 / 7396 / 7376, FP32
+                // 7799 / 6621 / 6008 / 6063, lap3d 40^3 "S" 15214 / 15200 / 15163 / 15274.
+                for (int sg = 0; sg < P->nfstreams; ++sg) {
+                  double us = 0;
+                  int last_level = -2;
+                  for (int64_t s = 0; s < ns; ++s)
+                    if (fstream[s] == sg) last_level = std::max(last_level, sub_of[s] >= 0 ? -1 : P->fronts[s].level);
+                  std::vector<int> lf;
+                  for (int L = -1; L <= last_level; ++L) {
+                    int here = 0, steps = 0;
+                    auto take = [&](int s) {
+                        if (fstream[s] != sg) return;
+                        lf.push_back(s);
+                        here = 1;
+                        if (!class_of(P->fronts[s])) steps = std::max(steps, (P->fronts[s].w + CHOL_NB - 1) / CHOL_NB);
+                    };
                     if (L < 0) {
                         for (int L2 = 0; L2 < P->nlevels; ++L2)
                             for (int s : P->level_fronts[L2])
-                                if (sub_of[s] >= 0) lf.push_back(s);
+                                if (sub_of[s] >= 0) take(s);
                     } else {
                         for (int s : P->level_fronts[L])
-                            if (sub_of[s] < 0) lf.push_back(s);
+                            if (sub_of[s] < 0) take(s);
                     }
-                    if (lf.empty()) continue;
+                    us += here ? 10.0 + 20.0 * steps : 0.0;
+                    if (!here || (us < PINV_GROUP_US && L < last_level)) continue;
+                    us = 0;
+                    const std::vector<int> group = std::move(lf);
+                    lf.clear();
                     std::vector<ProgLaunch>& side_b = side[{L, sg}];
                     std::vector<int> pf;   // the batch's inverse-panel fronts
                     // the warp fronts' L11^-1 in one launch per width class (8, 16, 32: the narrow
                     // kernels hold far fewer registers); the first also takes the diagonal blocks
                     std::vector<int32_t> by_w[3];
                     const int64_t blk0 = (int64_t)blk_sorted.size() / 2;
-                    for (int s : lf) {
-                        if (s == P->schur_front || fstream[s] != sg) continue;
+                    for (int s : group) {
+                        if (s == P->schur_front) continue;
                         if (!df[s].tiled) {
                             const int w = P->fronts[s].w;
                             by_w[w <= 8 ? 0 : w <= 16 ? 1 : 2].push_back(s);
@@ -1410,6 +1431,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                             }
                     }
                     push_launch(gw, 3);
+                  }
                 }
                 P->d_df_small = upload(P, small_sorted, st);
                 P->d_df_blkinv = upload(P, blk_sorted, st);
