@@ -1165,7 +1165,11 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 std::vector<int32_t> wl;
                 for (int s : P->level_fronts[L])
                     if (s != P->schur_front && !df[s].tiled) wl.push_back(s);
-                const size_t bsz = std::max<size_t>(DF_BUNDLE, (wl.size() + df_ctas - 1) / df_ctas);
+                // (a batch runs every task once per member: up to four tasks per resident CTA)
+                const size_t all = wl.size() * (size_t)P->nbatch;
+                const size_t bsz = P->nbatch > 1
+                                       ? std::min<size_t>(4 * DF_BUNDLE, std::max<size_t>(DF_BUNDLE, all / (4 * df_ctas)))
+                                       : std::max<size_t>(DF_BUNDLE, (wl.size() + df_ctas - 1) / df_ctas);
                 for (size_t o = 0; o < wl.size(); o += bsz) {
                     const int cnt = (int)std::min<size_t>(bsz, wl.size() - o);
                     tasks.push_back(DfTask{kind, (int32_t)bundles.size(), cnt, 0});

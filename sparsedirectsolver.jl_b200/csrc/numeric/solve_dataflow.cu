@@ -164,7 +164,7 @@ __device__ __forceinline__ void df_row_pull(const RowPull& rp, const int32_t* cs
 // ---------------------------------------------------------------------------------------------------
 // warp fronts (w <= 32, f <= DF_WARP_F); z: f x nrhs doubles of shared memory (ld f)
 
-template <typename T, int NR>
+template <typename T, int NR, int W, int K>
 __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, double* z, int64_t* stamp) {
     const DFront fd = A.fronts[s];
     const DfFront q = A.df[s];
@@ -174,13 +174,13 @@ __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, do
     const T* Iv = A.invf + q.inv;
     // before the children are done: the inverse row, the right-hand side of the own row, the
     // contribution lists of the lane's rows, and the panel into L2
-    double iv[DF_WARP_W];
+    double iv[W];
 #pragma unroll
-    for (int j = 0; j < DF_WARP_W; ++j) iv[j] = (lane < w && j < w) ? (double)Iv[lane + (int64_t)w * j] : 0.0;
-    double acc[4][NR];
-    RowPull rp[4];
+    for (int j = 0; j < W; ++j) iv[j] = (lane < w && j < w) ? (double)Iv[lane + (int64_t)w * j] : 0.0;
+    double acc[K][NR];
+    RowPull rp[K];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < K; ++k) {
         const int p = lane + 32 * k;
         rp[k] = p < f ? df_row_pull_prep(A.rptr, A.csrc, (int64_t)q.rbase + p) : RowPull{0, 0, {-1, -1, -1, -1}};
 #pragma unroll
@@ -192,7 +192,19 @@ __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, do
         for (int r = 0; r < NR; ++r)
             if (r < nrhs) acc[0][r] = A.in[src + r * A.ldin];
     }
-    df_prefetch_l2(L + w, (int64_t)(f * w - w) * sizeof(T), lane, 32);
+    // a narrow front's panel entries fit the registers: read now, not behind the wait
+    constexpr bool NARROW = W * K <= 16;
+    T pl[NARROW ? K : 1][NARROW ? W : 1];
+    if (NARROW) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+                pl[k % (NARROW ? K : 1)][j % (NARROW ? W : 1)] =
+                    (lane + 32 * k < m && j < w) ? L[w + lane + 32 * k + (int64_t)j * f] : T(0);
+    } else {
+        df_prefetch_l2(L + w, (int64_t)(f * w - w) * sizeof(T), lane, 32);
+    }
     if (q.fneed > 0) {
         if (lane == 0) df_wait(A.fcnt + s, (unsigned)q.fneed, A.status);
         __syncwarp();
@@ -201,10 +213,10 @@ __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, do
     // own rows z1 = b - children's updates, update rows u = sum of the children's updates (stored negated
     // like the own rows: z = -u, so that both take -= below); every row's loads before any store
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < K; ++k)
         if (lane + 32 * k < f) df_row_pull<NR>(rp[k], A.csrc, A.U, nrhs, acc[k]);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < K; ++k) {
         const int p = lane + 32 * k;
         if (p < f) {
 #pragma unroll
@@ -228,7 +240,7 @@ __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, do
 #pragma unroll
     for (int r = 0; r < NR; ++r) x[r] = 0.0;
 #pragma unroll
-    for (int j = 0; j < DF_WARP_W; ++j) {
+    for (int j = 0; j < W; ++j) {
         if (j < w) {
 #pragma unroll
             for (int r = 0; r < NR; ++r)
@@ -251,19 +263,30 @@ __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, do
     if (m > 0) {
         double* u = A.U + (int64_t)q.urow * nrhs;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < K; ++k)
 #pragma unroll
             for (int r = 0; r < NR; ++r)
                 acc[k][r] = (lane + 32 * k < m && r < nrhs) ? -z[w + lane + 32 * k + r * f] : 0.0;
-        for (int j = 0; j < w; j += 8) {
-            double lv[4][8];
+        if (NARROW) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int j = 0; j < W; ++j)
+                if (j < w) {
+#pragma unroll
+                    for (int k = 0; k < K; ++k)
+#pragma unroll
+                        for (int r = 0; r < NR; ++r)
+                            if (r < nrhs) acc[k][r] += (double)pl[k % (NARROW ? K : 1)][j % (NARROW ? W : 1)] * z[j + r * f];
+                }
+        }
+        for (int j = NARROW ? w : 0; j < w; j += 8) {
+            double lv[K][8];
+#pragma unroll
+            for (int k = 0; k < K; ++k)
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
                     lv[k][e] = (lane + 32 * k < m && j + e < w) ? (double)L[w + lane + 32 * k + (int64_t)(j + e) * f] : 0.0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < K; ++k)
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
                     if (j + e < w) {
@@ -273,7 +296,7 @@ __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, do
                     }
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < K; ++k)
             if (lane + 32 * k < m) {
 #pragma unroll
                 for (int r = 0; r < NR; ++r)
@@ -285,7 +308,7 @@ __device__ __noinline__ void df_warp_forward(const DataflowArgs<T>& A, int s, do
     __syncwarp();
 }
 
-template <typename T, int NR>
+template <typename T, int NR, int W, int K>
 __device__ __noinline__ void df_warp_backward(const DataflowArgs<T>& A, int s, double* z, int64_t* stamp) {
     const DFront fd = A.fronts[s];
     const DfFront q = A.df[s];
@@ -296,13 +319,13 @@ __device__ __noinline__ void df_warp_backward(const DataflowArgs<T>& A, int s, d
     // before the parent is done: column `lane` of the inverse (x1 = L11^-T y: x1[j] = sum_i inv[i, j]
     // y[i]), the rows of x2 this lane gathers, the first 16 entries of its panel column, and the panel
     // into L2
-    double iv[DF_WARP_W];
+    double iv[W];
 #pragma unroll
-    for (int i = 0; i < DF_WARP_W; ++i) iv[i] = (lane < w && i < w) ? (double)Iv[i + (int64_t)w * lane] : 0.0;
+    for (int i = 0; i < W; ++i) iv[i] = (lane < w && i < w) ? (double)Iv[i + (int64_t)w * lane] : 0.0;
     const int32_t* rows = A.rowval + fd.row_begin + w;
-    int32_t ridx[4];
+    int32_t ridx[K];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) ridx[k] = lane + 32 * k < m ? rows[lane + 32 * k] : 0;
+    for (int k = 0; k < K; ++k) ridx[k] = lane + 32 * k < m ? rows[lane + 32 * k] : 0;
     df_prefetch_l2(L + w, (int64_t)(f * w - w) * sizeof(T), lane, 32);
     const T* Lc = L + w + (int64_t)lane * f;
     double lv0[16];
@@ -322,7 +345,7 @@ __device__ __noinline__ void df_warp_backward(const DataflowArgs<T>& A, int s, d
     double* x2 = z;                 // m x nrhs
     double* ys = z + m * nrhs;      // w x nrhs
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < K; ++k)
         if (lane + 32 * k < m) {
 #pragma unroll
             for (int r = 0; r < NR; ++r)
@@ -359,7 +382,7 @@ __device__ __noinline__ void df_warp_backward(const DataflowArgs<T>& A, int s, d
 #pragma unroll
     for (int r = 0; r < NR; ++r) x[r] = 0.0;
 #pragma unroll
-    for (int i = 0; i < DF_WARP_W; ++i) {
+    for (int i = 0; i < W; ++i) {
         if (i < w) {
 #pragma unroll
             for (int r = 0; r < NR; ++r)
@@ -381,6 +404,105 @@ __device__ __noinline__ void df_warp_backward(const DataflowArgs<T>& A, int s, d
     __syncwarp();
     if (lane == 0) df_release(A.bdone + s, 1u);
     __syncwarp();
+}
+
+// The backward of a narrow warp front (w <= 8, f <= 32 K): lane (j, g) = (lane & 7, lane >> 3) takes the
+// update rows i = g (mod 4) of column j, all read before the parent is done, and the four partial sums
+// meet by shuffles; with one lane per column 24 of 32 lanes idled through a loop over every row.
+template <typename T, int NR, int K>
+__device__ __noinline__ void df_narrow_backward(const DataflowArgs<T>& A, int s, double* z, int64_t* stamp) {
+    constexpr int W = 8;
+    const DFront fd = A.fronts[s];
+    const DfFront q = A.df[s];
+    const int f = fd.f, w = fd.w, m = f - w, nrhs = A.nrhs, lane = threadIdx.x & 31, j = lane & 7, g = lane >> 3;
+    const int64_t n = A.n;
+    const T* L = A.facb + fd.panel;
+    const T* Iv = A.invb + q.inv;
+    T iv[W], lv[8 * K];
+#pragma unroll
+    for (int i = 0; i < W; ++i) iv[i] = (j < w && i < w) ? Iv[i + (int64_t)w * j] : T(0);
+    const int32_t* rows = A.rowval + fd.row_begin + w;
+    int32_t ridx[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) ridx[k] = lane + 32 * k < m ? rows[lane + 32 * k] : 0;
+    const T* Lc = L + w + (int64_t)j * f;
+#pragma unroll
+    for (int i = 0; i < 8 * K; ++i) lv[i] = (j < w && g + 4 * i < m) ? Lc[g + 4 * i] : T(0);
+    const int64_t dst = lane < w ? (A.reorder_bw ? A.piv[fd.c0 + lane] - 1 : fd.c0 + lane) : 0;
+    const int64_t o = lane < w ? A.perm[dst] : 0;
+    const unsigned pbsig = fd.parent >= 0 ? (unsigned)A.df[fd.parent].bsig : 0u;
+    if (lane == 0) {
+        if (fd.parent >= 0) df_wait(A.bdone + fd.parent, pbsig, A.status);
+        else df_wait(A.fcnt + s, (unsigned)(q.fneed + q.fsig), A.status);
+        if (stamp) *stamp = (int64_t)df_clock();
+    }
+    __syncwarp();
+    double y[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) y[r] = (lane < w && r < nrhs) ? df_dinv(A, A.Y, fd.c0 + lane, r) : 0.0;
+    double* x2 = z;                 // m x nrhs
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (lane + 32 * k < m) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                if (r < nrhs) x2[lane + 32 * k + r * m] = A.Y[ridx[k] + r * n];
+        }
+    __syncwarp();
+    double x[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        double acc = 0.0;
+        if (r < nrhs) {
+#pragma unroll
+            for (int i = 0; i < 8 * K; ++i)
+                if (g + 4 * i < m) acc += (double)lv[i] * x2[g + 4 * i + r * m];
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+        y[r] -= acc;                // lanes < 8: column lane
+        x[r] = 0.0;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            const double yi = __shfl_sync(0xffffffffu, y[r], i);
+            if (i < w) x[r] += (double)iv[i] * yi;
+        }
+    }
+    if (lane < w) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+            if (r < nrhs) {
+                A.Y[dst + r * n] = x[r];
+                double* op = A.out + o + r * A.ldout;
+                if (A.mode == 2) *op += x[r];
+                else *op = x[r];
+            }
+    }
+    __syncwarp();
+    if (lane == 0) df_release(A.bdone + s, 1u);
+    __syncwarp();
+}
+
+// A warp front by the instance of its size: the loops and registers of a front of 8 columns and 32 rows
+// are a fraction of a front's of 32 columns and 128 rows, and most fronts are that small. (One solve of the
+// uniform batch 96^2 x 256: 5.14 -> 3.45 ms, of 256 uneven FP32 systems 0.94 -> 0.69 ms, lap3d 48^3, 4 right-hand
+// sides, 0.90 -> 0.88 ms. Groups of 8 right-hand sides keep the wide instance: 1.64 against 1.70 ms, 40^3 LU.)
+template <typename T, int NR>
+__device__ __forceinline__ void df_warp_front(const DataflowArgs<T>& A, int s, bool forward, double* z, int64_t* stamp) {
+    const int f = A.fronts[s].f, w = A.fronts[s].w;
+    if (NR <= 4 && w <= 8 && f <= 32) {
+        if (forward) df_warp_forward<T, NR, 8, 1>(A, s, z, stamp);
+        else df_narrow_backward<T, NR, 1>(A, s, z, stamp);
+    } else if (NR <= 4 && w <= 8 && f <= 64) {
+        if (forward) df_warp_forward<T, NR, 8, 2>(A, s, z, stamp);
+        else df_narrow_backward<T, NR, 2>(A, s, z, stamp);
+    } else if (NR <= 4 && w <= 16 && f <= 64) {
+        if (forward) df_warp_forward<T, NR, 16, 2>(A, s, z, stamp);
+        else df_warp_backward<T, NR, 16, 2>(A, s, z, stamp);
+    } else {
+        if (forward) df_warp_forward<T, NR, DF_WARP_W, 4>(A, s, z, stamp);
+        else df_warp_backward<T, NR, DF_WARP_W, 4>(A, s, z, stamp);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -1096,8 +1218,7 @@ __global__ void __launch_bounds__(DF_THREADS, 2) dataflow_solve_kernel(DataflowA
                     if (i >= tk.b) break;
                     const int s = A.bundles[tk.a + i];
                     int64_t* st = i == 0 ? stamp : nullptr;
-                    if (tk.kind == DF_FW_BUNDLE) df_warp_forward<T, NR>(A, s, z, st);
-                    else df_warp_backward<T, NR>(A, s, z, st);
+                    df_warp_front<T, NR>(A, s, tk.kind == DF_FW_BUNDLE, z, st);
                 }
                 break;
             }
