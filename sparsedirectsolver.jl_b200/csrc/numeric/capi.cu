@@ -418,6 +418,8 @@ int run_factor(Plan* P, const double* nzval, double eps, double u, int pivot, in
             case L_STATS: {
                 StatsArgs a{};
                 a.stats = P->d_stats;
+                a.part = P->d_stat_part;
+                a.ticket = P->d_stat_ticket;
                 a.members = members;
                 a.super_ptr0 = P->d_super0;
                 a.perm0 = P->d_perm0;

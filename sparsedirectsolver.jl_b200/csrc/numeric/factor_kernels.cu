@@ -704,14 +704,15 @@ template cudaError_t launch_assemble_large<float>(int, const LargeAsmArgs<float>
 // ---------------------------------------------------------------------------
 // Totals of the per-front statistics and the smallest failed factor column
 // (reduce_stats! src/numeric/ldlt.jl:1276-1340, _cholesky_stats_kernel!
-// src/numeric/factorize.jl:13-45): one CTA per member, no atomics.
+// src/numeric/factorize.jl:13-45): sums of integers, the same in any order.
 __global__ void stats_kernel(StatsArgs A) {
-    const int member = A.members ? A.members[blockIdx.x] : blockIdx.x;
+    const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
     __shared__ int64_t red[NSTAT + 1][256];
+    __shared__ bool last;
     int64_t acc[NSTAT] = {0, 0, 0, 0, 0, 0};
     int64_t best = INT64_MAX;
     const int64_t* S = A.stats + (int64_t)member * A.ns * NSTAT;
-    for (int s = threadIdx.x; s < A.ns; s += blockDim.x) {
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < A.ns; s += gridDim.x * blockDim.x) {
         for (int q = 0; q < NSTAT - 1; ++q) acc[q] += S[(int64_t)s * NSTAT + q];
         int64_t fi = S[(int64_t)s * NSTAT + ST_INFO];
         if (fi != 0) {
@@ -729,6 +730,28 @@ __global__ void stats_kernel(StatsArgs A) {
         }
         __syncthreads();
     }
+    if (gridDim.x > 1) {   // the last CTA to finish adds every CTA's sums
+        int64_t* part = A.part + (int64_t)member * STATS_MAX_CTAS * (NSTAT + 1);
+        if (threadIdx.x == 0) {
+            for (int q = 0; q <= NSTAT; ++q) part[blockIdx.x * (NSTAT + 1) + q] = red[q][0];
+            __threadfence();
+            last = atomicAdd(A.ticket + member, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        if (threadIdx.x <= NSTAT) {
+            const int q = threadIdx.x;
+            int64_t v = __ldcg(part + q);
+            for (int c = 1; c < (int)gridDim.x; ++c) {
+                const int64_t x = __ldcg(part + c * (NSTAT + 1) + q);
+                v = q == NSTAT ? min(v, x) : v + x;
+            }
+            red[q][0] = v;
+        }
+        if (threadIdx.x == 0) A.ticket[member] = 0;
+        __syncthreads();
+    }
     if (threadIdx.x == 0) {
         for (int q = 0; q < NSTAT; ++q) A.totals[(int64_t)member * NSTAT + q] = red[q][0];
         int64_t b = red[NSTAT][0];
@@ -737,7 +760,9 @@ __global__ void stats_kernel(StatsArgs A) {
 }
 
 cudaError_t launch_stats(const StatsArgs& a, int nmembers, cudaStream_t st) {
-    stats_kernel<<<nmembers, 256, 0, st>>>(a);
+    // one CTA took 0.42 ms over the 136 600 fronts of 256 uneven systems, at the end of a 1.7 ms factorization
+    const int ctas = a.ns > 0 ? (a.ns + 2047) / 2048 : 1;
+    stats_kernel<<<dim3(ctas < STATS_MAX_CTAS ? ctas : STATS_MAX_CTAS, nmembers), 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 

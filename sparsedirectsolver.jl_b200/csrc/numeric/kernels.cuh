@@ -50,7 +50,10 @@ struct LargeAsmArgs {
     int64_t nnz, factor_len, cb_len;
 };
 
+constexpr int STATS_MAX_CTAS = 64;
 struct StatsArgs {
+    int64_t* part;              // STATS_MAX_CTAS x 7 partial sums per member
+    unsigned int* ticket;       // per member, zero between launches
     const int64_t* stats;
     const int32_t* members;
     const int32_t* super_ptr0;  // 0-based first column of each front

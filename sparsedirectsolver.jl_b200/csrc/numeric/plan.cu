@@ -1736,6 +1736,9 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         P->d_stats = dalloc<int64_t>(P, NSTAT * ns * nb);
         P->d_finfo = dalloc<int32_t>(P, ns * nb);
         P->d_totals = dalloc<int64_t>(P, NSTAT * nb);
+        P->d_stat_part = dalloc<int64_t>(P, STATS_MAX_CTAS * (NSTAT + 1) * nb);
+        P->d_stat_ticket = dalloc<unsigned int>(P, nb);
+        cudaMemsetAsync(P->d_stat_ticket, 0, sizeof(unsigned int) * nb, st);
         P->d_info = dalloc<int64_t>(P, nb);
         P->d_psign = dalloc<int8_t>(P, n);
         P->d_members = dalloc<int32_t>(P, nb);

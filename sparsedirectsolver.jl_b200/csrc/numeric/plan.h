@@ -82,6 +82,8 @@ struct Plan {
     int64_t* d_stats = nullptr;
     int32_t* d_finfo = nullptr;
     int64_t* d_totals = nullptr;
+    int64_t* d_stat_part = nullptr;     // the statistics reduction's partial sums and arrival counters
+    unsigned int* d_stat_ticket = nullptr;
     int64_t* d_info = nullptr;
     int8_t* d_psign = nullptr;
     int32_t* d_members = nullptr;
