@@ -6,7 +6,7 @@
 //   path (Schur updates of the fully-summed columns and of the contribution block; "lower" tiles
 //   write only on or below the diagonal; mode 2 tiles copy a deferred diagonal block). The FP32
 //   form uses the tcgen05 kernel of tc_kernels.cu.
-// * chol_step_kernel: one 32-column step of a large Cholesky front (diagonal block + trsm).
+// * chol_step_kernel: one 64-column step of a large Cholesky front (diagonal block + trsm).
 // * block_inv_kernel: inverses of the 64 x 64 diagonal blocks of the solve's wide fronts.
 // * scale_ld_kernel: W = L21 D for the contribution-block update of those fronts.
 // * gemm_nt_exact_kernel: that update in FP64 in the oracle's summation order (SIMT).
@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <stdint.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "front_factor.cuh"
@@ -311,22 +312,127 @@ cudaError_t launch_gemm(const GemmArgs<T>& a, int nmembers, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// One 32-column step of a large Cholesky front, diagonal block and trsm fused: every CTA factors the
-// 32 x 32 diagonal block (warp 0) while warps 1..3 stage its own 64-row tile of the rows below; the
-// CTA then replaces the tile by X = B L11^{-T}.
-// The diagonal block itself is read by every CTA of the step, so no CTA overwrites it: the head task
-// puts L11 in the scratch buffer and a copy tile of the next GEMM launch of the level writes it
-// into the panel (a diagonal block with no rows below is written directly by its only task).
+// One 64-column step of a large Cholesky front, diagonal block and trsm fused: every CTA factors the diagonal
+// block and replaces its own 64-row tile B of the rows below by X = B L11^{-T}. The block is read by every CTA
+// of the step, so no CTA overwrites it: the head task puts L11 in the scratch buffer and a copy tile of the
+// next GEMM launch of the level writes it into the panel (a block with no rows below is written directly by
+// its only task).
+//
+// What bounds a step is the chain of its columns. The block goes in two halves of 32 columns, each factored
+// by one warp with the rows in registers (column j + e of the row in a[e], so that the loop needs no
+// unrolling and its code stays in the instruction cache); the rows below then take one thread each.
+constexpr int CS_H = 32;              // a half
+constexpr int CS_LD = CHOL_NB + 2;    // leading dimension of the block and the tile in shared memory
+constexpr int CS_THREADS = 256;
 template <typename T>
-__global__ void __launch_bounds__(128) chol_step_kernel(CholStepArgs<T> A) {
-    // the arithmetic type is the factor's: FP32 steps compute in float (one 32-bit shuffle per value,
-    // single-precision reciprocal square root) instead of rounding double results to float
-    using CT = T;
-    constexpr int NB = CHOL_NB, LD = NB + 1, TR = 64;
-    __shared__ CT L[NB * LD];
-    __shared__ CT rdiag[NB];          // reciprocal diagonal of L11 (zero past the block)
-    __shared__ CT Bt[TR * LD];
-    __shared__ int s_status;
+struct CholStepSmem {
+    T D[CHOL_NB * CS_LD];             // the block, (i, j) at i + j CS_LD
+    T B[CHOL_NB * CS_LD];             // the tile's rows, likewise
+    T LT[CS_H][CS_H];                 // the half's columns below the diagonal: LT[j][e] = L(j + 1 + e, j)
+    T rdiag[CS_H];
+    int status;
+};
+
+template <typename T>
+__device__ __forceinline__ void cs_load2(const T* p, T& x, T& y) {
+    if constexpr (sizeof(T) == 8) {
+        const double2 v = *reinterpret_cast<const double2*>(p);
+        x = v.x; y = v.y;
+    } else {
+        const float2 v = *reinterpret_cast<const float2*>(p);
+        x = v.x; y = v.y;
+    }
+}
+
+// a[e] = a[e + 1] - x LT[e], e < N: every load before the first update
+template <int N, typename T>
+__device__ __forceinline__ void cs_shift(T (&a)[CS_H], T x, const T* lt) {
+    T u[N + (N & 1)];
+#pragma unroll
+    for (int e = 0; e < N; e += 2) cs_load2(lt + e, u[e], u[e + 1]);
+#pragma unroll
+    for (int e = 0; e < N; ++e) a[e] = a[e + 1] - x * u[e];
+}
+
+// Cholesky of columns and rows h .. h + 31 of the block by one warp, lane = row: L into D, its columns into
+// LT, the reciprocal diagonal into rdiag. Returns 0 or 1 + the half's failing column. The chain of a column is
+// its reciprocal square root and the next diagonal entry, which its own lane computes from its own l; the
+// column's way through shared memory and the other updates run beside it.
+template <typename T>
+__device__ __forceinline__ int cs_factor(CholStepSmem<T>& S, int h, T eps) {
+    const int lane = threadIdx.x & 31;
+    T a[CS_H];
+#pragma unroll
+    for (int e = 0; e < CS_H; ++e) a[e] = e <= lane ? S.D[h + lane + (h + e) * CS_LD] : T(0);
+    T ajj = __shfl_sync(0xffffffffu, a[0], 0);
+    T d = ajj > eps ? ajj : eps, r = fast_rsqrt(d);
+    int status = 0;
+    auto column = [&](int j, auto n) {
+        // a failing column is only noted (what follows it is never used): no branch in the chain
+        if (!(ajj > eps || (eps > 0 && ajj >= 0)) && status == 0) status = j + 1;
+        if (!fast_rsqrt_ok(d)) r = rsqrt(d);
+        const T l = lane == j ? d * r : a[0] * r;
+        S.LT[j][lane > j ? lane - j - 1 : CS_H - 1] = l;   // lanes <= j: the entry that is never used
+        __syncwarp();
+        ajj = __shfl_sync(0xffffffffu, a[1] - l * l, (j + 1) & 31);
+        d = ajj > eps ? ajj : eps;
+        const T rj = r;
+        r = fast_rsqrt(d);
+        cs_shift<decltype(n)::value>(a, l, S.LT[j]);       // what lands beyond column 31 is never read
+        if (lane >= j) S.D[h + lane + (h + j) * CS_LD] = l;
+        if (lane == 0) S.rdiag[j] = rj;
+    };
+    for (int j = 0; j < 8; ++j) column(j, std::integral_constant<int, 31>());
+    for (int j = 8; j < 16; ++j) column(j, std::integral_constant<int, 23>());
+    for (int j = 16; j < 24; ++j) column(j, std::integral_constant<int, 15>());
+    for (int j = 24; j < 32; ++j) column(j, std::integral_constant<int, 7>());
+    __syncwarp();
+    return status;
+}
+
+// One row by one thread: columns h .. h + 31 of M(row, .) (leading dimension CS_LD) become x with x L^T = b
+template <typename T>
+__device__ __forceinline__ void cs_solve(const CholStepSmem<T>& S, T* M, int row, int h) {
+    T a[CS_H];
+#pragma unroll
+    for (int e = 0; e < CS_H; ++e) a[e] = M[row + (h + e) * CS_LD];
+    auto column = [&](int j, auto n) {
+        const T x = a[0] * S.rdiag[j];
+        M[row + (h + j) * CS_LD] = x;
+        cs_shift<decltype(n)::value>(a, x, S.LT[j]);
+    };
+    for (int j = 0; j < 8; ++j) column(j, std::integral_constant<int, 31>());
+    for (int j = 8; j < 16; ++j) column(j, std::integral_constant<int, 23>());
+    for (int j = 16; j < 24; ++j) column(j, std::integral_constant<int, 15>());
+    for (int j = 24; j < 32; ++j) column(j, std::integral_constant<int, 7>());
+}
+
+// C(i, c) -= sum over the first half's columns of R(i, l) L21(c, l) for row i and the columns c0 .. c0 + NC - 1
+template <typename T, int NC>
+__device__ __forceinline__ void cs_update(CholStepSmem<T>& S, T* C, const T* R, int i, int c0) {
+    T acc[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] = C[i + (CS_H + c0 + c) * CS_LD];
+#pragma unroll 8
+    for (int l = 0; l < CS_H; ++l) {
+        const T x = R[i + l * CS_LD];
+#pragma unroll
+        for (int c = 0; c < NC; c += 2) {
+            T u0, u1;
+            cs_load2(&S.D[CS_H + c0 + c + l * CS_LD], u0, u1);
+            acc[c] -= x * u0;
+            acc[c + 1] -= x * u1;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) C[i + (CS_H + c0 + c) * CS_LD] = acc[c];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(CS_THREADS) chol_step_kernel(CholStepArgs<T> A) {
+    constexpr int NB = CHOL_NB, TR = 64;
+    extern __shared__ __align__(16) unsigned char cs_raw[];
+    CholStepSmem<T>& S = *reinterpret_cast<CholStepSmem<T>*>(cs_raw);
     const CholStepTask task = A.tasks[blockIdx.x];
     const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
     const int s = task.front;
@@ -337,105 +443,74 @@ __global__ void __launch_bounds__(128) chol_step_kernel(CholStepArgs<T> A) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = r1 + max(task.tile, 0) * TR;
     const int rows = task.tile >= 0 ? min(TR, f - row0) : 0;
-    if (warp == 0) {
-        // lane i holds row i of the block in registers; L[j][l] comes from lane j by shuffle, so the
-        // dependent path of a column is one shuffle, a short reduction and one reciprocal square root
-        const int i = lane;
-        CT x[NB];
+    // the block (beyond its columns: the identity) and the tile (zeros), every load before the first store
+    {
+        constexpr int U = NB * NB / CS_THREADS;
+        const int i = tid & (NB - 1), j0 = tid / NB;
+        T v[U], b[U];
 #pragma unroll
-        for (int j = 0; j < NB; ++j)
-            x[j] = (i < nbb && j < nbb && j <= i) ? P[(kb + i) + (int64_t)(kb + j) * f] : CT(0);
-        const CT eps = (CT)A.eps;
-        int status = 0;
-#pragma unroll
-        for (int j = 0; j < NB; ++j) {
-            if (j < nbb && status == 0) {
-                CT a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-#pragma unroll
-                for (int l = 0; l < j; ++l) {
-                    const CT t = x[l] * __shfl_sync(0xffffffffu, x[l], j);
-                    if ((l & 3) == 0) a0 += t;
-                    else if ((l & 3) == 1) a1 += t;
-                    else if ((l & 3) == 2) a2 += t;
-                    else a3 += t;
-                }
-                const CT sv = x[j] - ((a0 + a1) + (a2 + a3));
-                const CT ajj = __shfl_sync(0xffffffffu, sv, j);
-                if (!(ajj > eps || (eps > 0 && ajj >= 0))) {
-                    status = j + 1;
-                } else {
-                    const CT d = ajj > eps ? ajj : eps;
-                    const CT r = rsqrt(d);
-                    if (i == j) {
-                        x[j] = d * r;
-                        rdiag[j] = r;
-                    } else if (i > j && i < nbb) {
-                        x[j] = sv * r;
-                    }
-                }
-            }
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + u * (CS_THREADS / NB);
+            v[u] = (i < nbb && j <= i) ? P[(kb + i) + (int64_t)(kb + j) * f] : (i == j ? T(1) : T(0));
+            b[u] = (i < rows && j < nbb) ? P[(row0 + i) + (int64_t)(kb + j) * f] : T(0);
         }
 #pragma unroll
-        for (int j = 0; j < NB; ++j) L[i * LD + j] = x[j];
-        if (i >= nbb) rdiag[i] = CT(0);   // reciprocal diagonal beyond the block: zero
-        if (lane == 0) s_status = status;
-    } else {
-        batched_copy<8>(tid - 32, 96, TR * NB,
-                        [&](int q) {
-                            const int r = q % TR, c = q / TR;
-                            return (r < rows && c < nbb) ? (double)P[(row0 + r) + (int64_t)(kb + c) * f] : 0.0;
-                        },
-                        [&](int q, double v) { Bt[(q % TR) * LD + q / TR] = (CT)v; });
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + u * (CS_THREADS / NB);
+            S.D[i + j * CS_LD] = v[u];
+            S.B[i + j * CS_LD] = b[u];
+        }
     }
     __syncthreads();
     if (finfo[s] != 0) return;   // an earlier step of this front failed
-    const int status = s_status;
-    const bool head = task.tile <= 0;
-    if (head && tid == 0) {
-        int64_t* S = A.stats + ((int64_t)member * A.ns + s) * NSTAT;
-        if (status) {
-            finfo[s] = kb + status;
-            S[ST_NPOS] = kb + status - 1;
-            S[ST_INFO] = kb + status;
-        } else if (kb + nbb == w) {
-            S[ST_NPOS] = w;
-            S[ST_INFO] = 0;
+    const T eps = (T)A.eps;
+    int status = 0;
+    for (int h = 0; h < nbb; h += CS_H) {
+        if (warp == 0) {
+            int st = cs_factor(S, h, eps);
+            if (st && h + st > nbb) st = 0;   // never: the padding is the identity
+            if (lane == 0) S.status = st ? h + st : 0;
+        } else if (h > 0) {
+            // beside the second half's factorization: B2 -= X1 L21^T, a task of 32 rows x 8 columns per warp
+            for (int t = warp - 1; t < 8; t += CS_THREADS / 32 - 1)
+                if (32 * (t & 1) < rows) cs_update<T, 8>(S, S.B, S.B, lane + 32 * (t & 1), 8 * (t >> 1));
+        }
+        __syncthreads();
+        status = S.status;
+        if (status) break;
+        // the rows below the half: the block's second half first, then the tile's
+        if (h == 0 && nbb > CS_H && warp == 0) cs_solve(S, S.D, CS_H + lane, 0);
+        else if ((warp == 1 || warp == 2) && 32 * (warp - 1) < rows) cs_solve(S, S.B, 32 * (warp - 1) + lane, h);
+        __syncthreads();
+        if (h == 0 && nbb > CS_H) {
+            cs_update<T, 4>(S, S.D, S.D, CS_H + lane, 4 * warp);   // D22 -= L21 L21^T
+            __syncthreads();
         }
     }
+    const bool head = task.tile <= 0;
+    if (head && tid == 0) {
+        int64_t* St = A.stats + ((int64_t)member * A.ns + s) * NSTAT;
+        if (status) {
+            finfo[s] = kb + status;
+            St[ST_NPOS] = kb + status - 1;
+            St[ST_INFO] = kb + status;
+        } else if (kb + nbb == w) {
+            St[ST_NPOS] = w;
+            St[ST_INFO] = 0;
+        }
+    }
+    if (status) return;
+    const int i = tid & (NB - 1), j0 = tid / NB;
     if (head) {
         // L11 with zeros above the diagonal: the scratch (copied by the next GEMM launch), or the panel
         // when the block has no rows below it
         T* dst = task.tile < 0 ? P + kb + (int64_t)kb * f : A.scratch + (int64_t)member * A.scr_len + task.scr;
         const int64_t ld = task.tile < 0 ? f : NB;
-        for (int q = tid; q < nbb * nbb; q += blockDim.x) {
-            const int i = q % nbb, j = q / nbb;
-            dst[i + j * ld] = j <= i ? T(L[i * LD + j]) : T(0);
-        }
+        for (int j = j0; j < nbb; j += CS_THREADS / NB)
+            if (i < nbb) dst[i + j * ld] = j <= i ? S.D[i + j * CS_LD] : T(0);
     }
-    if (status || rows <= 0) return;
-    // X = B L11^{-T}: each of the first 64 threads solves its row, x L11^T = b, by forward
-    // substitution with x in registers (fully unrolled; four partial sums per entry); columns past
-    // the block have a zero reciprocal diagonal and come out zero
-    const int r = tid;
-    if (r < rows) {
-        CT x[NB];
-#pragma unroll
-        for (int j = 0; j < NB; ++j) {
-            CT a0 = Bt[r * LD + j], a1 = 0, a2 = 0, a3 = 0;
-#pragma unroll
-            for (int l = 0; l < j; ++l) {
-                const CT t = x[l] * L[j * LD + l];
-                if ((l & 3) == 0) a0 -= t;
-                else if ((l & 3) == 1) a1 -= t;
-                else if ((l & 3) == 2) a2 -= t;
-                else a3 -= t;
-            }
-            x[j] = ((a0 + a1) + (a2 + a3)) * rdiag[j];
-        }
-#pragma unroll
-        for (int j = 0; j < NB; ++j)
-            if (j < nbb) P[(row0 + r) + (int64_t)(kb + j) * f] = T(x[j]);
-    }
+    if (i < rows)
+        for (int j = j0; j < nbb; j += CS_THREADS / NB) P[(row0 + i) + (int64_t)(kb + j) * f] = S.B[i + j * CS_LD];
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -481,7 +556,7 @@ __device__ __forceinline__ void flow_dmma_64x32(int wp, int lane, double (&acc)[
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
-    for (int kk = 0; kk < CHOL_NB; kk += 4) {
+    for (int kk = 0; kk < FLOW_NB; kk += 4) {
         double av[2], bv[4];
 #pragma unroll
         for (int i = 0; i < 2; ++i) av[i] = getA(16 * wp + 8 * i + (lane >> 2), kk + (lane & 3));
@@ -538,7 +613,7 @@ __device__ __forceinline__ void flow_tile_update(T* P, int f, int r0, int c0, in
                 cv[q][p] = (i < nr && c < nc && r0 + i >= c0 + c) ? P[(r0 + i) + (int64_t)(c0 + c) * f] : T(0);
             }
 #pragma unroll 8
-        for (int l = 0; l < CHOL_NB; ++l) {
+        for (int l = 0; l < FLOW_NB; ++l) {
             T ra[4], rb[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) ra[q] = getA(tx + 16 * q, l);
@@ -564,7 +639,7 @@ __device__ __forceinline__ void flow_tile_update(T* P, int f, int r0, int c0, in
 // before the first store to shared memory.
 template <typename T>
 __device__ __forceinline__ void flow_update(const CholFlowArgs<T>& A, const FlowTask& t) {
-    constexpr int NB = CHOL_NB, TR = 64, LD = NB + 1;
+    constexpr int NB = FLOW_NB, TR = 64, LD = NB + 1;
     extern __shared__ __align__(16) unsigned char flow_dsm[];
     T* As = reinterpret_cast<T*>(flow_dsm);   // X[rows]: As[i * LD + l]
     T* Bs = As + TR * LD;                      // X[block rows]: Bs[c * LD + l]
@@ -607,7 +682,7 @@ __device__ __forceinline__ void flow_update(const CholFlowArgs<T>& A, const Flow
 template <typename T>
 __device__ __forceinline__ void flow_step(const CholFlowArgs<T>& A, const FlowTask& t) {
     using CT = T;
-    constexpr int NB = CHOL_NB, LD = NB + 1, TR = 64;
+    constexpr int NB = FLOW_NB, LD = NB + 1, TR = 64;
     __shared__ CT L[NB * LD];
     __shared__ CT rdiag[NB];          // reciprocal diagonal of L11 (zero past the block)
     __shared__ CT Bt[TR * LD];        // the tile's rows: B, then X
@@ -757,8 +832,8 @@ __global__ void __launch_bounds__(128) chol_flow_kernel(CholFlowArgs<T> A) {
         if (tid == 0) {
             if (A.trace) {
                 A.trace[4 * k] = (int64_t)flow_clock();
-                A.trace[4 * k + 3] = (int64_t)blockIdx.x | ((int64_t)t.kind << 12) | ((int64_t)(t.kb / CHOL_NB) << 16) |
-                                     ((int64_t)(t.kind == FLOW_UPD ? t.a / CHOL_NB : 0) << 28) | ((int64_t)t.front << 40);
+                A.trace[4 * k + 3] = (int64_t)blockIdx.x | ((int64_t)t.kind << 12) | ((int64_t)(t.kb / FLOW_NB) << 16) |
+                                     ((int64_t)(t.kind == FLOW_UPD ? t.a / FLOW_NB : 0) << 28) | ((int64_t)t.front << 40);
             }
             if (t.w1 >= 0) flow_wait(A.cnt + t.w1, (unsigned)t.v1, A.status);
             if (t.w2 >= 0 && t.kind != FLOW_STEPN) flow_wait(A.cnt + t.w2, (unsigned)t.v2, A.status);
@@ -768,11 +843,11 @@ __global__ void __launch_bounds__(128) chol_flow_kernel(CholFlowArgs<T> A) {
         if (t.kind == FLOW_STEP || t.kind == FLOW_STEPN) {
             flow_step<T>(A, t);
         } else if (t.kind == FLOW_COPY) {
-            const int nbb = min(CHOL_NB, t.w - t.kb);
+            const int nbb = min(FLOW_NB, t.w - t.kb);
             const T* src = A.scratch + t.scr;
             T* dst = A.factor + t.panel + t.kb + (int64_t)t.kb * t.f;
             for (int q = tid; q < nbb * nbb; q += blockDim.x)
-                dst[q % nbb + (int64_t)(q / nbb) * t.f] = src[q % nbb + (q / nbb) * CHOL_NB];
+                dst[q % nbb + (int64_t)(q / nbb) * t.f] = src[q % nbb + (q / nbb) * FLOW_NB];
         } else if (t.kind == FLOW_UPD) {
             if (A.finfo[t.front] == 0) flow_update<T>(A, t);
         }
@@ -788,7 +863,7 @@ __global__ void __launch_bounds__(128) chol_flow_kernel(CholFlowArgs<T> A) {
 
 template <typename T>
 constexpr size_t chol_flow_smem() {
-    return sizeof(T) * (64 + CHOL_NB) * (CHOL_NB + 1);
+    return sizeof(T) * (64 + FLOW_NB) * (FLOW_NB + 1);
 }
 
 template <typename T>
@@ -810,7 +885,7 @@ template <typename T>
 cudaError_t launch_chol_step(const CholStepArgs<T>& a, int nmembers, cudaStream_t st) {
     if (a.count == 0) return cudaSuccess;
     dim3 grid(a.count, nmembers);
-    chol_step_kernel<T><<<grid, 128, 0, st>>>(a);
+    chol_step_kernel<T><<<grid, CS_THREADS, sizeof(CholStepSmem<T>), st>>>(a);
     return cudaGetLastError();
 }
 
@@ -959,12 +1034,15 @@ template cudaError_t launch_block_inv<double>(const BlockInvArgs<double>&, int, 
 template cudaError_t launch_block_inv<float>(const BlockInvArgs<float>&, int, cudaStream_t);
 
 cudaError_t prepare_dense_kernels(int max_smem) {
-    (void)max_smem;   // static shared memory, but for the flow kernel's update stage
+    (void)max_smem;   // static shared memory, but for the flow kernel's update stage and the step kernel
     cudaError_t e = cudaFuncSetAttribute(chol_flow_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)chol_flow_smem<double>());
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(chol_flow_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)chol_flow_smem<float>());
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(chol_step_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(CholStepSmem<double>));
     return e;
 }
 

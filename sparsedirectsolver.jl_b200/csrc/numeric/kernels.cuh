@@ -80,7 +80,7 @@ struct CholStepTask {
     int32_t f, w;      // record before the block loads)
 };
 
-// The 32-column steps of a batch of large Cholesky fronts as dataflow in one persistent launch
+// The FLOW_NB-column steps of a batch of large Cholesky fronts as dataflow in one persistent launch
 // (single-system plans). Tasks, in list order:
 //  * STEP: the step's diagonal block (factored by every task of the step, as chol_step_kernel does) and
 //    one 64-row tile of the rows below, forward-substituted; for the front's last step;
@@ -278,7 +278,8 @@ cudaError_t launch_small_inv(const SmallInvArgs<T>& a, int nmembers, int wmax, c
                                                                                              // front (0: 32)
 cudaError_t prepare_dataflow_kernels(int max_smem);
 
-constexpr int CHOL_NB = 32;   // column block of the large-front Cholesky (one warp per diagonal block)
+constexpr int CHOL_NB = 64;   // column block of the large-front Cholesky steps
+constexpr int FLOW_NB = 32;   // column block of the dataflow steps (CholFlowArgs)
 cudaError_t prepare_factor_kernels(int max_smem);
 cudaError_t prepare_dense_kernels(int max_smem);
 cudaError_t prepare_solve_kernels(int max_smem);   // column block of the large-front Cholesky

@@ -395,7 +395,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 std::vector<int64_t> cp(ns, 0);
                 for (int64_t s = 0; s < ns; ++s) {   // children precede parents
                     const DFront& F = P->fronts[s];
-                    cp[s] += 1 + (class_of(F) ? 0 : (F.w + CHOL_NB - 1) / CHOL_NB);
+                    cp[s] += 1 + (class_of(F) ? 0 : (F.w + FLOW_NB - 1) / FLOW_NB);
                     if (F.parent >= 0) cp[F.parent] = std::max(cp[F.parent], cp[s]);
                 }
                 for (int64_t s = ns - 1; s >= 0; --s) {
@@ -773,7 +773,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 // contribution-block update. Per front: counters of the steps' tasks done (sd), of the
                 // column blocks' tiles updated by their previous step (cr), of tile 0 substituted (hd),
                 // and per (block, row tile) the steps applied (tf).
-                const int NB = CHOL_NB;
+                const int NB = FLOW_NB;
                 ProgLaunch fl{};
                 fl.kind = L_CHOL_FLOW;
                 fl.level = L;
@@ -1276,7 +1276,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                         if (fstream[s] != sg) return;
                         lf.push_back(s);
                         here = 1;
-                        if (!class_of(P->fronts[s])) steps = std::max(steps, (P->fronts[s].w + CHOL_NB - 1) / CHOL_NB);
+                        if (!class_of(P->fronts[s])) steps = std::max(steps, (P->fronts[s].w + FLOW_NB - 1) / FLOW_NB);
                     };
                     if (L < 0) {
                         for (int L2 = 0; L2 < P->nlevels; ++L2)
