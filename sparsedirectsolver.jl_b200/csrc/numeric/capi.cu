@@ -570,7 +570,8 @@ int run_dataflow(Plan* P, int nrhs, bool transpose, const double* in, int64_t ld
     a.pcnt = fl + 2 * ns + P->df_nblk;
     a.tcnt = fl + 2 * ns + 2 * (int64_t)P->df_nblk;
     a.ccnt = a.tcnt + P->df_ntcnt;
-    a.head = fl + P->df_flags_len * P->nbatch;   // one task counter after every member's flags
+    const int64_t nflags = P->df_flags_len * std::max(P->nbatch, P->df_groups);
+    a.head = fl + nflags;   // one task counter after every member's flags
     a.status = P->d_solve_status;
     a.reorder_fw = ldl || (gen && !transpose);
     a.reorder_bw = ldl || (gen && transpose);
@@ -594,8 +595,23 @@ int run_dataflow(Plan* P, int nrhs, bool transpose, const double* in, int64_t ld
     a.trace = (P->profile && P->nact == 1) ? P->d_df_trace : nullptr;
     double ent = 0.0;
     for (double v : P->level_panel_entries) ent += v;
-    for (int r0 = 0; r0 < nrhs; r0 += DF_MAX_NRHS) {
-        a.nrhs = std::min(DF_MAX_NRHS, nrhs - r0);
+    const int per_launch = DF_MAX_NRHS * P->df_groups;
+    for (int r0 = 0; r0 < nrhs; r0 += per_launch) {
+        const int here = std::min(per_launch, nrhs - r0);   // this launch's right-hand sides
+        a.nrhs = std::min(DF_MAX_NRHS, here);
+        a.nrhs_total = 0;
+        if (P->df_groups > 1 && here > DF_MAX_NRHS) {
+            a.nmembers = (here + DF_MAX_NRHS - 1) / DF_MAX_NRHS;
+            a.nrhs_total = here;
+            a.s_fac = a.s_inv = a.s_piv = a.s_d = 0;
+            a.s_in = ldin * DF_MAX_NRHS;
+            a.s_out = ldout * DF_MAX_NRHS;
+            a.s_y = P->n * DF_MAX_NRHS;
+            a.s_u = P->df_urows * DF_MAX_NRHS;
+        } else if (P->df_groups > 1) {
+            a.nmembers = 1;
+        }
+        a.trace = (P->profile && a.nmembers == 1 && P->nact == 1) ? P->d_df_trace : nullptr;
         // shared memory: per warp of a bundle f x nrhs doubles; a tiled task 2 x 64 + DF_CHUNK rows of
         // nrhs doubles; an inverse-panel forward task DF_PCOLS + 5 x 64 rows
         a.warp_smem = (int32_t)(((int64_t)P->df_fwarp_max * a.nrhs + 1) & ~int64_t(1));
@@ -606,14 +622,13 @@ int run_dataflow(Plan* P, int nrhs, bool transpose, const double* in, int64_t ld
         if (grid <= 0) return fail(SDSB200_CUDA_ERROR, "no co-resident grid for the dataflow solve");
         a.in = in + (int64_t)r0 * ldin;
         a.out = out + (int64_t)r0 * ldout;
-        CK(cudaMemsetAsync(P->d_df_flags, 0, sizeof(unsigned int) * (P->df_flags_len * P->nbatch + 1), st),
+        CK(cudaMemsetAsync(P->d_df_flags, 0, sizeof(unsigned int) * (nflags + 1), st),
            "dataflow flag reset");
         prof_begin(P, st);
         cudaError_t e = launch_dataflow_solve<T>(a, grid, smem, st);
         // algorithmic work: every stored panel entry read once per sweep (2 flops per entry and rhs
         // each way), the right-hand side read and the solution written, per member
-        prof_end(P, st, PK_FWD, 4.0 * ent * a.nrhs * P->nact,
-                 (2.0 * sizeof(T) * ent + 24.0 * P->n * a.nrhs) * P->nact);
+        prof_end(P, st, PK_FWD, 4.0 * ent * here * P->nact, (2.0 * sizeof(T) * ent + 24.0 * P->n * here) * P->nact);
         if (e != cudaSuccess) return cuda_fail(e, "dataflow solve");
     }
     return SDSB200_OK;

@@ -1126,6 +1126,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                     ur += P->fronts[s].f - P->fronts[s].w;
                     rb += P->fronts[s].f + 1;
                 }
+                P->df_urows = ur;
                 rptr.assign(rb, 0);
                 std::vector<std::pair<int32_t, int32_t>> hits;   // (front row, global update row)
                 for (int64_t s = 0; s < ns; ++s) {
@@ -1241,8 +1242,9 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
             P->d_df_rptr = upload(P, rptr, st);
             P->d_df_csrc = upload(P, csrc, st);
             P->df_part_len = std::max<int64_t>(1, std::max<int64_t>(npart, npslot) * DF_BLK * DF_MAX_NRHS);
-            P->d_df_part = dalloc<double>(P, P->df_part_len * P->nbatch);
-            P->d_df_flags = dalloc<unsigned int>(P, P->df_flags_len * P->nbatch + 1);
+            P->df_groups = P->nbatch > 1 ? 1 : std::min(DF_MAX_GROUPS, (P->max_nrhs + DF_MAX_NRHS - 1) / DF_MAX_NRHS);
+            P->d_df_part = dalloc<double>(P, P->df_part_len * std::max(P->nbatch, P->df_groups));
+            P->d_df_flags = dalloc<unsigned int>(P, P->df_flags_len * std::max(P->nbatch, P->df_groups) + 1);
             P->d_df_trace = dalloc<int64_t>(P, 6 * (int64_t)std::max<int32_t>(1, P->n_df_tasks));
             // The inverses are built level by level on the side stream, each level's right after its
             // factorization launches (single-system plans only: a batch is solved by the per-level

@@ -132,6 +132,8 @@ struct Plan {
     unsigned int* d_df_flags = nullptr; // fcnt (ns), bdone (ns), xflag (nblk), pcnt (nblk), head
     int64_t df_flags_len = 0;            // per member (the task counter follows every member's flags)
     int64_t df_part_len = 0;             // partial-product doubles per member
+    int64_t df_urows = 0;                // update rows of all fronts
+    int df_groups = 1;                   // groups of right-hand sides that one launch takes (one system)
     int32_t df_nblk = 0;
     int32_t df_ntcnt = 0, df_nccnt = 0;  // inverse panels: forward row-tile and backward column-block counters
     bool df_pinv = false;               // tiled fronts solved through their inverse panels

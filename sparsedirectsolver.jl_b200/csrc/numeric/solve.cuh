@@ -60,7 +60,8 @@ constexpr int DF_WARP_F = 128;    // tallest warp front (the plan's tuning may l
 constexpr int DF_BUNDLE = 8;      // warp fronts per task (one per warp)
 constexpr int DF_BLK = 64;        // tile rows and block columns of the tiled fronts
 constexpr int DF_CHUNK = 128;     // update rows per backward partial task
-constexpr int DF_MAX_NRHS = 8;    // right-hand sides per launch (more are solved in groups of 8)
+constexpr int DF_MAX_NRHS = 8;    // right-hand sides per group
+constexpr int DF_MAX_GROUPS = 4;  // groups of right-hand sides per launch
 constexpr int DF_THREADS = 256;
 constexpr int DF_PCOLS = 128;     // inverse panels, forward: columns per task (a 64 x 128 part of P)
 constexpr int DF_PBCOLS = 32;     // inverse panels, backward: columns per task ...
@@ -152,6 +153,9 @@ struct DataflowArgs {
     // member 0's and advance by these strides (elements)
     int32_t nmembers;
     const int32_t* members;    // the members' indices (NULL: 0 .. nmembers - 1)
+    // more than DF_MAX_NRHS right-hand sides of one system: groups of DF_MAX_NRHS as the launch's members, over
+    // one factor (a solve is latency along the tree, so the groups hide in one another); the last has the rest
+    int32_t nrhs_total;        // 0: every member has nrhs
     int64_t s_fac, s_inv, s_piv, s_d, s_in, s_out, s_y, s_u, s_part, s_flags;
 };
 

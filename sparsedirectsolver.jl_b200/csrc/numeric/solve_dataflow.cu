@@ -1159,6 +1159,7 @@ template <typename T>
 __device__ __forceinline__ void df_member_args(const DataflowArgs<T>& A, int member, DataflowArgs<T>& B) {
     B = A;
     const int64_t q = member;
+    if (A.nrhs_total > 0) B.nrhs = min(DF_MAX_NRHS, A.nrhs_total - DF_MAX_NRHS * member);
     B.facf += q * A.s_fac;
     B.facb += q * A.s_fac;
     B.invf += q * A.s_inv;
