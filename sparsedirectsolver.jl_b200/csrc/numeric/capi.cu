@@ -103,12 +103,24 @@ int prof_kind_of(LaunchKind k) {
 }
 
 // Run `body` (launches only, no host synchronization) captured as a CUDA graph on the plan's own
-// stream, replayed while `key` is unchanged. Without graphs (or when profiling) it runs eagerly.
+// stream, replayed while `key` is unchanged. Without graphs (or when profiling, or `eager`) it runs eagerly.
 template <class F>
-int run_graph(Plan* P, Plan::CachedGraph& g, const std::vector<uint64_t>& key, cudaStream_t st, F body) {
+int run_graph(Plan* P, Plan::CachedGraph& g, const std::vector<uint64_t>& key, cudaStream_t st, bool eager, F body) {
     if (!P->use_graphs || P->profile) return body(st);
+    if (eager) {
+        // calls on several streams share the plan's buffers: each waits for the last, as on the plan's own
+        // stream (a caller's capture orders its calls itself)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(st, &cap), "capture status");
+        if (cap != cudaStreamCaptureStatusNone) return body(st);
+        CK(cudaStreamWaitEvent(st, P->join_out, 0), "join");
+        const int rc = body(st);
+        CK(cudaEventRecord(P->join_out, st), "join");
+        return rc;
+    }
     CK(cudaEventRecord(P->join_in, st), "join");
     CK(cudaStreamWaitEvent(P->own, P->join_in, 0), "join");
+    CK(cudaStreamWaitEvent(P->own, P->join_out, 0), "join");
     if (!g.exec || g.key != key) {
         if (g.exec) {
             cudaGraphExecDestroy(g.exec);
@@ -592,7 +604,6 @@ int run_dataflow(Plan* P, int nrhs, bool transpose, const double* in, int64_t ld
     a.s_u = P->ulen;
     a.s_part = P->df_part_len;
     a.s_flags = P->df_flags_len;
-    a.trace = (P->profile && P->nact == 1) ? P->d_df_trace : nullptr;
     double ent = 0.0;
     for (double v : P->level_panel_entries) ent += v;
     const int per_launch = DF_MAX_NRHS * P->df_groups;
@@ -744,7 +755,11 @@ int sdsb200_factor(sdsb200_plan* plan, const double* nzval, const int8_t* h_psig
     if (interrupted(P)) return fail(SDSB200_INTERRUPTED, "interrupted by user_host_interrupt");
     std::vector<uint64_t> key = {(uint64_t)(uintptr_t)nzval, bits(eps), bits(o.pivot_threshold), (uint64_t)pivot,
                                  (uint64_t)lu_pivot, (uint64_t)P->nact, (uint64_t)P->all_members};
-    int rc = run_graph(P, P->g_factor, key, st, [&](cudaStream_t s) -> int {
+    // a first call with these buffers and options launches directly (capturing and instantiating a graph of a
+    // thousand launches takes 15 ms, the launches themselves less than the factorization); the second captures
+    const bool first = P->factor_key != key;
+    P->factor_key = key;
+    int rc = run_graph(P, P->g_factor, key, st, first && P->g_factor.key != key, [&](cudaStream_t s) -> int {
         CK(cudaMemsetAsync(P->d_finfo, 0, sizeof(int32_t) * P->ns * P->nbatch, s), "memset finfo");
         CK(cudaMemsetAsync(P->d_stats, 0, sizeof(int64_t) * NSTAT * P->ns * P->nbatch, s), "memset stats");
         return P->elsize == 8 ? run_factor<double>(P, nzval, eps, o.pivot_threshold, pivot, lu_pivot, s)
@@ -806,7 +821,9 @@ int sdsb200_solve(sdsb200_plan* plan, double* X, int64_t ldx, const double* B, i
     const uint64_t common = ((uint64_t)nrhs << 32) | ((uint64_t)transpose << 8) | ((uint64_t)P->all_members << 4);
     std::vector<uint64_t> key = {(uint64_t)(uintptr_t)X, (uint64_t)ldx, (uint64_t)(uintptr_t)B, (uint64_t)ldb, common,
                                  (uint64_t)P->nact};
-    int rc = run_graph(P, P->g_solve, key, st, [&](cudaStream_t s) -> int {
+    // the one-launch solve needs no graph: a memset and a kernel, whose buffers may be new in every call
+    const bool eager = use_persistent(P);
+    int rc = run_graph(P, P->g_solve, key, st, eager, [&](cudaStream_t s) -> int {
         if (use_persistent(P)) return run_one_launch(P, nrhs, transpose, B, ldb, X, ldx, 0, s);
         int r = permute(P, 0, B, ldb, nullptr, 0, nrhs, s);
         if (r) return r;
@@ -826,7 +843,7 @@ int sdsb200_solve(sdsb200_plan* plan, double* X, int64_t ldx, const double* B, i
         std::vector<uint64_t> rkey = key;
         rkey.push_back((uint64_t)(uintptr_t)nzval);
         rkey.push_back(check);
-        rc = run_graph(P, P->g_resid, rkey, st, [&](cudaStream_t s) -> int {
+        rc = run_graph(P, P->g_resid, rkey, st, eager, [&](cudaStream_t s) -> int {
             ResidualArgs r{};
             r.members = P->all_members ? nullptr : P->d_members;
             if (transpose) {
@@ -867,7 +884,7 @@ int sdsb200_solve(sdsb200_plan* plan, double* X, int64_t ldx, const double* B, i
             if (rel <= o.ir_tol) break;
         }
         std::vector<uint64_t> ckey = key;
-        rc = run_graph(P, P->g_corr, ckey, st, [&](cudaStream_t s) -> int {
+        rc = run_graph(P, P->g_corr, ckey, st, eager, [&](cudaStream_t s) -> int {
             if (use_persistent(P)) return run_one_launch(P, nrhs, transpose, P->d_R, P->n, X, ldx, 2, s);
             int r = permute(P, 0, P->d_R, P->n, nullptr, 0, nrhs, s);
             if (r) return r;

@@ -199,6 +199,8 @@ struct Plan {
     std::vector<int32_t> fwaits;         // per launch wait lists (ProgLaunch::wait_begin / wait_count)
     cudaEvent_t fstream_fork = nullptr;  // the extra streams start after the caller's prior work
     CachedGraph g_factor, g_solve, g_resid, g_corr;
+    std::vector<uint64_t> factor_key;    // the last factorization's buffers and options: a graph is captured
+                                         // for the second call in a row with the same
 
     bool profile = false;
     ProfAcc prof[PK_COUNT];
