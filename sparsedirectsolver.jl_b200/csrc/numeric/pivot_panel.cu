@@ -95,6 +95,19 @@ __device__ __forceinline__ void pp_load2(const float* p, float& x, float& y) {
     y = v.y;
 }
 
+// one value from global into shared memory in the background (zero when not valid)
+__device__ __forceinline__ void pp_fetch(double* s, const double* g, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g),
+                 "r"(valid ? 8 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void pp_fetch(float* s, const float* g, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g),
+                 "r"(valid ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void pp_fetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ void pp_cluster_barrier() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -105,8 +118,8 @@ __device__ __forceinline__ void pp_cluster_barrier() {
 // clears *ok (shared), as does a status word that is already set
 __device__ __forceinline__ void pp_group_barrier(unsigned int* bar, unsigned int& epoch, int gs, int32_t* status, int* ok) {
     __syncthreads();
-    epoch += gs;
     if (threadIdx.x == 0) {
+        epoch += gs;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         unsigned int v;
         for (long spins = 0;; ++spins) {

@@ -7,10 +7,11 @@
 // at once: the block's rows are solved against its unit triangle (T1), then every entry takes the block's
 // products one after another (T2), by the leader and the front's helper CTAs.
 //
-// What bounds it: the chain of pivot steps, 2.2 us a column with everything (lap3d 40^3 "S": 12.0 ms over the
-// 5477 columns of the tree's wide fronts, level by level; 40^3 LU 12.2 ms; with plain remote stores and a
-// cluster barrier per step 14.4 and 14.1 ms; the cooperative kernel's two group barriers a column in global
-// memory 58.8 and 71.3 ms). The updates run at a few percent of the FP64 rate.
+// What bounds it: the chain of pivot steps, 2 us a column with everything (lap3d 40^3 "S": 10.8 ms over the
+// 5477 columns of the tree's wide fronts, level by level; 40^3 LU 12.3 ms; with the statistics in every thread
+// and D written inside the chain 12.2 ms "S"; with plain remote stores and a cluster barrier per step 14.4 and
+// 14.1 ms; the cooperative kernel's two group barriers a column in global memory 58.8 and 71.3 ms). The
+// updates run at a few percent of the FP64 rate; T2's tiles double-buffered cost LU 14.7 ms (registers).
 //
 // Every entry receives the products of ldlt_front_steps / lu_front_steps (front_factor.cuh) in the same
 // order, each product and difference rounded on its own, and every pivot decision sees the same values, so
@@ -45,16 +46,18 @@ struct PanelSmem {
     unsigned long long sg[PP_MAXC * PP_WARPS], m1[PP_MAXC * PP_WARPS], m2[PP_MAXC * PP_WARPS];
     T sc[4];                                               // F[r, r], F[k, r], F[r, k]
     int plp, nbd, ok;
+    unsigned epoch, xn;
     int sel[2];
     int kind[PP_NB];
-    double tdk[PP_NB];
+    double tdk[PP_NB], tee[PP_NB];
+    int st[NSTAT];                                         // the statistics (thread 0 of the leader's first CTA)
     double red[PP_WARPS];
     int redi[PP_WARPS];
     PanelHdr<T> hdr;                                       // T1 / T2: the block's header
     union {
         T L[PP_NB][PP_THREADS];                            // the block: the rows' multipliers
         struct {
-            T Rs[PP_NB][PP_TR];                            // T2: the operands of a tile
+            T Rs[PP_NB][PP_TR];                            // T2: a tile's operands
             T Cs[PP_NB][PP_TC];
         };
     };
@@ -119,7 +122,7 @@ struct PanelFront {
     int gs, grank;     // the front's CTAs and this CTA's rank among them
     unsigned xn;       // exchanges of the leader's CTAs so far (the same in each)
     unsigned int* bar;
-    unsigned int epoch;
+    unsigned int* epoch;   // shared memory
     int32_t* status;
     int* ok;           // shared memory: the front's barriers have held so far
     // F[i, j], i or j < w
@@ -142,7 +145,7 @@ __device__ __forceinline__ void pp_sync(const PanelFront<T, GEN>& F) {
 // every CTA of the front meets; false once a bounded wait has given up (the same for the whole CTA)
 template <typename T, bool GEN>
 __device__ __forceinline__ bool pp_group_sync(PanelFront<T, GEN>& F) {
-    if (F.gs > F.C) pp_group_barrier(F.bar, F.epoch, F.gs, F.status, F.ok);
+    if (F.gs > F.C) pp_group_barrier(F.bar, *F.epoch, F.gs, F.status, F.ok);
     else pp_sync(F);
     return *F.ok != 0;
 }
@@ -164,24 +167,27 @@ __device__ __forceinline__ T pp_pick(const T (&a)[PP_NB], int x) {
 // Only the warps that hold rows take part. One CTA alone meets at a barrier of those warps instead.
 template <typename T, bool GEN>
 struct PanelX {
-    PanelFront<T, GEN>& F;
     PanelSmem<T>& S;
-    int nw, b;
-    __device__ PanelX(PanelFront<T, GEN>& F_, PanelSmem<T>& S_, int nw_) : F(F_), S(S_), nw(nw_), b(0) {}
+    const int C, rank, nw;
+    int b;
+    unsigned xn;
+    int32_t* const status;
+    __device__ PanelX(const PanelFront<T, GEN>& F, PanelSmem<T>& S_, int nw_)
+        : S(S_), C(F.C), rank(F.rank), nw(nw_), b(0), xn(F.xn), status(F.status) {}
     // opens the next exchange, of `bytes` bytes into each CTA
     __device__ __forceinline__ void open(int bytes) {
-        b = F.xn & 1;
-        if (F.C > 1 && threadIdx.x == 0) pp_x_arm(&S.mbar[b], bytes);
+        b = xn & 1;
+        if (C > 1 && threadIdx.x == 0) pp_x_arm(&S.mbar[b], bytes);
     }
     template <typename V>
     __device__ __forceinline__ void put(V* p, int q, V v) const {   // into CTA q's copy of *p
-        if (F.C > 1) pp_x_store(p, q, v, &S.mbar[b]);
+        if (C > 1) pp_x_store(p, q, v, &S.mbar[b]);
         else *p = v;
     }
     __device__ __forceinline__ void close() {
-        if (F.C > 1) pp_x_wait(&S.mbar[b], (F.xn >> 1) & 1, F.status);
+        if (C > 1) pp_x_wait(&S.mbar[b], (xn >> 1) & 1, status);
         else pp_warps_barrier(nw * 32);
-        F.xn++;
+        xn++;
     }
     // the warps meet: what they read before may be overwritten after, and (fence) what they wrote to global
     // memory is visible
@@ -189,10 +195,10 @@ struct PanelX {
         if (fence) __threadfence();
         __syncwarp();
         if (fence) __threadfence();
-        if (F.C > 1) {
-            open(F.C * nw * 4);
+        if (C > 1) {
+            open(C * nw * 4);
             const int lane = threadIdx.x & 31;
-            if (lane < F.C) put(&S.hi[b][F.rank * nw + (threadIdx.x >> 5)], lane, 0u);
+            if (lane < C) put(&S.hi[b][rank * nw + (threadIdx.x >> 5)], lane, 0u);
             close();
         } else {
             pp_warps_barrier(nw * 32);
@@ -217,8 +223,8 @@ struct PanelX {
             row[PP_NB] = a[PP_NB - 1];
         }
         __syncwarp();
-        if (F.C > 1) {
-            const int lane = threadIdx.x & 31, per = 32 / F.C, q = lane / per, ch = (left + 2) / 2;
+        if (C > 1) {
+            const int lane = threadIdx.x & 31, per = 32 / C, q = lane / per, ch = (left + 2) / 2;
             for (int c = lane % per; c < ch; c += per) pp_x_store2(row + 2 * c, q, row[2 * c], row[2 * c + 1], &S.mbar[b]);
         }
     }
@@ -305,20 +311,20 @@ struct PanelPivot {
 };
 
 // The pivot steps of the block that starts at column k0, by the leader's CTAs. Returns k1, the first column
-// that is left; st[] collects the statistics (every thread of the warps that hold rows has the same).
+// that is left.
 //
 // A step is a chain of latencies, not of work: the maxima and the pivot row to the other CTAs, the decision,
 // a division, the update of up to 31 columns.
 template <typename T, int STRUCT>
-__device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelPivot& pv, int k0, int64_t* st) {
+__device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelPivot& pv, int k0) {
     constexpr bool GEN = STRUCT == STRUCT_G;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int f = F.f, w = F.w, C = F.C;
+    const int f = F.f, w = F.w, C = F.C, rank = F.rank;
     const int nb = min(PP_NB, w - k0), kend = k0 + nb;
     // rows k0 .. f - 1 in one contiguous, warp-aligned chunk per CTA
     const int chunk = ((f - k0 + C - 1) / C + 31) & ~31;
     const int nw = chunk >> 5, nparts = C * nw;
-    const int orig = tid < chunk && k0 + F.rank * chunk + tid < f ? k0 + F.rank * chunk + tid : -1;
+    const int orig = tid < chunk && k0 + rank * chunk + tid < f ? k0 + rank * chunk + tid : -1;
     int rp = orig;                      // the row's place; a finished row keeps its own (<= k)
     T a[PP_NB];                         // the row's entries of columns k, k + 1, ...: the columns move down by one
                                         // with every eliminated one, so that no index depends on k
@@ -330,7 +336,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
         mylp = (orig >= 0 && orig < w) ? F.lp[orig] : 0;
     };
     load();
-    if (F.rank == 0 && tid == 0) F.hdr->ndisp = F.hdr->moved = 0;
+    if (rank == 0 && tid == 0) F.hdr->ndisp = F.hdr->moved = 0;
     if (warp < nw) {
         PanelX<T, GEN> X(F, S, nw);
         int j = 0;
@@ -339,7 +345,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
             // a bound of the column below row k, and row k itself, to every leader CTA
             X.open(nparts * 4 + X.row_bytes(left));
             unsigned h = __reduce_max_sync(0xffffffffu, rp > k ? pp_hi(a[0]) : 0u);
-            if (lane < C) X.put(&S.hi[X.b][F.rank * nw + warp], lane, h);
+            if (lane < C) X.put(&S.hi[X.b][rank * nw + warp], lane, h);
             X.row(a, rp, k, j, left);
             X.close();
             h = 0;
@@ -361,7 +367,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     pp_warp_argmax<T>(rp > k && rp < w && key <= pp_inf<T>() ? key : 0ull, ri);
                 X.open(nparts * 20);
                 if (lane < C) {
-                    const int at = F.rank * nw + warp;
+                    const int at = rank * nw + warp;
                     X.put(&S.lam[at], lane, lkey);
                     X.put(&S.mx[at], lane, mkey);
                     X.put(&S.ridx[at], lane, ri);
@@ -395,7 +401,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         unsigned long long s3 = pp_warp_max<T>(rp > k && rp != r ? pp_key(a[0]) : 0ull);
                         X.open(nparts * 24 + 3 * (int)sizeof(T));
                         if (lane < C) {
-                            const int at = F.rank * nw + warp;
+                            const int at = rank * nw + warp;
                             X.put(&S.sg[at], lane, s1);
                             X.put(&S.m2[at], lane, s2);
                             X.put(&S.m1[at], lane, s3);
@@ -440,7 +446,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     if (!acc) {
                         if (j > 0) break;                // the search needs the whole front up to date
                         X.open(8);
-                        if (F.rank == 0) {
+                        if (rank == 0) {
                             int cs = k, rs = -1;
                             pp_search(F, S, nw, k, pv.pivot, pv.u, pv.eps, bc, br, cs, rs);
                             if (tid == 0)
@@ -473,7 +479,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         if (rp == p) rp = q;
                         else if (rp == q) rp = p;
                     } else if (p != q) {                 // outside it (j = 0): the interchange in memory
-                        const int gt = F.rank * nw * 32 + tid, GT = C * nw * 32;
+                        const int gt = rank * nw * 32 + tid, GT = C * nw * 32;
                         for (int i = gt; i < f; i += GT) {
                             if (i == p || i == q) continue;
                             const T t = F.at(i, p);
@@ -506,12 +512,11 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     X.close();
                 }
             }
-            const bool lead = F.rank == 0 && tid == 0;
             if (GEN || r2 < 0) {
                 double dk = (double)S.prow[j][1];
                 int kk = KIND_1X1;
                 if (!(fabs(dk) >= pv.eps) || dk == 0.0) {
-                    if (dk == 0.0) st[ST_NZERO]++;
+                    const bool zero = dk == 0.0;
                     int lpk = 0;
                     if (!GEN) {   // the column this row is of
                         X.open(4);
@@ -523,21 +528,16 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     const int req = !GEN && pv.psign ? (int)pv.psign[pv.perm[F.c0 + lpk]] : 0;
                     dk = perturb_sign_of(dk, req) * pv.eps;
                     kk = KIND_PERTURBED;
-                    st[ST_NPERT]++;
-                    if (dk == 0.0 && st[ST_INFO] == 0) st[ST_INFO] = (GEN ? k : lpk) + 1;
-                }
-                if (!GEN) {
-                    if (dk > 0) st[ST_NPOS]++;
-                    else if (dk < 0) st[ST_NNEG]++;
-                }
-                if (lead) {
-                    F.dd[k] = dk;
-                    if (!GEN) F.ee[k] = 0.0;
-                    F.kd[k] = (signed char)kk;
+                    if (tid == 0) {
+                        S.st[ST_NZERO] += zero;
+                        S.st[ST_NPERT]++;
+                        if (dk == 0.0 && S.st[ST_INFO] == 0) S.st[ST_INFO] = (GEN ? k : lpk) + 1;
+                    }
                 }
                 if (tid == 0) {
                     S.kind[j] = kk;
                     S.tdk[j] = dk;
+                    S.tee[j] = 0.0;
                 }
                 if (rp > k) {
                     const T l = GEN ? a[0] / T(dk) : T((double)a[0] / dk);
@@ -545,16 +545,16 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     const T* row = S.prow[j] + 1;
                     // columns at and beyond `left` hold nothing any more, whatever lands in them
 #pragma unroll
-                    for (int g = 0; g < PP_NB; g += 8)
+                    for (int g = 0; g < PP_NB; g += 16)
                         if (g + 1 < left) {
+                            T u[16];   // every load before the first update
 #pragma unroll
-                            for (int e = g; e < g + 8; e += 2) {
-                                T u0, u1 = T(0);
-                                if (e + 2 < PP_NB) pp_load2(row + e + 1, u0, u1);
-                                else u0 = row[e + 1];
-                                a[e] = a[e + 1] - l * u0;
-                                if (e + 2 < PP_NB) a[e + 1] = a[e + 2] - l * u1;
-                            }
+                            for (int e = 0; e < 16; e += 2)
+                                if (g + e + 2 < PP_NB) pp_load2(row + g + e + 1, u[e], u[e + 1]);
+                                else u[e] = row[g + e + 1];
+#pragma unroll
+                            for (int e = 0; e < 16; ++e)
+                                if (g + e + 1 < PP_NB) a[g + e] = a[g + e + 1] - l * u[e];
                         }
                 }
                 j += 1;
@@ -562,18 +562,16 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                 const double fa = (double)S.prow[j][1], fb = (double)S.prow[j + 1][1], fc = (double)S.prow[j + 1][2];
                 const double det = fa * fc - fb * fb;
                 const double e11 = fc / det, e12 = -fb / det, e21 = -fb / det, e22 = fa / det;
-                st[ST_N2X2]++;
-                if (det < 0) { st[ST_NPOS]++; st[ST_NNEG]++; }
-                else if (fa > 0) st[ST_NPOS] += 2;
-                else st[ST_NNEG] += 2;
-                if (lead) {
-                    F.dd[k] = fa; F.dd[k + 1] = fc; F.ee[k] = fb; F.ee[k + 1] = 0.0;
-                    F.kd[k] = KIND_2X2_FIRST; F.kd[k + 1] = KIND_2X2_SECOND;
-                }
                 if (tid == 0) {
+                    S.st[ST_N2X2]++;
+                    if (det < 0) { S.st[ST_NPOS]++; S.st[ST_NNEG]++; }
+                    else S.st[fa > 0 ? ST_NPOS : ST_NNEG] += 2;
                     S.kind[j] = KIND_2X2_FIRST;
                     S.kind[j + 1] = KIND_2X2_SECOND;
-                    S.tdk[j] = S.tdk[j + 1] = 1.0;
+                    S.tdk[j] = fa;
+                    S.tdk[j + 1] = fc;
+                    S.tee[j] = fb;
+                    S.tee[j + 1] = 0.0;
                 }
                 if (rp == k + 1) S.L[j][tid] = T(0);
                 if (rp > k + 1) {
@@ -588,9 +586,13 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                 j += 2;
             }
         }
-        if (tid == 0) S.nbd = j;
+        if (tid == 0) {
+            S.nbd = j;
+            S.xn = X.xn;
+        }
     }
     __syncthreads();
+    F.xn = S.xn;
     const int nbd = S.nbd, k1 = k0 + nbd;
     // the multipliers and what is left of the columns out to the rows' places
     if (orig >= 0 && rp >= k1) {
@@ -614,7 +616,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
     }
     if (orig >= 0 && rp != orig) F.hdr->moved = 1;
     if (orig >= 0 && rp < w) F.lp[rp] = mylp;
-    if (F.rank == 0) {
+    if (rank == 0) {
         if (GEN)
             for (int q = tid; q < nbd * nb; q += PP_THREADS) {
                 const int t = q / nb, s = q % nb;        // row t, column s
@@ -623,11 +625,20 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
         if (tid < nbd) {
             F.hdr->kind[tid] = S.kind[tid];
             F.hdr->tdk[tid] = T(S.tdk[tid]);
+            F.dd[k0 + tid] = S.tdk[tid];
+            if (!GEN) F.ee[k0 + tid] = S.tee[tid];
+            F.kd[k0 + tid] = (signed char)S.kind[tid];
         }
+        const int kt = tid < nbd ? S.kind[tid] : 0;
+        const double dt = tid < nbd && (kt == KIND_1X1 || kt == KIND_PERTURBED) ? S.tdk[tid] : 0.0;
+        const unsigned pos = __ballot_sync(0xffffffffu, dt > 0), neg = __ballot_sync(0xffffffffu, dt < 0),
+                       two = __ballot_sync(0xffffffffu, kt == KIND_2X2_FIRST);
         if (tid == 0) {
-            int pairs = 0;
-            for (int t = 0; !GEN && t < nbd; ++t) pairs |= S.kind[t] == KIND_2X2_FIRST;
-            F.hdr->pairs = pairs;
+            if (!GEN) {
+                S.st[ST_NPOS] += __popc(pos);
+                S.st[ST_NNEG] += __popc(neg);
+            }
+            F.hdr->pairs = two != 0;
             F.hdr->k0 = k0;
             F.hdr->k1 = k1;
             F.hdr->kend = kend;
@@ -658,6 +669,26 @@ __device__ void pp_rows(const PanelFront<T, STRUCT == STRUCT_G>& F, const PanelH
             const int t = 4 * i + sub;
             g[i] = live && t < nbd ? F.at(H.moved ? H.rowmap[t] : H.k0 + t, c) : T(0);
         }
+        if (!H.pairs) {
+            for (int s = 0; s < nbd; s += 4) {
+                T l[4][NG];   // every multiplier of the four columns before the chain
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int i = 0; i < NG; ++i) l[q][i] = s + 4 * i < PP_NB ? H.lt[s + q][s + sub + 4 * i] : T(0);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const T u = __shfl_sync(0xffffffffu, g[0], (lane & ~3) + q);
+                    if (live && sub == q && s + q < nbd) F.us[(int64_t)(s + q) * f + c] = u;
+#pragma unroll
+                    for (int i = 0; i < NG; ++i)
+                        if (i > 0 || sub > q) g[i] -= l[q][i] * u;   // rows beyond nbd are never used
+                }
+#pragma unroll
+                for (int i = 0; i + 1 < NG; ++i) g[i] = g[i + 1];
+            }
+            continue;
+        }
         T u0 = T(0);   // the first of a 2x2 pair's two rows
         for (int s = 0; s < nbd; s += 4) {
 #pragma unroll
@@ -666,7 +697,7 @@ __device__ void pp_rows(const PanelFront<T, STRUCT == STRUCT_G>& F, const PanelH
                 const T u = __shfl_sync(0xffffffffu, g[0], (lane & ~3) + q);
                 if (live && sub == q) F.us[(int64_t)(s + q) * f + c] = u;
                 const T* l = &H.lt[s + q][s + sub];
-                const int kd = GEN || !H.pairs ? KIND_1X1 : H.kind[s + q];
+                const int kd = H.kind[s + q];
                 if (kd == KIND_2X2_FIRST) {
                     u0 = u;
                 } else if (kd == KIND_2X2_SECOND) {
@@ -810,9 +841,10 @@ template <typename T, int STRUCT>
 __device__ void pp_update(const PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelHdr<T>& H) {
     const int cf = STRUCT == STRUCT_G ? H.k1 : H.kend;
     if (cf >= F.w) return;
-    // 128-row tiles while every CTA has two of them, 64-row tiles below that: half the time of the last round
-    const int nt = ((F.f - H.k1 + PP_TR - 1) / PP_TR) * ((F.w - cf + PP_TC - 1) / PP_TC);
-    if (nt >= 2 * F.gs) pp_update_tiles<T, STRUCT, 4>(F, S, H);
+    // 128-row tiles (fewer operand bytes per entry) unless 64-row tiles end in fewer half rounds
+    const int sides = STRUCT == STRUCT_G ? 2 : 1, ntc = (F.w - cf + PP_TC - 1) / PP_TC, m = F.f - H.k1;
+    const int n4 = sides * ((m + PP_TR - 1) / PP_TR) * ntc, n2 = sides * ((m + PP_TR / 2 - 1) / (PP_TR / 2)) * ntc;
+    if (2 * ((n4 + F.gs - 1) / F.gs) <= (n2 + F.gs - 1) / F.gs) pp_update_tiles<T, STRUCT, 4>(F, S, H);
     else pp_update_tiles<T, STRUCT, 2>(F, S, H);
 }
 
@@ -835,12 +867,12 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
     const int s = A.list[job.fi];
     const DFront fd = A.fronts[s];
     PanelFront<T, GEN> F;
+    const int f = fd.f, w = fd.w, ncta = job.role == PANEL_SINGLE ? 1 : C;
     F.P = A.factor + fd.panel;
     F.U = GEN ? A.ufactor + fd.panel : nullptr;
-    F.f = fd.f;
-    F.w = fd.w;
+    F.f = f;
+    F.w = w;
     F.c0 = fd.c0;
-    const int f = fd.f, w = fd.w;
     double* scr = A.scratch + A.scr_off[job.fi];
     F.dd = scr;
     F.ee = scr + w;
@@ -849,19 +881,23 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
     double* h = F.ee + w + (w + 1) / 2 + (w + 7) / 8;
     F.hdr = reinterpret_cast<PanelHdr<T>*>(h);
     F.us = reinterpret_cast<T*>(h + sizeof(PanelHdr<double>) / 8 + 1);
-    F.C = job.role == PANEL_SINGLE ? 1 : C;
-    F.rank = job.rank < F.C ? job.rank : 0;
+    F.C = ncta;
+    F.rank = job.rank < ncta ? job.rank : 0;
     F.gs = job.gs;
     F.grank = job.rank;
     F.xn = xn;
     F.bar = bar + job.fi;
-    F.epoch = 0;
+    F.epoch = &S.epoch;
     F.status = status;
     F.ok = &S.ok;
-    if (threadIdx.x == 0) S.ok = 1;
+    if (threadIdx.x == 0) {
+        S.ok = 1;
+        S.epoch = 0;
+        for (int q = 0; q < NSTAT; ++q) S.st[q] = 0;
+    }
     __syncthreads();
-    const bool leads = job.rank < F.C;
-    const int tid = threadIdx.x, gt = F.grank * PP_THREADS + tid, GT = F.gs * PP_THREADS;
+    const bool leads = job.rank < ncta;
+    const int tid = threadIdx.x, gt = job.rank * PP_THREADS + tid, GT = job.gs * PP_THREADS;
     const PanelPivot pv{A.pivot, A.lu_pivot, A.u, A.eps, A.psign, A.perm};
     if (STRUCT == STRUCT_S)
         for (int64_t q = gt; q < (int64_t)w * w; q += GT) {
@@ -870,7 +906,6 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
         }
     for (int q = gt; q < w; q += GT) F.lp[q] = q;
     bool ok = pp_group_sync(F);
-    int64_t st[NSTAT] = {0, 0, 0, 0, 0, 0};
     PanelHdr<T>& H = S.hdr;
     // A barrier that gave up (a status word, no fault): helpers leave, the leader's CTAs go through the
     // blocks together without the shared phases, so that they still meet at every cluster barrier
@@ -881,7 +916,7 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
             else if (!first && ok && !leads) pp_urows<T>(F, H, F.grank - F.C, helpers);
         }
         int k1 = 0;
-        if (leads) k1 = pp_block<T, STRUCT>(F, S, pv, k, st);
+        if (leads) k1 = pp_block<T, STRUCT>(F, S, pv, k);
         if (ok) ok = pp_group_sync(F);
         if (!ok && !leads) return;
         if (ok) {
@@ -923,8 +958,8 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
     }
     if (F.grank == 0 && tid == 0) {
         int64_t* So = A.stats + (int64_t)s * NSTAT;
-        for (int q = 0; q < NSTAT; ++q) So[q] = st[q];
-        A.finfo[s] = (int32_t)st[ST_INFO];
+        for (int q = 0; q < NSTAT; ++q) So[q] = S.st[q];
+        A.finfo[s] = S.st[ST_INFO];
     }
 }
 
