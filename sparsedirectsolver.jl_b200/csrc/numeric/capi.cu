@@ -231,7 +231,6 @@ int run_factor(Plan* P, const double* nzval, double eps, double u, int pivot, in
             case L_SUBTREE: {
                 SmallArgs<T> a{};
                 a.maps = P->maps;
-                a.list = P->d_lists + (L.kind == L_SUBTREE ? L.list2 : L.list);
                 a.sf = P->d_sfronts + L.sf;
                 a.kids = P->d_skids; a.sri = P->d_ssri; a.items = P->d_sitems; a.ep = P->d_sep;
                 a.sub_ptr = L.kind == L_SUBTREE ? P->d_lists + L.list : nullptr;

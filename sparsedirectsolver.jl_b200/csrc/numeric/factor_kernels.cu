@@ -24,7 +24,10 @@
 // contribution, in child order. No atomics.
 #include <cuda_runtime.h>
 #include <math.h>
+#include <math_constants.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -33,54 +36,96 @@
 
 namespace sds {
 
+// The pivot of a Cholesky column: d = max(ajj, eps), its reciprocal square root and square root. False: it fails.
+__device__ __forceinline__ bool spd_pivot(double ajj, double eps, double& r, double& root) {
+    const bool ok = ajj > eps || (eps > 0 && ajj >= 0);
+    const double d = fmax(ajj, eps);
+    r = fast_rsqrt(d);
+    if (!fast_rsqrt_ok(d)) r = rsqrt(d);
+    root = d * r;   // and Newton's correction, off the chain of columns
+    root = d < CUDART_INF ? fma(fma(-root, root, d), 0.5 * r, root) : d;
+    return ok;
+}
+
 // The in-front Cholesky of a front of at most 32 RPL rows by eight warps, in registers: warp q holds the
 // columns p = q (mod 8), lane the rows lane + 32 i. Per column one exchange: the owner scales it by the
-// reciprocal square root and puts it in shared memory (two buffers, one barrier), and every warp updates its
-// later columns. A column costs 0.2 us, against 0.35 with the front in shared memory and three barriers.
-// Returns 0, or 1 + the column whose pivot fails.
+// reciprocal square root and puts it in shared memory (two buffers, one barrier); every warp updates its
+// later columns, the owner of the next one that column first, so that its pivot is on its way meanwhile.
+// What bounds it: that chain while few fronts are in flight, the FP64 units with many: 768 fronts of 96 rows
+// 63 us (the columns as a loop that the compiler did not unroll, the registers in local memory: 253 us; one front
+// by itself 0.35 us a column in shared memory with three barriers, 0.2 in registers). Returns 0, or 1 + the
+// column whose pivot fails.
+template <typename T, int RPL>
+struct SpdRegs {
+    static constexpr int CPW = 4 * RPL, R = 32 * RPL;
+    T (&a)[CPW][RPL];
+    const int w, lane, warp;
+    const double eps;
+    T* const lcol;
+    volatile int* const fail;
+
+    // this warp's column k in a[c]: final, and into its buffer
+    template <int c>
+    __device__ __forceinline__ void scale(int k) {
+        constexpr int i0 = (8 * c) >> 5;   // the row chunk of row k
+        double r, root;
+        if (!spd_pivot((double)__shfl_sync(0xffffffffu, a[c][i0], k & 31), eps, r, root)) {
+            if (lane == 0) fail[k & 1] = k + 1;   // read after the next barrier; the other word until then
+            return;
+        }
+        T* l = lcol + (k & 1) * R;
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+            a[c][i] *= T(r);   // rows above k are never read
+            l[lane + 32 * i] = a[c][i];
+        }
+        if (lane == (k & 31)) a[c][i0] = T(root);
+    }
+    template <int c>
+    __device__ __forceinline__ void update(const T* l, const T (&li)[RPL], int p) {
+        const T lp = l[p];
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) a[c][i] = fma(-li[i], lp, a[c][i]);
+    }
+    template <int c, int c1>
+    __device__ __forceinline__ void update_from(const T* l, const T (&li)[RPL]) {
+        if constexpr (c < c1) {
+            update<c>(l, li, 8 * c + warp);
+            update_from<c + 1, c1>(l, li);
+        }
+    }
+    // the columns n = 8 c .. : the update by column n - 1, the next pivot first (as a recursion over c: every
+    // register index is a constant)
+    template <int c>
+    __device__ __forceinline__ int columns() {
+        if constexpr (c < CPW) {
+            for (int q = 0; q < 8; ++q) {
+                const int n = 8 * c + q, k = n - 1;
+                if (n > w) return 0;
+                const T* l = lcol + (k & 1) * R;
+                T li[RPL];
+                if (c > 0 || q > 0) {
+                    __syncthreads();
+                    if (const int at = fail[k & 1]) return at;
+#pragma unroll
+                    for (int i = 0; i < RPL; ++i) li[i] = l[lane + 32 * i];
+                    if (warp >= q) update<c>(l, li, 8 * c + warp);
+                }
+                if (warp == q && n < w) scale<c>(n);
+                if (c > 0 || q > 0) update_from<c + 1, CPW>(l, li);
+            }
+            return columns<c + 1>();
+        }
+        // a front that fills the registers: its last column's pivot
+        __syncthreads();
+        return w == 8 * CPW ? fail[(w - 1) & 1] : 0;
+    }
+};
+
 template <typename T, int RPL>
 __device__ __forceinline__ int spd_front_regs(T (&a)[4 * RPL][RPL], int w, double eps, T* lcol, volatile int* fail) {
-    constexpr int CPW = 4 * RPL, R = 32 * RPL;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < CPW; ++c)
-        for (int q = 0; q < 8; ++q) {
-            const int k = 8 * c + q;
-            if (k >= w) return 0;
-            const int i0 = (8 * c) >> 5;   // the row chunk of row k
-            T* l = lcol + (k & 1) * R;
-            double d = 0.0;
-            if (warp == q) {
-                const double ajj = (double)__shfl_sync(0xffffffffu, a[c][i0], k & 31);
-                if (ajj > eps || (eps > 0 && ajj >= 0)) {
-                    d = fmax(ajj, eps);
-                    const T r = T(rsqrt(d));
-#pragma unroll
-                    for (int i = 0; i < RPL; ++i) {
-                        a[c][i] *= r;      // row k itself is set below; rows above are never read
-                        l[lane + 32 * i] = a[c][i];
-                    }
-                } else if (lane == 0) {
-                    *fail = k + 1;
-                }
-            }
-            __syncthreads();
-            if (*fail) return *fail;
-            T li[RPL];
-#pragma unroll
-            for (int i = 0; i < RPL; ++i) li[i] = l[lane + 32 * i];
-#pragma unroll
-            for (int c2 = c; c2 < CPW; ++c2) {
-                const int p = 8 * c2 + warp;
-                if (p > k) {
-                    const T lp = l[p];
-#pragma unroll
-                    for (int i = 0; i < RPL; ++i) a[c2][i] = fma(-li[i], lp, a[c2][i]);
-                }
-            }
-            if (warp == q && lane == (k & 31)) a[c][i0] = T(sqrt(d));
-        }
-    return 0;
+    SpdRegs<T, RPL> f{a, w, (int)threadIdx.x & 31, (int)threadIdx.x >> 5, eps, lcol, fail};
+    return f.template columns<0>();
 }
 
 // One front by the whole CTA, in shared memory (smem_raw holds at least small_front_smem(f)). The CTA's
@@ -368,102 +413,185 @@ __global__ void __launch_bounds__(256) subtree_kernel(SmallArgs<T> A) {
     }
 }
 
-// One Cholesky front of at most WARP_FRONT_F rows by one warp, in its own shared-memory slice F: the
-// lower triangle packed by columns (column j holds rows j .. f - 1 from offset j f - j (j - 1) / 2),
-// since a Cholesky front reads and writes nothing above its diagonal. The arithmetic of every entry is
-// small_front's, in the same order (assembly runs summed in entry order by the run's first lane;
-// children's contributions added in child order; per column the scaling by the reciprocal square
-// root and the rank-1 update in column order), so the results are bit for bit the CTA kernel's; only
-// the mapping of entries to threads differs. Batches of small systems have hundreds of thousands of
-// such fronts, and a warp per front keeps eight of them in flight per CTA instead of one; a launch of
-// few fronts keeps the CTA kernel, whose 128 threads shorten each front's chain (lap2d 64^2: 1.04
-// against 1.35 ms per factorization). Fused subtrees keep the CTA kernel too: one warp per subtree was
-// slower (1024 uneven systems: 6.79 against 5.93 ms).
+// One Cholesky front of at most WARP_FRONT_F rows by one warp: assembled in its own shared-memory slice F (the
+// lower triangle packed by columns: column j holds rows j .. f - 1 from offset j f - j (j - 1) / 2), then a row
+// per lane in registers that shift down by one column a step. The arithmetic of every entry is small_front's
+// with the front in registers, in the same order, so the results are its bit for bit. Batches of small systems
+// have hundreds of thousands of such fronts; a launch of few fronts keeps the CTA kernel, whose 256 threads
+// shorten each front's chain (lap2d 64^2 by the kernels before these: 1.04 against 1.35 ms a factorization). Fused subtrees keep the CTA
+// kernel too: one warp per subtree was slower (1024 uneven systems: 6.79 against 5.93 ms).
+//
+// What bounds it: issue slots (half of them busy; a level of 488k fronts of about 12 rows 427 us, 703 with every
+// front in 32 registers instead of 8, 16, 24 or 32 and the items by shuffles), then the dependent loads. 256
+// systems of lap2d 96^2: factorization 5.8 -> 4.4 ms with this and the registers above. One warp for 16 members
+// of a front, what they share loaded once: 1073 us for that level (neighbouring panels written far apart).
 constexpr int WARP_FRONT_F = 32;
-constexpr int WARP_FRONTS_PER_CTA = 8;
+constexpr int WARP_FRONTS_PER_CTA = 4;
 constexpr int WARP_FRONT_LEN = WARP_FRONT_F * (WARP_FRONT_F + 1) / 2;   // packed entries per warp
 constexpr int64_t WARP_FRONT_MIN_LAUNCH = 4096;   // fronts x members of a launch for the warp kernel
-
+constexpr int WARP_FRONT_U = 8;                   // columns of contributions in flight
 template <typename T>
-__device__ __forceinline__ void warp_front_spd(const SmallArgs<T>& A, const int s, const int member, T* F) {
-    const DFront fd = A.maps.fronts[s];
-    const int f = fd.f, w = fd.w, m = f - w;
-    const int lane = threadIdx.x & 31;
-    auto at = [&](int i, int j) -> T& { return F[j * f - ((j * (j - 1)) >> 1) + (i - j)]; };   // i >= j
-    const double* nz = A.nzval + (int64_t)member * A.nnz;
-    for (int q = lane; q < (f * (f + 1)) / 2; q += 32) F[q] = T(0);
-    __syncwarp();
-    for (int k = fd.am_begin + lane; k < fd.am_end; k += 32) {
-        const int code = A.maps.am_loc[k];
-        if (k > fd.am_begin && A.maps.am_loc[k - 1] == code) continue;
-        T acc = T(0);
-        for (int q = k; q < fd.am_end && A.maps.am_loc[q] == code; ++q) acc += T(nz[A.maps.am_src[q]]);
-        const int loc = (code > 0 ? code : -code) - 1;
-        const int i = loc % f, j = loc / f;
-        // (an entry above the diagonal is never read by a Cholesky front: the CTA kernel's square
-        // slice holds it unused)
-        if (code > 0 && i >= j) at(i, j) += acc;
-        else if (code < 0 && j >= i) at(j, i) += acc;
-    }
-    __syncwarp();
-    const T* cbar = A.cb + (int64_t)member * A.cb_len;
-    for (int q = fd.ch_begin; q < fd.ch_end; ++q) {
-        const DFront cd = A.maps.fronts[A.maps.child_list[q]];
-        const int mc = cd.f - cd.w;
-        if (mc <= 0 || cd.cb < 0) continue;
-        const int32_t* ri = A.maps.relind + cd.ri_begin;
-        const T* C = cbar + cd.cb;
-        for (int jj = 0; jj < mc; ++jj) {
-            const int pj = ri[jj];
-            batched_add<4, T>(jj + lane, 32, mc, [&](int ii) { return (double)C[ii + (int64_t)jj * mc]; },
-                              [&](int ii) -> T* { return &at(ri[ii], pj); });
-        }
-        __syncwarp();
-    }
-    int status = 0;
-    const double eps = A.eps;
-    for (int j = 0; j < w; ++j) {
-        const double ajj = (double)at(j, j);
-        const bool ok = ajj > eps || (eps > 0 && ajj >= 0);
-        if (!ok) { status = j + 1; break; }
-        const double djj = sqrt(fmax(ajj, eps));
-        const T inv = T(1.0 / djj);
-        __syncwarp();
-        for (int i = j + 1 + lane; i < f; i += 32) at(i, j) *= inv;
-        if (lane == 0) at(j, j) = T(djj);
-        __syncwarp();
-        for (int l = j + 1; l < f; ++l) {
-            const T flj = at(l, j);
-            for (int i = l + lane; i < f; i += 32) at(i, l) -= at(i, j) * flj;
-        }
-        __syncwarp();
-    }
-    T* P = A.factor + (int64_t)member * A.factor_len + fd.panel;
-    for (int j = 0; j < w; ++j)
-        for (int i = lane; i < f; i += 32) P[i + (int64_t)j * f] = i < j ? T(0) : at(i, j);
-    if (lane == 0) {
-        int64_t* S = A.stats + ((int64_t)member * A.ns + s) * NSTAT;
-        S[ST_NPOS] = status ? status - 1 : w;
-        for (int q = 1; q < NSTAT; ++q) S[q] = q == ST_INFO ? status : 0;
-        A.finfo[(int64_t)member * A.ns + s] = status;
-    }
-    if (fd.cb >= 0 && m > 0 && status == 0) {
-        T* C = A.cb + (int64_t)member * A.cb_len + fd.cb;
-        for (int jj = 0; jj < m; ++jj)
-            for (int ii = jj + lane; ii < m; ii += 32) C[ii + (int64_t)jj * m] = at(w + ii, w + jj);
-    }
-    __syncwarp();
+struct WarpItem {     // a column of a child's contribution: rows t .. mc - 1 at col, theirs in the front at sri
+    const T* col;
+    int sri, to;      // to: the packed place of the front's column | t << 16 | mc << 24
+};
+template <typename T>
+__host__ __device__ constexpr int warp_front_bytes() {   // a warp's shared memory: its front, 32 items
+    return WARP_FRONT_LEN * (int)sizeof(T) + 32 * (int)sizeof(WarpItem<T>);
 }
 
-// Level launches of Cholesky fronts of at most 32 rows: one warp per front, eight per CTA.
+// The assembled front F of f <= 8 G rows: factored in registers and written out. Rows above the diagonal and
+// beyond the front hold whatever shared memory held: they reach no entry of the front.
+template <typename T, int G>
+__device__ __forceinline__ void warp_front_factor(const SmallArgs<T>& A, const SFront& fd, const int member, T* F) {
+    const int f = fd.f, w = fd.w, m = f - w;
+    const int lane = threadIdx.x & 31;
+    T a[8 * G];
+    const T* Fp = F + lane;
+#pragma unroll
+    for (int p = 0; p < 8 * G; ++p) {
+        a[p] = *Fp;
+        if (p + 1 < f) Fp += f - p - 1;
+    }
+    __syncwarp();
+    // column j: lane's entry l, kept in F's place at the two buffers L[j & 1] (rows from j + 1 on)
+    T* P = A.factor + (int64_t)member * A.factor_len + fd.panel + lane;
+    int status = 0, j = 0;
+    auto column = [&](auto n) {
+        constexpr int N = decltype(n)::value;   // at least the columns that are left
+        double r, root;
+        if (!spd_pivot((double)__shfl_sync(0xffffffffu, a[0], j), A.eps, r, root)) {
+            status = j + 1;
+            return false;
+        }
+        T* L = F + (j & 1) * WARP_FRONT_F;
+        const T l = a[0] * T(r);
+        if (lane > j) L[lane - j - 1] = l;
+        if (lane < f) *P = lane < j ? T(0) : lane == j ? T(root) : l;
+        P += f;
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < N; e += 2) {
+            using T2 = std::conditional_t<sizeof(T) == 8, double2, float2>;
+            const T2 u = *reinterpret_cast<const T2*>(L + e);
+            a[e] = fma(-l, u.x, a[e + 1]);
+            if (e + 1 < N) a[e + 1] = fma(-l, u.y, a[e + 2]);
+        }
+        ++j;
+        return true;
+    };
+    if constexpr (G >= 4)
+        while (j < w && f - 1 - j > 23 && column(std::integral_constant<int, 31>())) {}
+    if constexpr (G >= 3)
+        while (status == 0 && j < w && f - 1 - j > 15 && column(std::integral_constant<int, 23>())) {}
+    if constexpr (G >= 2)
+        while (status == 0 && j < w && f - 1 - j > 7 && column(std::integral_constant<int, 15>())) {}
+    while (status == 0 && j < w && column(std::integral_constant<int, 7>())) {}
+    if (lane < NSTAT) {
+        A.stats[((int64_t)member * A.ns + fd.s) * NSTAT + lane] =
+            lane == ST_NPOS ? (status ? status - 1 : w) : lane == ST_INFO ? status : 0;
+        if (lane == 0) A.finfo[(int64_t)member * A.ns + fd.s] = status;
+    }
+    if (fd.cb >= 0 && m > 0 && status == 0) {
+        T* C = A.cb + (int64_t)member * A.cb_len + fd.cb + (lane - w);
+#pragma unroll
+        for (int e = 0; e < 8 * G; ++e) {
+            if (lane >= w + e && lane < f) *C = a[e];
+            C += m;
+        }
+    }
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256) warp_front_kernel(SmallArgs<T> A) {
+__device__ __forceinline__ void warp_front_spd(const SmallArgs<T>& A, const int at, const int member, T* F,
+                                               WarpItem<T>* items) {
+    const SFront fd = A.sf[at];
+    const int f = fd.f;
+    const int lane = threadIdx.x & 31;
+    auto column_at = [&](int j) { return j * f - ((j * (j + 1)) >> 1); };   // entry (i, j) is at column_at(j) + i
+    const double* nz = A.nzval + (int64_t)member * A.nnz;
+    const T* cbar = A.cb + (int64_t)member * A.cb_len;
+    // the loads that do not depend on one another first
+    int k = fd.am_begin + lane, code = 0, before = 0;
+    double v0 = 0.0;
+    if (k < fd.am_end) {
+        code = A.maps.am_loc[k];
+        before = k > fd.am_begin ? A.maps.am_loc[k - 1] : 0;
+        v0 = nz[A.maps.am_src[k]];
+    }
+    auto fetch = [&](int e) {   // lane: item e + lane
+        WarpItem<T> x{nullptr, 0, 255 << 16};
+        if (e + lane < fd.nsri) {
+            const uint32_t it = A.items[fd.sri_begin + e + lane];
+            const SKid kid = A.kids[fd.kid_begin + ((it >> 8) & 0xffffu)];
+            const int t = it & 0xffu;
+            x = {cbar + kid.cb + (int64_t)t * kid.mc, fd.sri_begin + kid.sri,
+                 column_at(it >> 24) | t << 16 | kid.mc << 24};
+        }
+        items[lane] = x;
+    };
+    if (fd.nsri > 0) fetch(0);
+    for (int q = lane; q < (f * (f + 1)) / 2; q += 32) F[q] = T(0);
+    __syncwarp();
+    const int inv = 65536 / f + 1;   // loc / f = loc inv >> 16 for loc < f^2 <= 1024
+    for (; k < fd.am_end; k += 32) {
+        if (k != fd.am_begin + lane) {
+            code = A.maps.am_loc[k];
+            before = A.maps.am_loc[k - 1];
+            v0 = nz[A.maps.am_src[k]];
+        }
+        if (before == code) continue;
+        T acc = T(v0);
+        for (int q = k + 1; q < fd.am_end && A.maps.am_loc[q] == code; ++q) acc += T(nz[A.maps.am_src[q]]);
+        const int loc = (code > 0 ? code : -code) - 1;
+        const int j = (loc * inv) >> 16, i = loc - j * f;
+        // (an entry above the diagonal is never read by a Cholesky front)
+        if (code > 0 && i >= j) F[column_at(j) + i] += acc;
+        else if (code < 0 && j >= i) F[column_at(i) + j] += acc;
+    }
+    __syncwarp();
+    // the children's columns by p mod 8, p and child: every entry's additions in child order
+    for (int e = 0; e < fd.nsri; e += 32) {
+        if (e > 0) {
+            fetch(e);
+            __syncwarp();
+        }
+        const int cnt = min(32, fd.nsri - e);
+        for (int u0 = 0; u0 < cnt; u0 += WARP_FRONT_U) {
+            T v[WARP_FRONT_U];
+            int to[WARP_FRONT_U];
+#pragma unroll
+            for (int u = 0; u < WARP_FRONT_U; ++u) {
+                const WarpItem<T> x = items[u0 + u];
+                to[u] = -1;
+                if (lane >= ((x.to >> 16) & 0xff) && lane < (x.to >> 24)) {
+                    v[u] = x.col[lane];
+                    to[u] = (x.to & 0xffff) + A.sri[x.sri + lane];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < WARP_FRONT_U; ++u) {
+                if (to[u] >= 0) F[to[u]] += v[u];
+                __syncwarp();
+            }
+        }
+    }
+    if (f <= 8) warp_front_factor<T, 1>(A, fd, member, F);
+    else if (f <= 16) warp_front_factor<T, 2>(A, fd, member, F);
+    else if (f <= 24) warp_front_factor<T, 3>(A, fd, member, F);
+    else warp_front_factor<T, 4>(A, fd, member, F);
+}
+
+// Level launches of Cholesky fronts of at most 32 rows: one warp per front, WARP_FRONTS_PER_CTA per CTA.
+template <typename T>
+__global__ void __launch_bounds__(32 * WARP_FRONTS_PER_CTA) warp_front_kernel(SmallArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int wi = blockIdx.x * WARP_FRONTS_PER_CTA + (threadIdx.x >> 5);
-    const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
     if (wi >= A.count) return;
-    T* F = reinterpret_cast<T*>(smem_raw) + (threadIdx.x >> 5) * WARP_FRONT_LEN;
-    warp_front_spd<T>(A, A.list[wi], member, F);
+    const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
+    unsigned char* mine = smem_raw + (threadIdx.x >> 5) * warp_front_bytes<T>();
+    warp_front_spd<T>(A, wi, member, reinterpret_cast<T*>(mine),
+                      reinterpret_cast<WarpItem<T>*>(mine + WARP_FRONT_LEN * sizeof(T)));
 }
 
 size_t small_front_smem(int fmax, int elsize) {
@@ -481,10 +609,10 @@ cudaError_t launch_small(int structure, const SmallArgs<T>& a, int count, int nm
     const bool sub = a.sub_ptr != nullptr;
     if (structure == STRUCT_SPD && fmax <= WARP_FRONT_F && !sub &&
         (int64_t)count * nmembers >= WARP_FRONT_MIN_LAUNCH) {   // a warp per front
-        const size_t wsmem = sizeof(T) * WARP_FRONTS_PER_CTA * WARP_FRONT_LEN;
-        dim3 wgrid((count + WARP_FRONTS_PER_CTA - 1) / WARP_FRONTS_PER_CTA, nmembers);
+        const size_t wsmem = (size_t)WARP_FRONTS_PER_CTA * warp_front_bytes<T>();
         SmallArgs<T> b = a;
         b.count = count;
+        dim3 wgrid((count + WARP_FRONTS_PER_CTA - 1) / WARP_FRONTS_PER_CTA, nmembers);
         warp_front_kernel<T><<<wgrid, 32 * WARP_FRONTS_PER_CTA, wsmem, st>>>(b);
         return cudaGetLastError();
     }

@@ -11,8 +11,7 @@ template <typename T>
 struct SmallArgs {
     DeviceMaps maps;
     int32_t count;           // fronts of the launch (the warp-per-front kernel)
-    const int32_t* list;     // fronts of this launch (the warp-per-front kernel)
-    const SFront* sf;        // the same fronts' records, with their kids, rows and items
+    const SFront* sf;        // the launch's fronts, with their kids, rows and items
     const SKid* kids;
     const uint8_t* sri;
     const uint32_t* items;

@@ -679,7 +679,6 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 pl.kind = L_SUBTREE; pl.level = -1; pl.cls = kv.first; pl.fstream = sg;
                 pl.count = (int)kv.second.size();
                 pl.list = (int64_t)lists.size();
-                pl.list2 = pl.list + pl.count + 1;
                 int32_t at = 0;
                 for (int t : kv.second) {
                     lists.push_back(at);
@@ -690,7 +689,6 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 pl.sf = (int64_t)sfronts.size();
                 for (int t : kv.second)
                     for (int s : subs[t].order) {
-                        lists.push_back(s);
                         add_sfront(s);
                         const DFront& F = P->fronts[s];
                         double f = F.f, w = F.w, m = F.f - F.w;
@@ -736,8 +734,6 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
             for (auto& kv : small) {
                 ProgLaunch pl{};
                 pl.kind = L_SMALL; pl.level = L; pl.count = (int)kv.second.size(); pl.cls = kv.first;
-                pl.list = (int64_t)lists.size();
-                lists.insert(lists.end(), kv.second.begin(), kv.second.end());
                 pl.sf = (int64_t)sfronts.size();
                 for (int s : kv.second) add_sfront(s);
                 for (int s : kv.second) {
