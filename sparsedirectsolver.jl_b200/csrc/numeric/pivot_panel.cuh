@@ -2,14 +2,15 @@
 //
 // A front's leader (one CTA, or one cluster whose CTAs share the rows) holds the current block of at most
 // 32 columns in registers, one row per thread, and runs the pivot steps there: per step one exchange of
-// the column's maxima and of the pivot row over distributed shared memory, one cluster barrier, and the
+// the column's maxima over distributed shared memory (the block's own rows are held by every CTA), and the
 // rank-1 (rank-2) update of the block's columns in registers. The rest of the front takes the whole block
 // at once: the block's rows are solved against its unit triangle (T1), then every entry takes the block's
 // products one after another (T2), by the leader and the front's helper CTAs.
 //
-// What bounds it: the chain of pivot steps, 2 us a column with everything (lap3d 40^3 "S": 10.8 ms over the
-// 5477 columns of the tree's wide fronts, level by level; 40^3 LU 12.3 ms; with the statistics in every thread
-// and D written inside the chain 12.2 ms "S"; with plain remote stores and a cluster barrier per step 14.4 and
+// What bounds it: the chain of pivot steps, 1.8 us a column with everything (lap3d 40^3 "S": 9.6 ms over the
+// 5477 columns of the tree's wide fronts, level by level; 40^3 LU 11.2 ms; with every pivot row sent by the CTA
+// that holds it 10.8 and 12.3 ms; with the statistics in every thread and D written inside the chain as well
+// 12.2 ms "S"; with plain remote stores and a cluster barrier per step 14.4 and
 // 14.1 ms; the cooperative kernel's two group barriers a column in global memory 58.8 and 71.3 ms). The
 // updates run at a few percent of the FP64 rate; T2's tiles double-buffered cost LU 14.7 ms (registers).
 //
@@ -163,8 +164,9 @@ __device__ __forceinline__ T pp_pick(const T (&a)[PP_NB], int x) {
 // Every leader CTA sends what the others need with asynchronous stores that count into the receiver's
 // mbarrier, and waits for its own. (Stores, then a cluster barrier: 0.25 us for the barrier alone, 0.7 us with
 // the maxima and the row, whose completion the barrier's release waits for.)
-// Two mbarriers take turns: a CTA sends for the turn after next only when every CTA has finished this one.
-// Only the warps that hold rows take part. One CTA alone meets at a barrier of those warps instead.
+// Two mbarriers take turns: a CTA sends for the turn after next only when every warp has finished this one. So
+// of two exchanges in a row, one has a part from every warp.
+// Only the warps that hold rows (or the copies, below) take part. One CTA alone meets at a barrier of those warps instead.
 template <typename T, bool GEN>
 struct PanelX {
     PanelSmem<T>& S;
@@ -205,6 +207,25 @@ struct PanelX {
         }
         if (fence) __threadfence();
     }
+    // The next exchange, of maxima, with row `pos` from the CTA's own copy: the warp that holds it (`copy`) writes
+    // the row and then opens the exchange, so whoever has waited for the maxima sees the row. Whole warps call it.
+    __device__ __forceinline__ void open_with_copy(bool copy, const T (&a)[PP_NB], int rp, int pos, int t, int left) {
+        b = xn & 1;
+        if (!copy) return;
+        if (rp == pos) write_row(a, S.prow[t], left);
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) pp_x_arm(&S.mbar[b], C * nw * 4);
+    }
+    __device__ static __forceinline__ void write_row(const T (&a)[PP_NB], T* row, int left) {
+        row[1] = a[0];
+#pragma unroll
+        for (int g = 0; g < PP_NB; g += 8)
+            if (g + 1 < left) {
+#pragma unroll
+                for (int e = g + 1; e < g + 9 && e + 1 < PP_NB; e += 2) pp_store2(row + e + 1, a[e], a[e + 1]);
+            }
+        row[PP_NB] = a[PP_NB - 1];
+    }
     // bytes of a pivot row with `left` live entries, as whole pairs
     __device__ static int row_bytes(int left) { return (left + 2) / 2 * 2 * (int)sizeof(T); }
     // The thread that holds row `pos` writes its `left` live entries to prow[t], and its warp sends them to
@@ -212,16 +233,7 @@ struct PanelX {
     __device__ __forceinline__ void row(const T (&a)[PP_NB], int rp, int pos, int t, int left) const {
         if (__ballot_sync(0xffffffffu, rp == pos) == 0) return;
         T* row = S.prow[t];
-        if (rp == pos) {
-            row[1] = a[0];
-#pragma unroll
-            for (int g = 0; g < PP_NB; g += 8)
-                if (g + 1 < left) {
-#pragma unroll
-                    for (int e = g + 1; e < g + 9 && e + 1 < PP_NB; e += 2) pp_store2(row + e + 1, a[e], a[e + 1]);
-                }
-            row[PP_NB] = a[PP_NB - 1];
-        }
+        if (rp == pos) write_row(a, row, left);
         __syncwarp();
         if (C > 1) {
             const int lane = threadIdx.x & 31, per = 32 / C, q = lane / per, ch = (left + 2) / 2;
@@ -313,7 +325,7 @@ struct PanelPivot {
 // The pivot steps of the block that starts at column k0, by the leader's CTAs. Returns k1, the first column
 // that is left.
 //
-// A step is a chain of latencies, not of work: the maxima and the pivot row to the other CTAs, the decision,
+// A step is a chain of latencies, not of work: the maxima to the other CTAs, the decision,
 // a division, the update of up to 31 columns.
 template <typename T, int STRUCT>
 __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelPivot& pv, int k0) {
@@ -323,16 +335,22 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
     const int nb = min(PP_NB, w - k0), kend = k0 + nb;
     // rows k0 .. f - 1 in one contiguous, warp-aligned chunk per CTA
     const int chunk = ((f - k0 + C - 1) / C + 31) & ~31;
-    const int nw = chunk >> 5, nparts = C * nw;
+    const int rows = chunk >> 5;
     const int orig = tid < chunk && k0 + rank * chunk + tid < f ? k0 + rank * chunk + tid : -1;
-    int rp = orig;                      // the row's place; a finished row keeps its own (<= k)
+    // Every leader CTA has a copy of the block's rows, in one warp more, and updates them like its own: the pivot
+    // row of a step never travels unless it comes from outside the block. The warp takes part in every exchange
+    // (with zeros), so that nobody is two of them ahead of it. Blocks of more than 15 warps a CTA go without.
+    const bool copies = C > 1 && rows < PP_WARPS, spare = copies && warp == rows;
+    const int nw = rows + copies, nparts = C * nw;
+    const int src = spare ? (k0 + lane < f ? k0 + lane : -1) : orig;
+    int rp = src;                       // the row's place; a finished row keeps its own (<= k)
     T a[PP_NB];                         // the row's entries of columns k, k + 1, ...: the columns move down by one
                                         // with every eliminated one, so that no index depends on k
     int mylp = 0;
     const double alpha = (1.0 + sqrt(17.0)) / 8.0;
     auto load = [&]() {
 #pragma unroll
-        for (int e = 0; e < PP_NB; ++e) a[e] = (orig >= 0 && e < nb) ? F.at(orig, k0 + e) : T(0);
+        for (int e = 0; e < PP_NB; ++e) a[e] = (src >= 0 && e < nb) ? F.at(src, k0 + e) : T(0);
         mylp = (orig >= 0 && orig < w) ? F.lp[orig] : 0;
     };
     load();
@@ -343,10 +361,11 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
         while (j < nb) {
             const int k = k0 + j, left = nb - j;   // columns k .. kend - 1
             // a bound of the column below row k, and row k itself, to every leader CTA
-            X.open(nparts * 4 + X.row_bytes(left));
-            unsigned h = __reduce_max_sync(0xffffffffu, rp > k ? pp_hi(a[0]) : 0u);
+            if (copies) X.open_with_copy(spare, a, rp, k, j, left);
+            else X.open(nparts * 4 + X.row_bytes(left));
+            unsigned h = __reduce_max_sync(0xffffffffu, rp > k && !spare ? pp_hi(a[0]) : 0u);
             if (lane < C) X.put(&S.hi[X.b][rank * nw + warp], lane, h);
-            X.row(a, rp, k, j, left);
+            if (!copies) X.row(a, rp, k, j, left);
             X.close();
             h = 0;
             for (int i = lane; i < nparts; i += 32) h = max(h, S.hi[X.b][i]);
@@ -394,7 +413,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         if (r >= kend && j > 0) break;   // the partner's column is not up to date
                         // column r: its maxima, those of column k without row r, and the corner entries
                         T v = T(0);
-                        if (rp >= k) v = r < kend ? pp_pick(a, r - k) : F.at(orig, r);
+                        if (rp >= k) v = r < kend ? pp_pick(a, r - k) : F.at(src, r);
                         const unsigned long long kv = rp >= k && rp != r ? pp_key(v) : 0ull;
                         unsigned long long s1 = pp_warp_max<T>(rp < w ? kv : 0ull);
                         unsigned long long s2 = pp_warp_max<T>(rp != k ? kv : 0ull);
@@ -406,12 +425,12 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                             X.put(&S.m2[at], lane, s2);
                             X.put(&S.m1[at], lane, s3);
                         }
-                        if (rp == r)
+                        if (rp == r && !spare)
                             for (int q = 0; q < C; ++q) {
                                 X.put(&S.sc[0], q, v);
                                 X.put(&S.sc[2], q, a[0]);
                             }
-                        if (rp == k)
+                        if (rp == k && !spare)
                             for (int q = 0; q < C; ++q) X.put(&S.sc[1], q, v);
                         X.close();
                         s1 = s2 = s3 = 0;
@@ -507,8 +526,8 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         load();
                     }
                     X.open((r2 >= 0 ? 2 : 1) * X.row_bytes(left));
-                    X.row(a, rp, k, j, left);
-                    if (r2 >= 0) X.row(a, rp, k + 1, j + 1, left);
+                    X.row(a, spare ? -1 : rp, k, j, left);
+                    if (r2 >= 0) X.row(a, spare ? -1 : rp, k + 1, j + 1, left);
                     X.close();
                 }
             }
@@ -519,8 +538,9 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     const bool zero = dk == 0.0;
                     int lpk = 0;
                     if (!GEN) {   // the column this row is of
+                        X.meet();   // (the exchange before may be one that only its sender had a part in)
                         X.open(4);
-                        if (rp == k)
+                        if (rp == k && !spare)
                             for (int q = 0; q < C; ++q) X.put(&S.plp, q, mylp);
                         X.close();
                         lpk = S.plp;
