@@ -94,10 +94,10 @@ enum LaunchKind : int32_t {
     L_SMALL = 1,       // fused small fronts (one CTA per front, front in shared memory)
     L_ASSEMBLE,        // column-task assembly of large fronts
     L_GEMM,            // grouped GEMM tiles
-    L_PIVOT_FRONT,     // large LDLT / LU: cooperative pivoting over the panel
+    L_PIVOT_FRONT,     // large LDLT / LU: the pivot steps over the panel
     L_STATS,           // statistics reduction
     L_SCALE,           // W = L21 D of large LDLT / LU fronts
-    L_CHOL_STEP,       // large Cholesky: one 32-column step (diagonal block + trsm of the rows below)
+    L_CHOL_STEP,       // large Cholesky: one 64-column step (diagonal block + trsm of the rows below)
     L_DFINV,           // diagonal-block inverses of every front for the dataflow solve
     L_PINV,            // GEMM tiles that build the inverse panels of the dataflow solve's tiled fronts
     L_CHOL_FLOW,       // large Cholesky: every 32-column step of a batch as dataflow tasks in one launch
@@ -120,7 +120,7 @@ constexpr double PINV_GROUP_US = 300.0;   // factorization time that a group of 
 constexpr int PINV_KSPLIT = 256;   // longest inner dimension of one CTA's part
 
 constexpr int FSTREAM_DEFAULT = 4;   // factorization streams of a single-system Cholesky plan
-constexpr int FSTREAM_MIN_CP = 16;   // the critical path (32-column steps) of a subtree given its own stream
+constexpr int FSTREAM_MIN_CP = 16;   // the critical path (in 32 columns) of a subtree given its own stream
 
 struct Launch {
     LaunchKind kind;

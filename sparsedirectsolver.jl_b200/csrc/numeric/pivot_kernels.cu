@@ -1,6 +1,7 @@
 // Pivoting kernels of the wide LDLT / LU fronts: the reference's in-front steps (front_factor.cuh,
 // pivot.cuh) on the global panels, by one CTA (large_pivot_kernel, batched plans) or by a group of
-// co-resident CTAs (large_pivot_coop_kernel, one-member plans).
+// co-resident CTAs (large_pivot_coop_kernel, one-member plans, where a launch has fronts of more than 8192
+// rows: pivot_panel.cuh takes the others).
 //
 // This file is compiled without floating-point contraction (--fmad=false), like the small-front
 // kernels: the reference computes a - b c as a rounded product and a rounded difference

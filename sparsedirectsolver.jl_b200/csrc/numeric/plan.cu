@@ -383,8 +383,8 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
 
         // Factorization streams (single-system Cholesky plans): the level-batched launches run per
         // (level, stream). Walking down from the roots, a front's heaviest child subtree (by its
-        // critical path of 32-column steps) stays on the front's stream and every other child subtree
-        // with a critical path of at least FSTREAM_MIN_CP steps starts a new stream while fewer than
+        // critical path in units of 32 columns) stays on the front's stream and every other child subtree
+        // with a critical path of at least FSTREAM_MIN_CP of them starts a new stream while fewer than
         // `streams` are in use, so that independent subtrees factor concurrently instead of level by
         // level. A front waits for its children on other streams through events.
         std::vector<int> fstream(ns, 0);
