@@ -612,6 +612,7 @@ int run_dataflow(Plan* P, int nrhs, bool transpose, const double* in, int64_t ld
         a.nrhs_total = 0;
         if (P->df_groups > 1 && here > DF_MAX_NRHS) {
             a.nmembers = (here + DF_MAX_NRHS - 1) / DF_MAX_NRHS;
+            a.members = nullptr;   // the groups are 0 .. nmembers - 1; the one system's factor has stride 0
             a.nrhs_total = here;
             a.s_fac = a.s_inv = a.s_piv = a.s_d = 0;
             a.s_in = ldin * DF_MAX_NRHS;
