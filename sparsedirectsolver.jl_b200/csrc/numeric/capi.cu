@@ -152,6 +152,10 @@ int run_graph(Plan* P, Plan::CachedGraph& g, const std::vector<uint64_t>& key, c
     return SDSB200_OK;
 }
 
+// The active members' indices, NULL for all of them in order: also for the only member of a one-member plan,
+// whose selection (all that a non-empty one can be) changes nothing and must not change the kernels that run
+const int32_t* member_list(const Plan* P) { return P->all_members || P->nbatch == 1 ? nullptr : P->d_members; }
+
 uint64_t bits(double x) {
     uint64_t u;
     memcpy(&u, &x, sizeof(u));
@@ -178,7 +182,7 @@ __global__ void absmax_kernel(const double* x, int64_t len, double* out) {
 template <typename T>
 int run_factor(Plan* P, const double* nzval, double eps, double u, int pivot, int lu_pivot, cudaStream_t st) {
     const int nm = P->nact;
-    const int32_t* members = P->all_members ? nullptr : P->d_members;
+    const int32_t* members = member_list(P);
     T* factor = static_cast<T*>(P->d_factor);
     T* ufactor = static_cast<T*>(P->d_ufactor);
     T* cb = static_cast<T*>(P->d_cb);
@@ -458,7 +462,7 @@ template <typename T>
 // last level) is only pulled into by the forward sweep and skipped by the backward one.
 int run_sweeps(Plan* P, int nrhs, bool transpose, cudaStream_t st, int which) {
     const int nm = P->nact;
-    const int32_t* members = P->all_members ? nullptr : P->d_members;
+    const int32_t* members = member_list(P);
     const bool gen = P->structure == STRUCT_G, ldl = P->structure == STRUCT_S;
     const T* factor = static_cast<const T*>(P->d_factor);
     const T* ufactor = static_cast<const T*>(P->d_ufactor);
@@ -592,7 +596,7 @@ int run_dataflow(Plan* P, int nrhs, bool transpose, const double* in, int64_t ld
     a.ldout = ldout;
     // batch members: every task once per active member, member-dependent arrays by stride
     a.nmembers = P->nact;
-    a.members = P->all_members ? nullptr : P->d_members;
+    a.members = member_list(P);
     a.s_fac = P->factor_len;
     a.s_inv = P->df_inv_len;
     a.s_piv = P->n;
@@ -663,7 +667,7 @@ int sweeps(Plan* P, int nrhs, bool transpose, cudaStream_t st, int which = 7) {
 int permute(Plan* P, int mode, const double* in, int64_t ldin, double* out, int64_t ldout, int nrhs, cudaStream_t st,
             bool identity = false) {
     PermArgs a{};
-    a.members = P->all_members ? nullptr : P->d_members;
+    a.members = member_list(P);
     a.perm = identity ? nullptr : P->d_perm0;
     a.Y = P->d_Y;
     a.in = in; a.out = out; a.ldin = ldin; a.ldout = ldout;
@@ -845,7 +849,7 @@ int sdsb200_solve(sdsb200_plan* plan, double* X, int64_t ldx, const double* B, i
         rkey.push_back(check);
         rc = run_graph(P, P->g_resid, rkey, st, eager, [&](cudaStream_t s) -> int {
             ResidualArgs r{};
-            r.members = P->all_members ? nullptr : P->d_members;
+            r.members = member_list(P);
             if (transpose) {
                 r.rowptr = P->d_fullT_rowptr; r.colval = P->d_fullT_colval; r.srcptr = P->d_fullT_srcptr;
                 r.src = P->d_fullT_src;
@@ -1159,7 +1163,7 @@ extern "C" int sdsb200_residual(sdsb200_plan* plan, double* R, const double* X, 
     if (solve_mode < 0 || solve_mode > 2) return fail(SDSB200_INVALID_VALUE, "solve_mode must be 0, 1 or 2");
     const bool transpose = P->structure == STRUCT_G && solve_mode != 0;
     ResidualArgs r{};
-    r.members = P->all_members ? nullptr : P->d_members;
+    r.members = member_list(P);
     if (transpose) {
         r.rowptr = P->d_fullT_rowptr; r.colval = P->d_fullT_colval; r.srcptr = P->d_fullT_srcptr; r.src = P->d_fullT_src;
     } else {
