@@ -164,8 +164,10 @@ __device__ __forceinline__ T pp_pick(const T (&a)[PP_NB], int x) {
 // Every leader CTA sends what the others need with asynchronous stores that count into the receiver's
 // mbarrier, and waits for its own. (Stores, then a cluster barrier: 0.25 us for the barrier alone, 0.7 us with
 // the maxima and the row, whose completion the barrier's release waits for.)
-// Two mbarriers take turns: a CTA sends for the turn after next only when every warp has finished this one. So
-// of two exchanges in a row, one has a part from every warp.
+// Two mbarriers take turns, so an exchange's bytes must not arrive while a receiver still waits for the one
+// before the last. Every warp of every CTA therefore has a part in every exchange, sent when it has closed the
+// last: whoever closes an exchange knows that all the others have closed the one before, and with it that all
+// its bytes have arrived everywhere. An exchange of one sender alone (a row, a choice) takes join() of the rest.
 // Only the warps that hold rows (or the copies, below) take part. One CTA alone meets at a barrier of those warps instead.
 template <typename T, bool GEN>
 struct PanelX {
@@ -191,20 +193,21 @@ struct PanelX {
         else pp_warps_barrier(nw * 32);
         xn++;
     }
+    // the warp's part in an exchange to which it has nothing to say, and the bytes of all of them
+    __device__ __forceinline__ void join() const {
+        const int lane = threadIdx.x & 31;
+        if (C > 1 && lane < C) put(&S.hi[b][rank * nw + (threadIdx.x >> 5)], lane, 0u);
+    }
+    __device__ int join_bytes() const { return C * nw * 4; }
     // the warps meet: what they read before may be overwritten after, and (fence) what they wrote to global
     // memory is visible
     __device__ __forceinline__ void meet(bool fence = false) {
         if (fence) __threadfence();
         __syncwarp();
         if (fence) __threadfence();
-        if (C > 1) {
-            open(C * nw * 4);
-            const int lane = threadIdx.x & 31;
-            if (lane < C) put(&S.hi[b][rank * nw + (threadIdx.x >> 5)], lane, 0u);
-            close();
-        } else {
-            pp_warps_barrier(nw * 32);
-        }
+        open(join_bytes());
+        join();
+        close();
         if (fence) __threadfence();
     }
     // The next exchange, of maxima, with row `pos` from the CTA's own copy: the warp that holds it (`copy`) writes
@@ -339,7 +342,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
     const int orig = tid < chunk && k0 + rank * chunk + tid < f ? k0 + rank * chunk + tid : -1;
     // Every leader CTA has a copy of the block's rows, in one warp more, and updates them like its own: the pivot
     // row of a step never travels unless it comes from outside the block. The warp takes part in every exchange
-    // (with zeros), so that nobody is two of them ahead of it. Blocks of more than 15 warps a CTA go without.
+    // (with zeros). Blocks of more than 15 warps a CTA go without.
     const bool copies = C > 1 && rows < PP_WARPS, spare = copies && warp == rows;
     const int nw = rows + copies, nparts = C * nw;
     const int src = spare ? (k0 + lane < f ? k0 + lane : -1) : orig;
@@ -370,7 +373,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
             h = 0;
             for (int i = lane; i < nparts; i += 32) h = max(h, S.hi[X.b][i]);
             const double bound = pp_bound<T>(__reduce_max_sync(0xffffffffu, h));
-            const double akk = fabs((double)S.prow[j][1]);
+            const double fkk = (double)S.prow[j][1], akk = fabs(fkk);   // read once: an interchange overwrites the row
             // The bound alone accepts most pivots (every test grows with the maxima). Else the exact maxima:
             // lambda = max over the rows k < i < w with its first row r, mall = max over all rows i > k (NaN wins).
             bool fast;
@@ -441,8 +444,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         }
                         const double sigma = pp_val<T>(pp_warp_max<T>(s1)), m2 = pp_val<T>(pp_warp_max<T>(s2)),
                                      m1 = pp_val<T>(pp_warp_max<T>(s3));
-                        const double fkk = (double)S.prow[j][1], frr = (double)S.sc[0], fkr = (double)S.sc[1],
-                                     frk = (double)S.sc[2];
+                        const double frr = (double)S.sc[0], fkr = (double)S.sc[1], frk = (double)S.sc[2];
                         if (akk * sigma >= alpha * lambda * lambda) {
                             acc = akk >= pv.eps && akk >= pv.u * mall;
                         } else if (fabs(frr) >= alpha * sigma) {
@@ -464,7 +466,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     r2 = br;
                     if (!acc) {
                         if (j > 0) break;                // the search needs the whole front up to date
-                        X.open(8);
+                        X.open(X.join_bytes() + 8);
                         if (rank == 0) {
                             int cs = k, rs = -1;
                             pp_search(F, S, nw, k, pv.pivot, pv.u, pv.eps, bc, br, cs, rs);
@@ -474,6 +476,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                                     X.put(&S.sel[1], q, rs);
                                 }
                         }
+                        X.join();                        // behind the search: its reads are done when this closes
                         X.close();
                         c = S.sel[0];
                         r2 = S.sel[1];
@@ -481,7 +484,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                 }
                 const int p = r2 < 0 ? k : k + 1, q = r2 < 0 ? c : r2;
                 if (p != q || r2 >= 0) {
-                    X.meet();                            // everyone has read what the exchange below overwrites
+                    // (the last exchange is closed: everyone has read row k and the columns that change below)
                     if (p != q && q < kend) {            // "S" inside the block: columns in registers; rows by place
                         if (!GEN && rp >= k) {
                             const int y = q - k;
@@ -525,7 +528,8 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         X.meet(true);
                         load();
                     }
-                    X.open((r2 >= 0 ? 2 : 1) * X.row_bytes(left));
+                    X.open(X.join_bytes() + (r2 >= 0 ? 2 : 1) * X.row_bytes(left));
+                    X.join();
                     X.row(a, spare ? -1 : rp, k, j, left);
                     if (r2 >= 0) X.row(a, spare ? -1 : rp, k + 1, j + 1, left);
                     X.close();
@@ -538,8 +542,8 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     const bool zero = dk == 0.0;
                     int lpk = 0;
                     if (!GEN) {   // the column this row is of
-                        X.meet();   // (the exchange before may be one that only its sender had a part in)
-                        X.open(4);
+                        X.open(X.join_bytes() + 4);
+                        X.join();
                         if (rp == k && !spare)
                             for (int q = 0; q < C; ++q) X.put(&S.plp, q, mylp);
                         X.close();
@@ -833,9 +837,10 @@ __device__ void pp_update_tiles(const PanelFront<T, STRUCT == STRUCT_G>& F, Pane
     const int ntr = (f - k1 + TR - 1) / TR, ntc = (w - cf + PP_TC - 1) / PP_TC;
     const int nt = ntr * ntc, all = GEN ? 2 * nt : nt;
     const T* Lb = F.P + (int64_t)H.k0 * f;
+    const int ndisp = H.ndisp;
     auto row_of = [&](int i) {
         int s = i;
-        for (int d = 0; d < H.ndisp; ++d)
+        for (int d = 0; d < ndisp; ++d)
             if (H.ddst[d] == i) s = H.dsrc[d];
         return s;
     };
