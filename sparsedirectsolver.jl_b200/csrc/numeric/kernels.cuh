@@ -324,8 +324,9 @@ struct PanelGroups {
 // What the block leaves for T1 and T2, in the front's scratch
 template <typename T>
 struct PanelHdr {
-    int k0, k1, kend, ndisp;      // eliminated columns k0 .. k1 - 1 of the block k0 .. kend - 1
-    int moved, pairs;             // a row changed its place; the block has 2x2 pivots
+    int k0, k1, kend;             // eliminated columns k0 .. k1 - 1 of the block k0 .. kend - 1
+    int pairs;                    // the block has 2x2 pivots
+    int ndisp[2], moved[2];       // by the block's parity: entries of ddst / dsrc, a row changed its place
     int kind[PP_NB];
     int rowmap[PP_NB];            // the row (as the block started) that is now row k0 + t
     int ddst[PP_NB], dsrc[PP_NB]; // rows beyond k1 that hold another row: ddst holds dsrc (a block row)

@@ -121,6 +121,7 @@ struct PanelFront {
     T* us;             // the block's rows right of it, solved and unscaled: us[t f + c]
     int C, rank;       // the leader's CTAs and this CTA's rank among them
     int gs, grank;     // the front's CTAs and this CTA's rank among them
+    int par;           // the block's parity
     unsigned xn;       // exchanges of the leader's CTAs so far (the same in each)
     unsigned int* bar;
     unsigned int* epoch;   // shared memory
@@ -357,7 +358,9 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
         mylp = (orig >= 0 && orig < w) ? F.lp[orig] : 0;
     };
     load();
-    if (rank == 0 && tid == 0) F.hdr->ndisp = F.hdr->moved = 0;
+    // the next block's counters: the last one's, which every CTA has read, and the meetings of the group behind this
+    // block come before anyone counts in them
+    if (rank == 0 && tid == 0) F.hdr->ndisp[F.par ^ 1] = F.hdr->moved[F.par ^ 1] = 0;
     if (warp < nw) {
         PanelX<T, GEN> X(F, S, nw);
         int j = 0;
@@ -625,7 +628,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
         for (int e = 0; e < PP_NB; ++e)
             if (nbd + e < nb) F.P[rp + (int64_t)(k1 + e) * f] = a[e];
         if (rp != orig) {
-            const int d = atomicAdd(&F.hdr->ndisp, 1);
+            const int d = atomicAdd(&F.hdr->ndisp[F.par], 1);
             F.hdr->ddst[d] = rp;
             F.hdr->dsrc[d] = orig;
         }
@@ -638,7 +641,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
             F.hdr->lt[s][t] = l;
         }
     }
-    if (orig >= 0 && rp != orig) F.hdr->moved = 1;
+    if (orig >= 0 && rp != orig) F.hdr->moved[F.par] = 1;
     if (orig >= 0 && rp < w) F.lp[rp] = mylp;
     if (rank == 0) {
         if (GEN)
@@ -691,7 +694,7 @@ __device__ void pp_rows(const PanelFront<T, STRUCT == STRUCT_G>& F, const PanelH
 #pragma unroll
         for (int i = 0; i < NG; ++i) {
             const int t = 4 * i + sub;
-            g[i] = live && t < nbd ? F.at(H.moved ? H.rowmap[t] : H.k0 + t, c) : T(0);
+            g[i] = live && t < nbd ? F.at(H.moved[F.par] ? H.rowmap[t] : H.k0 + t, c) : T(0);
         }
         if (!H.pairs) {
             for (int s = 0; s < nbd; s += 4) {
@@ -739,14 +742,14 @@ __device__ void pp_rows(const PanelFront<T, STRUCT == STRUCT_G>& F, const PanelH
             for (int i = 0; i + 1 < NG; ++i) g[i] = g[i + 1];
         }
     }
-    if (!H.moved) return;
+    if (!H.moved[F.par]) return;
     for (int c = gt; c < H.k0; c += GT) {
         T* col = F.P + (int64_t)c * f;
         T b[2 * PP_NB];
         for (int t = 0; t < nbd; ++t) b[t] = col[H.rowmap[t]];
-        for (int d = 0; d < H.ndisp; ++d) b[PP_NB + d] = col[H.dsrc[d]];
+        for (int d = 0; d < H.ndisp[F.par]; ++d) b[PP_NB + d] = col[H.dsrc[d]];
         for (int t = 0; t < nbd; ++t) col[H.k0 + t] = b[t];
-        for (int d = 0; d < H.ndisp; ++d) col[H.ddst[d]] = b[PP_NB + d];
+        for (int d = 0; d < H.ndisp[F.par]; ++d) col[H.ddst[d]] = b[PP_NB + d];
     }
 }
 
@@ -837,7 +840,7 @@ __device__ void pp_update_tiles(const PanelFront<T, STRUCT == STRUCT_G>& F, Pane
     const int ntr = (f - k1 + TR - 1) / TR, ntc = (w - cf + PP_TC - 1) / PP_TC;
     const int nt = ntr * ntc, all = GEN ? 2 * nt : nt;
     const T* Lb = F.P + (int64_t)H.k0 * f;
-    const int ndisp = H.ndisp;
+    const int ndisp = H.ndisp[F.par];
     auto row_of = [&](int i) {
         int s = i;
         for (int d = 0; d < ndisp; ++d)
@@ -911,6 +914,7 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
     F.gs = job.gs;
     F.grank = job.rank;
     F.xn = xn;
+    F.par = 0;
     F.bar = bar + job.fi;
     F.epoch = &S.epoch;
     F.status = status;
@@ -930,11 +934,12 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
             if (i > j) F.P[j + (int64_t)i * f] = F.P[i + (int64_t)j * f];
         }
     for (int q = gt; q < w; q += GT) F.lp[q] = q;
+    if (gt == 0) F.hdr->ndisp[0] = F.hdr->moved[0] = 0;
     bool ok = pp_group_sync(F);
     PanelHdr<T>& H = S.hdr;
     // A barrier that gave up (a status word, no fault): helpers leave, the leader's CTAs go through the
     // blocks together without the shared phases, so that they still meet at every cluster barrier
-    for (int k = 0, first = 1; k < w; first = 0) {
+    for (int k = 0, first = 1; k < w; first = 0, F.par ^= 1) {
         if constexpr (GEN) {   // the previous block's rows: the helpers while the leader factors, or everyone
             const int helpers = F.gs - F.C;
             if (!first && ok && helpers == 0) pp_urows<T>(F, H, F.grank, F.gs);
