@@ -219,6 +219,10 @@ int sdsb200_set_graphs(sdsb200_plan* plan, int32_t on);
  * tasks in the same launch); 0: one launch per level and sweep (the engine of the solve sub-phases). */
 int sdsb200_set_persistent(sdsb200_plan* plan, int32_t on);
 
+/* Longest wait, in ns, of the CTAs of a wide LDLT / LU front for one another (2e9 by default). A factorization in
+ * which one takes longer returns SDSB200_TIMEOUT; the next call starts afresh. */
+int sdsb200_set_wait_limit(sdsb200_plan* plan, int64_t ns);
+
 /* Profiling mode (on != 0): CUDA events around every launch of the following factor and solve
  * calls, accumulated per kernel kind (resets the totals). Costs one event record per launch. */
 int sdsb200_set_profiling(sdsb200_plan* plan, int32_t on);

@@ -279,7 +279,7 @@ int run_factor(Plan* P, const double* nzval, double eps, double u, int pivot, in
                 a.cbuf = buf(L.cbuf, a.cstride);
                 a.finfo = P->d_finfo;
                 a.ns = (int32_t)P->ns;
-                a.status = P->d_solve_status;
+                a.status = P->d_flow_status;
                 a.copy_src = static_cast<const T*>(P->d_inv);
                 a.copy_stride = P->inv_len;
                 a.exact = sizeof(T) == 8 ? L.exact : 0;
@@ -337,11 +337,11 @@ int run_factor(Plan* P, const double* nzval, double eps, double u, int pivot, in
                 a.pivot = pivot; a.lu_pivot = lu_pivot; a.u = u; a.eps = eps;
                 if (L.panel >= 0 && nm == 1 && !members) {
                     e = cudaMemsetAsync(P->d_coop_bar, 0, sizeof(unsigned int) * L.count, st);
-                    PanelGroups g{P->d_panel_jobs, P->d_panel_ptr + L.panel, P->d_coop_bar, P->d_solve_status, L.panel_csize};
+                    PanelGroups g{P->d_panel_jobs, P->d_panel_ptr + L.panel, P->d_coop_bar, P->d_flow_status, P->wait_ns, L.panel_csize};
                     if (e == cudaSuccess) e = launch_pivot_panel<T>(P->structure, a, g, L.coop_grid, st);
                 } else if (L.coop >= 0 && nm == 1 && !members) {
                     e = cudaMemsetAsync(P->d_coop_bar, 0, sizeof(unsigned int) * L.count, st);
-                    CoopGroups g{P->d_coop_first + L.coop, P->d_coop_bar, P->d_solve_status};
+                    CoopGroups g{P->d_coop_first + L.coop, P->d_coop_bar, P->d_flow_status, P->wait_ns};
                     if (e == cudaSuccess) e = launch_large_pivot_coop<T>(P->structure, a, g, L.coop_grid, st);
                 } else {
                     e = launch_large_pivot<T>(P->structure, a, nm, st);
@@ -758,7 +758,7 @@ int sdsb200_factor(sdsb200_plan* plan, const double* nzval, const int8_t* h_psig
     P->factored = false;
     if (interrupted(P)) return fail(SDSB200_INTERRUPTED, "interrupted by user_host_interrupt");
     std::vector<uint64_t> key = {(uint64_t)(uintptr_t)nzval, bits(eps), bits(o.pivot_threshold), (uint64_t)pivot,
-                                 (uint64_t)lu_pivot, (uint64_t)P->nact, (uint64_t)P->all_members};
+                                 (uint64_t)lu_pivot, (uint64_t)P->nact, (uint64_t)P->all_members, P->wait_ns};
     // a first call with these buffers and options launches directly (capturing and instantiating a graph of a
     // thousand launches takes 15 ms, the launches themselves less than the factorization); the second captures
     const bool first = P->factor_key != key;
@@ -777,8 +777,10 @@ int sdsb200_factor(sdsb200_plan* plan, const double* nzval, const int8_t* h_psig
     CK(cudaStreamSynchronize(st), "factorization");
     prof_resolve(P);
     if (*h_flow_status != 0) {
-        cudaMemsetAsync(P->d_flow_status, 0, sizeof(int32_t), st);
-        return fail(SDSB200_TIMEOUT, "a bounded wait of the factorization's step tasks gave up");
+        // the next call, on whatever stream, comes behind the reset
+        CK(cudaMemsetAsync(P->d_flow_status, 0, sizeof(int32_t), st), "status reset");
+        CK(cudaStreamSynchronize(st), "status reset");
+        return fail(SDSB200_TIMEOUT, "a bounded wait of the factorization's kernels gave up");
     }
     if (h_info) {
         if (P->all_members) {
@@ -1079,6 +1081,14 @@ int sdsb200_set_graphs(sdsb200_plan* plan, int32_t on) {
     Plan* P = reinterpret_cast<Plan*>(plan);
     if (!P) return fail(SDSB200_INVALID_VALUE, "plan is NULL");
     P->use_graphs = on != 0;
+    return SDSB200_OK;
+}
+
+int sdsb200_set_wait_limit(sdsb200_plan* plan, int64_t ns) {
+    Plan* P = reinterpret_cast<Plan*>(plan);
+    if (!P) return fail(SDSB200_INVALID_VALUE, "plan is NULL");
+    if (ns < 0) return fail(SDSB200_INVALID_VALUE, "the wait limit must be nonnegative");
+    P->wait_ns = (uint64_t)std::min<int64_t>(ns, int64_t(1) << 58);   // (ten times that still fits)
     return SDSB200_OK;
 }
 

@@ -291,7 +291,8 @@ cudaError_t launch_scale_ld_front(int structure, const ScaleArgs<T>& a, int maxw
 struct CoopGroups {
     const int32_t* cta_first;  // per listed front: first CTA of its group (count + 1 entries)
     unsigned int* bar;         // per listed front: group barrier counter, zeroed before the launch
-    int32_t* status;           // nonzero: a group barrier wait gave up
+    int32_t* status;           // nonzero: a group barrier wait gave up, and with it the factorization
+    uint64_t wait_ns;          // the longest wait
 };
 constexpr int COOP_THREADS = 256;
 template <typename T>
@@ -318,7 +319,8 @@ struct PanelGroups {
     const PanelJob* jobs;
     const int32_t* job_ptr;   // per CTA, grid + 1
     unsigned int* bar;        // per listed front: group barrier counter, zeroed before the launch
-    int32_t* status;          // nonzero: a bounded group barrier gave up
+    int32_t* status;          // nonzero: a wait gave up, and with it the factorization
+    uint64_t wait_ns;         // the longest wait
     int32_t csize;
 };
 // What the block leaves for T1 and T2, in the front's scratch

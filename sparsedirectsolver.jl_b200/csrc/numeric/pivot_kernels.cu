@@ -95,27 +95,34 @@ template cudaError_t launch_large_pivot<float>(int, const LargePivotArgs<float>&
 // decision (one warp) | column / row interchanges | multipliers | rank-1 or rank-2 update.
 // Each entry receives the same floating-point operations in the same order as in the one-CTA
 // kernel, so pivots, D and the panels are identical; only the update is spread over the group.
-// A group barrier waits at most ~2 s, then records a nonzero status and goes on (no hang).
-__device__ __forceinline__ void group_barrier(unsigned int* bar, unsigned int& epoch, int gs, int32_t* status) {
+// A group barrier that waits longer than ten times the limit (a decision may read the whole front) records a
+// nonzero status; it and the others then return false, and the CTAs leave the front.
+__device__ __forceinline__ bool group_barrier(unsigned int* bar, unsigned int& epoch, int gs, const CoopGroups& G, int* ok) {
     __syncthreads();
     epoch += gs;
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(bar, 1u);
         unsigned int v;
-        long spins = 0;
-        while (true) {
+        uint64_t t0 = 0, now;
+        for (unsigned spins = 0;; ++spins) {
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(bar));
             if ((int)(v - epoch) >= 0) break;
-            if (++spins > (1L << 26)) {
-                atomicExch(status, 1);
-                break;
+            if ((spins & 255) == 255) {
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+                if (t0 == 0) t0 = now;
+                if (*(volatile int32_t*)G.status != 0 || now - t0 >= 10 * G.wait_ns) {
+                    atomicExch(G.status, 1);
+                    *ok = 0;
+                    break;
+                }
             }
             __nanosleep(32);
         }
         __threadfence();
     }
     __syncthreads();
+    return *(volatile int*)ok != 0;
 }
 
 static_assert(COOP_ROWS == COOP_THREADS, "an update item holds one row per thread");
@@ -280,6 +287,8 @@ __global__ void __launch_bounds__(COOP_THREADS) large_pivot_coop_kernel(LargePiv
     __shared__ double team_red[COOP_THREADS / 32];
     __shared__ int team_redi[COOP_THREADS / 32];
     __shared__ double pred[COOP_THREADS / 32][COOP_COLS];
+    __shared__ int held;   // the front's barriers have held so far
+    if (tid == 0) held = 1;
     const CtaTeam team{tid, nt, team_red, team_redi};
     if (STRUCT == STRUCT_S) {
         for (int q = gt; q < w * w; q += GT) {
@@ -296,7 +305,7 @@ __global__ void __launch_bounds__(COOP_THREADS) large_pivot_coop_kernel(LargePiv
             coop_panel_item<0>(F, 0, q, w, jb, je, je - jb, CoopStep{}, T(1), pred, tid);
         }
     }
-    group_barrier(bar, epoch, gs, G.status);
+    if (!group_barrier(bar, epoch, gs, G, &held)) return;
     int64_t st[NSTAT] = {0, 0, 0, 0, 0, 0};
     if constexpr (STRUCT == STRUCT_S) {
         int pk = -1, pkind = 0;   // the step whose multipliers are still to be written (1: 1x1, 2: 2x2)
@@ -327,7 +336,7 @@ __global__ void __launch_bounds__(COOP_THREADS) large_pivot_coop_kernel(LargePiv
                 choose_pivot(F, k, w, A.pivot, A.u, A.eps, team, c, r);
                 if (tid == 0) { sc.ctl[0] = c; sc.ctl[1] = r; }
             }
-            group_barrier(bar, epoch, gs, G.status);
+            if (!group_barrier(bar, epoch, gs, G, &held)) return;
             const int c = sc.ctl[0], r = sc.ctl[1];
             const int p = r < 0 ? k : k + 1, qsw = r < 0 ? c : r;
             if (p != qsw) {
@@ -346,7 +355,7 @@ __global__ void __launch_bounds__(COOP_THREADS) large_pivot_coop_kernel(LargePiv
                     t = F.at(p, qsw); F.at(p, qsw) = F.at(qsw, p); F.at(qsw, p) = t;
                     int tl = sc.lp[p]; sc.lp[p] = sc.lp[qsw]; sc.lp[qsw] = tl;
                 }
-                group_barrier(bar, epoch, gs, G.status);
+                if (!group_barrier(bar, epoch, gs, G, &held)) return;
             }
             CoopStep cs{};
             const int nb = r < 0 ? 1 : 2;
@@ -387,7 +396,7 @@ __global__ void __launch_bounds__(COOP_THREADS) large_pivot_coop_kernel(LargePiv
                 if (r < 0) coop_panel_item<1>(F, k, q, j0, jb, je, nmax, cs, T(1), pred, tid);
                 else coop_panel_item<2>(F, k, q, j0, jb, je, nmax, cs, T(1), pred, tid);
             }
-            group_barrier(bar, epoch, gs, G.status);
+            if (!group_barrier(bar, epoch, gs, G, &held)) return;
             pk = k; pkind = nb; pc = cs;
             k += nb;
         }
@@ -411,14 +420,14 @@ __global__ void __launch_bounds__(COOP_THREADS) large_pivot_coop_kernel(LargePiv
                 int r = pivoting ? lu_choose_row(F, k, w, A.u, team) : k;
                 if (tid == 0) sc.ctl[0] = r;
             }
-            group_barrier(bar, epoch, gs, G.status);
+            if (!group_barrier(bar, epoch, gs, G, &held)) return;
             const int r = sc.ctl[0];
             if (r != k) {
                 for (int j = gt; j < f; j += GT) {
                     T t = F.at(k, j); F.at(k, j) = F.at(r, j); F.at(r, j) = t;
                 }
                 if (lead) { int t = sc.lp[k]; sc.lp[k] = sc.lp[r]; sc.lp[r] = t; }
-                group_barrier(bar, epoch, gs, G.status);
+                if (!group_barrier(bar, epoch, gs, G, &held)) return;
             }
             double dk = F.get(k, k);
             signed char kk = KIND_1X1;
@@ -447,7 +456,7 @@ __global__ void __launch_bounds__(COOP_THREADS) large_pivot_coop_kernel(LargePiv
                     coop_u_item(F, k, rb, re, k + 1 + ct * COOP_ROWS, tdk, tid);
                 }
             }
-            group_barrier(bar, epoch, gs, G.status);
+            if (!group_barrier(bar, epoch, gs, G, &held)) return;
             pk = k; ptdk = tdk; pdk = dk;
         }
         flush(true);

@@ -55,9 +55,30 @@ __device__ __forceinline__ void pp_x_arm(unsigned long long* mbar, int bytes) {
                  "r"(bytes)
                  : "memory");
 }
-// a wait of some seconds at most, then the status word (which later waits do not outlast)
-__device__ __forceinline__ void pp_x_wait(unsigned long long* mbar, int parity, int32_t* status) {
+__device__ __forceinline__ uint64_t pp_clock() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// The longest wait, and the status word that a wait sets when it gives up, which ends the others too (in shared
+// memory: a wait that does not last needs neither in a register)
+struct PanelLimit {
+    int32_t* status;
+    uint64_t ns;
+};
+// A waiting thread's look at the clock: the time of its first (t0 = 0: this is it), or 0: it gives up.
+__device__ __forceinline__ uint64_t pp_waited(const PanelLimit& limit, uint64_t t0) {
+    if (*(volatile int32_t*)limit.status != 0) return 0;
+    const uint64_t now = pp_clock();
+    if (t0 == 0) t0 = now;
+    if (now - t0 < limit.ns) return t0;
+    atomicExch(limit.status, 1);
+    return 0;
+}
+// true: the phase is complete; false: the wait has given up, and nothing of the exchange may be used
+__device__ __forceinline__ bool pp_x_wait(unsigned long long* mbar, int parity, const PanelLimit& limit) {
     const unsigned m = (unsigned)__cvta_generic_to_shared(mbar);
+    uint64_t t0 = 0;
     for (unsigned spins = 0;; ++spins) {
         unsigned done;
         asm volatile(
@@ -67,12 +88,8 @@ __device__ __forceinline__ void pp_x_wait(unsigned long long* mbar, int parity, 
             : "=r"(done)
             : "r"(m), "r"(parity)
             : "memory");
-        if (done) return;
-        if ((spins & 1023) == 1023 && *(volatile int32_t*)status != 0) return;
-        if (spins > (1u << 24)) {
-            atomicExch(status, 1);
-            return;
-        }
+        if (done) return true;
+        if ((spins & 63) == 63 && (t0 = pp_waited(limit, t0)) == 0) return false;
     }
 }
 __device__ __forceinline__ void pp_x_init(unsigned long long* mbar) {
@@ -95,42 +112,24 @@ __device__ __forceinline__ void pp_load2(const float* p, float& x, float& y) {
     y = v.y;
 }
 
-// one value from global into shared memory in the background (zero when not valid)
-__device__ __forceinline__ void pp_fetch(double* s, const double* g, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g),
-                 "r"(valid ? 8 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ void pp_fetch(float* s, const float* g, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g),
-                 "r"(valid ? 4 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ void pp_fetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 __device__ __forceinline__ void pp_cluster_barrier() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// a front's CTAs meet in global memory; a wait of about two seconds gives up, records the status word and
-// clears *ok (shared), as does a status word that is already set
-__device__ __forceinline__ void pp_group_barrier(unsigned int* bar, unsigned int& epoch, int gs, int32_t* status, int* ok) {
+// a front's CTAs meet in global memory; a wait that gives up clears *ok (shared)
+__device__ __forceinline__ void pp_group_barrier(unsigned int* bar, unsigned int& epoch, int gs, const PanelLimit& limit, int* ok) {
     __syncthreads();
     if (threadIdx.x == 0) {
         epoch += gs;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         unsigned int v;
-        for (long spins = 0;; ++spins) {
+        uint64_t t0 = 0;
+        for (unsigned spins = 0;; ++spins) {
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             if ((int)(v - epoch) >= 0) break;
-            if ((spins & 255) == 255 && *(volatile int32_t*)status != 0) {
-                *ok = 0;
-                break;
-            }
-            if (spins > (1L << 25)) {
-                atomicExch(status, 1);
+            if ((spins & 63) == 63 && (t0 = pp_waited(limit, t0)) == 0) {
                 *ok = 0;
                 break;
             }
@@ -138,6 +137,35 @@ __device__ __forceinline__ void pp_group_barrier(unsigned int* bar, unsigned int
         }
     }
     __syncthreads();
+}
+// *gate (shared): n warps go through together, or none. One that waits too long closes it, which the last to
+// arrive forestalls: the word decides, so that nobody stands alone at a barrier behind it. One lane calls it.
+__device__ __forceinline__ bool pp_gate(int* gate, int n, const PanelLimit& limit) {
+    constexpr int CLOSED = 1 << 30;
+    for (int v = 0;;) {   // arrive, unless it is closed
+        const int old = atomicCAS(gate, v, v + 1);
+        if (old == v) break;
+        if (old & CLOSED) return false;
+        v = old;
+    }
+    uint64_t t0 = 0;
+    for (unsigned spins = 0;; ++spins) {
+        int v = *(volatile int*)gate;
+        if (v == n) return true;
+        if (v & CLOSED) return false;
+        if ((spins & 63) == 63 && (t0 = pp_waited(limit, t0)) == 0)
+            while (v < n) {   // close it, unless the last has come
+                const int old = atomicCAS(gate, v, v | CLOSED);
+                if (old == v) break;
+                v = old;
+            }
+    }
+}
+// CTA q's copy of *p
+__device__ __forceinline__ void pp_remote_set(int* p, int q, int v) {
+    unsigned ra;
+    pp_remote(p, q, ra);
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ra), "r"(v) : "memory");
 }
 
 }  // namespace sds
@@ -153,15 +181,23 @@ __global__ void __launch_bounds__(PP_THREADS, 1) pivot_panel_kernel(LargePivotAr
     if (threadIdx.x == 0) {
         pp_x_init(&S.mbar[0]);
         pp_x_init(&S.mbar[1]);
+        S.dead = 0;
     }
     pp_cluster_barrier();
     unsigned xn = 0;
     for (int q = G.job_ptr[blockIdx.x]; q < G.job_ptr[blockIdx.x + 1]; ++q) {
         const PanelJob job = G.jobs[q];
-        if (job.role != PANEL_IDLE) pp_front<T, STRUCT>(A, job, S, G.csize, G.bar, G.status, xn);
+        if (job.role != PANEL_IDLE) pp_front<T, STRUCT>(A, job, S, G, xn);
         // the cluster's CTAs start their next job, or leave, together: none writes into another's shared
         // memory before or after its front
         pp_cluster_barrier();
+        // A wait gave up in this job, in any of them: the mbarriers hold what did not arrive, so no further job.
+        // (A CTA that were a job ahead could set the word here only in its exchanges, which come behind a meeting
+        // with this one.) Stores that nobody waits for may still be on their way: their CTAs stay a little.
+        if (S.dead) {
+            for (int i = 0; i < 100; ++i) __nanosleep(1000);
+            return;
+        }
     }
 }
 

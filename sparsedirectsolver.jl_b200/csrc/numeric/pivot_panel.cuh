@@ -47,6 +47,10 @@ struct PanelSmem {
     unsigned long long sg[PP_MAXC * PP_WARPS], m1[PP_MAXC * PP_WARPS], m2[PP_MAXC * PP_WARPS];
     T sc[4];                                               // F[r, r], F[k, r], F[r, k]
     int plp, nbd, ok;
+    int gate;                                              // the leader's first CTA: its warps go into the search together
+    int fail;                                              // a warp's wait in this block gave up
+    int dead;                                              // ... one of the cluster's; every CTA's word is set
+    PanelLimit limit;
     unsigned epoch, xn;
     int sel[2];
     int kind[PP_NB];
@@ -125,8 +129,9 @@ struct PanelFront {
     unsigned xn;       // exchanges of the leader's CTAs so far (the same in each)
     unsigned int* bar;
     unsigned int* epoch;   // shared memory
-    int32_t* status;
+    const PanelLimit* limit;   // shared memory
     int* ok;           // shared memory: the front's barriers have held so far
+    int* dead;         // shared memory, set in every CTA of the cluster
     // F[i, j], i or j < w
     __device__ T& at(int i, int j) const {
         if (!GEN || (i >= j && j < w)) return P[i + (int64_t)j * f];
@@ -147,9 +152,18 @@ __device__ __forceinline__ void pp_sync(const PanelFront<T, GEN>& F) {
 // every CTA of the front meets; false once a bounded wait has given up (the same for the whole CTA)
 template <typename T, bool GEN>
 __device__ __forceinline__ bool pp_group_sync(PanelFront<T, GEN>& F) {
-    if (F.gs > F.C) pp_group_barrier(F.bar, *F.epoch, F.gs, F.status, F.ok);
-    else pp_sync(F);
-    return *F.ok != 0;
+    if (F.gs > F.C) {
+        pp_group_barrier(F.bar, *F.epoch, F.gs, *F.limit, F.ok);
+        return *F.ok != 0;
+    }
+    pp_sync(F);
+    return true;
+}
+// This CTA has given up: the cluster's CTAs learn of it at their next cluster barrier
+template <typename T, bool GEN>
+__device__ __forceinline__ void pp_give_up(const PanelFront<T, GEN>& F) {
+    if (threadIdx.x == 0)
+        for (int q = 0; q < F.C; ++q) pp_remote_set(F.dead, q, 1);
 }
 
 template <typename T>
@@ -176,9 +190,8 @@ struct PanelX {
     const int C, rank, nw;
     int b;
     unsigned xn;
-    int32_t* const status;
     __device__ PanelX(const PanelFront<T, GEN>& F, PanelSmem<T>& S_, int nw_)
-        : S(S_), C(F.C), rank(F.rank), nw(nw_), b(0), xn(F.xn), status(F.status) {}
+        : S(S_), C(F.C), rank(F.rank), nw(nw_), b(0), xn(F.xn) {}
     // opens the next exchange, of `bytes` bytes into each CTA
     __device__ __forceinline__ void open(int bytes) {
         b = xn & 1;
@@ -189,27 +202,32 @@ struct PanelX {
         if (C > 1) pp_x_store(p, q, v, &S.mbar[b]);
         else *p = v;
     }
-    __device__ __forceinline__ void close() {
-        if (C > 1) pp_x_wait(&S.mbar[b], (xn >> 1) & 1, status);
+    // This lane's view: false, its wait gave up. A warp leaves the block when a lane's did; nothing that was
+    // exchanged may be used then. The others wait in vain for its next part and follow.
+    __device__ __forceinline__ bool close_lane() {
+        bool ok = true;
+        if (C > 1) ok = pp_x_wait(&S.mbar[b], (xn >> 1) & 1, S.limit);
         else pp_warps_barrier(nw * 32);
         xn++;
+        return ok;
     }
+    __device__ __forceinline__ bool close() { return __all_sync(0xffffffffu, close_lane()); }
     // the warp's part in an exchange to which it has nothing to say, and the bytes of all of them
     __device__ __forceinline__ void join() const {
         const int lane = threadIdx.x & 31;
         if (C > 1 && lane < C) put(&S.hi[b][rank * nw + (threadIdx.x >> 5)], lane, 0u);
     }
     __device__ int join_bytes() const { return C * nw * 4; }
-    // the warps meet: what they read before may be overwritten after, and (fence) what they wrote to global
-    // memory is visible
-    __device__ __forceinline__ void meet(bool fence = false) {
-        if (fence) __threadfence();
+    // the warps meet: what they wrote to global memory is visible
+    __device__ __forceinline__ bool meet() {
+        __threadfence();
         __syncwarp();
-        if (fence) __threadfence();
+        __threadfence();
         open(join_bytes());
         join();
-        close();
-        if (fence) __threadfence();
+        const bool ok = close();
+        __threadfence();
+        return ok;
     }
     // The next exchange, of maxima, with row `pos` from the CTA's own copy: the warp that holds it (`copy`) writes
     // the row and then opens the exchange, so whoever has waited for the maxima sees the row. Whole warps call it.
@@ -327,7 +345,7 @@ struct PanelPivot {
 };
 
 // The pivot steps of the block that starts at column k0, by the leader's CTAs. Returns k1, the first column
-// that is left.
+// that is left, or -1 (the whole CTA) after a wait that gave up.
 //
 // A step is a chain of latencies, not of work: the maxima to the other CTAs, the decision,
 // a division, the update of up to 31 columns.
@@ -364,6 +382,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
     if (warp < nw) {
         PanelX<T, GEN> X(F, S, nw);
         int j = 0;
+        bool gave_up = false;
         while (j < nb) {
             const int k = k0 + j, left = nb - j;   // columns k .. kend - 1
             // a bound of the column below row k, and row k itself, to every leader CTA
@@ -372,10 +391,12 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
             unsigned h = __reduce_max_sync(0xffffffffu, rp > k && !spare ? pp_hi(a[0]) : 0u);
             if (lane < C) X.put(&S.hi[X.b][rank * nw + warp], lane, h);
             if (!copies) X.row(a, rp, k, j, left);
-            X.close();
-            h = 0;
+            // (no entry's part is all ones: its sign is cleared)
+            h = X.close_lane() ? 0u : 0xffffffffu;
             for (int i = lane; i < nparts; i += 32) h = max(h, S.hi[X.b][i]);
-            const double bound = pp_bound<T>(__reduce_max_sync(0xffffffffu, h));
+            h = __reduce_max_sync(0xffffffffu, h);
+            if (h == 0xffffffffu) { gave_up = true; break; }
+            const double bound = pp_bound<T>(h);
             const double fkk = (double)S.prow[j][1], akk = fabs(fkk);   // read once: an interchange overwrites the row
             // The bound alone accepts most pivots (every test grows with the maxima). Else the exact maxima:
             // lambda = max over the rows k < i < w with its first row r, mall = max over all rows i > k (NaN wins).
@@ -397,7 +418,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     X.put(&S.mx[at], lane, mkey);
                     X.put(&S.ridx[at], lane, ri);
                 }
-                X.close();
+                if (!X.close()) { gave_up = true; break; }
                 unsigned long long lk = 0, mk = 0;
                 int r = 0x7fffffff;
                 for (int i = lane; i < nparts; i += 32) {
@@ -438,7 +459,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                             }
                         if (rp == k && !spare)
                             for (int q = 0; q < C; ++q) X.put(&S.sc[1], q, v);
-                        X.close();
+                        if (!X.close()) { gave_up = true; break; }
                         s1 = s2 = s3 = 0;
                         for (int i = lane; i < nparts; i += 32) {
                             if (S.sg[i] > s1) s1 = S.sg[i];
@@ -471,6 +492,10 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         if (j > 0) break;                // the search needs the whole front up to date
                         X.open(X.join_bytes() + 8);
                         if (rank == 0) {
+                            // the search has barriers of the CTA's warps: all of them, or none
+                            bool in = C == 1;
+                            if (C > 1 && lane == 0) in = pp_gate(&S.gate, nw, S.limit);
+                            if (!__any_sync(0xffffffffu, in)) { gave_up = true; break; }
                             int cs = k, rs = -1;
                             pp_search(F, S, nw, k, pv.pivot, pv.u, pv.eps, bc, br, cs, rs);
                             if (tid == 0)
@@ -480,7 +505,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                                 }
                         }
                         X.join();                        // behind the search: its reads are done when this closes
-                        X.close();
+                        if (!X.close()) { gave_up = true; break; }
                         c = S.sel[0];
                         r2 = S.sel[1];
                     }
@@ -528,14 +553,14 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                             F.lp[p] = F.lp[q];
                             F.lp[q] = tl;
                         }
-                        X.meet(true);
+                        if (!X.meet()) { gave_up = true; break; }
                         load();
                     }
                     X.open(X.join_bytes() + (r2 >= 0 ? 2 : 1) * X.row_bytes(left));
                     X.join();
                     X.row(a, spare ? -1 : rp, k, j, left);
                     if (r2 >= 0) X.row(a, spare ? -1 : rp, k + 1, j + 1, left);
-                    X.close();
+                    if (!X.close()) { gave_up = true; break; }
                 }
             }
             if (GEN || r2 < 0) {
@@ -549,7 +574,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         X.join();
                         if (rp == k && !spare)
                             for (int q = 0; q < C; ++q) X.put(&S.plp, q, mylp);
-                        X.close();
+                        if (!X.close()) { gave_up = true; break; }
                         lpk = S.plp;
                     }
                     const int req = !GEN && pv.psign ? (int)pv.psign[pv.perm[F.c0 + lpk]] : 0;
@@ -613,12 +638,15 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                 j += 2;
             }
         }
+        if (gave_up && lane == 0) S.fail = 1;
         if (tid == 0) {
             S.nbd = j;
             S.xn = X.xn;
         }
     }
     __syncthreads();
+    if (S.fail) return -1;
+    if (tid == 0) S.gate = 0;   // for the next block: its group's meetings come first
     F.xn = S.xn;
     const int nbd = S.nbd, k1 = k0 + nbd;
     // the multipliers and what is left of the columns out to the rows' places
@@ -889,9 +917,10 @@ __device__ void pp_urows(const PanelFront<T, true>& F, const PanelHdr<T>& H, int
 
 // One front, by every CTA of its group
 template <typename T, int STRUCT>
-__device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelSmem<T>& S, int C, unsigned int* bar,
-                         int32_t* status, unsigned& xn) {
+__device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelSmem<T>& S, const PanelGroups& G,
+                         unsigned& xn) {
     constexpr bool GEN = STRUCT == STRUCT_G;
+    const int C = G.csize;
     const int s = A.list[job.fi];
     const DFront fd = A.fronts[s];
     PanelFront<T, GEN> F;
@@ -915,12 +944,15 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
     F.grank = job.rank;
     F.xn = xn;
     F.par = 0;
-    F.bar = bar + job.fi;
+    F.bar = G.bar + job.fi;
     F.epoch = &S.epoch;
-    F.status = status;
+    F.limit = &S.limit;
     F.ok = &S.ok;
+    F.dead = &S.dead;
     if (threadIdx.x == 0) {
         S.ok = 1;
+        S.limit = {G.status, G.wait_ns};
+        S.gate = S.fail = 0;
         S.epoch = 0;
         for (int q = 0; q < NSTAT; ++q) S.st[q] = 0;
     }
@@ -935,39 +967,43 @@ __device__ void pp_front(const LargePivotArgs<T>& A, const PanelJob& job, PanelS
         }
     for (int q = gt; q < w; q += GT) F.lp[q] = q;
     if (gt == 0) F.hdr->ndisp[0] = F.hdr->moved[0] = 0;
-    bool ok = pp_group_sync(F);
     PanelHdr<T>& H = S.hdr;
-    // A barrier that gave up (a status word, no fault): helpers leave, the leader's CTAs go through the
-    // blocks together without the shared phases, so that they still meet at every cluster barrier
-    for (int k = 0, first = 1; k < w; first = 0, F.par ^= 1) {
+    // A wait that gave up (a status word, no fault) ends the front. With helper clusters, whose meetings are in
+    // global memory, each CTA leaves by itself: the cluster's next barrier is the kernel's, behind the front.
+    // Without, the meetings are cluster barriers, and its CTAs leave together, at the one behind the exchanges:
+    // nobody can set `dead` between that barrier and its look at it.
+    const bool alone = F.gs == F.C;
+    bool ok = pp_group_sync(F);
+    for (int k = 0, first = 1; ok && k < w; first = 0, F.par ^= 1) {
         if constexpr (GEN) {   // the previous block's rows: the helpers while the leader factors, or everyone
             const int helpers = F.gs - F.C;
-            if (!first && ok && helpers == 0) pp_urows<T>(F, H, F.grank, F.gs);
-            else if (!first && ok && !leads) pp_urows<T>(F, H, F.grank - F.C, helpers);
+            if (!first && helpers == 0) pp_urows<T>(F, H, F.grank, F.gs);
+            else if (!first && !leads) pp_urows<T>(F, H, F.grank - F.C, helpers);
         }
         int k1 = 0;
         if (leads) k1 = pp_block<T, STRUCT>(F, S, pv, k);
+        if (k1 < 0) pp_give_up(F);
+        ok = alone || k1 >= 0;
         if (ok) ok = pp_group_sync(F);
-        if (!ok && !leads) return;
-        if (ok) {
-            const int* src = reinterpret_cast<const int*>(F.hdr);
-            int* dst = reinterpret_cast<int*>(&H);
-            for (int q = tid; q < (int)(sizeof(PanelHdr<T>) / 4); q += PP_THREADS) dst[q] = src[q];
-            __syncthreads();
-            k1 = H.k1;
-            pp_rows<T, STRUCT>(F, H);
-            ok = pp_group_sync(F);
-            if (!ok && !leads) return;
-        }
-        k = k1;
-        if (k < w && ok) {
+        if (alone) ok = *(volatile int*)F.dead == 0;
+        if (!ok) break;
+        const int* src = reinterpret_cast<const int*>(F.hdr);
+        int* dst = reinterpret_cast<int*>(&H);
+        for (int q = tid; q < (int)(sizeof(PanelHdr<T>) / 4); q += PP_THREADS) dst[q] = src[q];
+        __syncthreads();
+        k = H.k1;
+        pp_rows<T, STRUCT>(F, H);
+        ok = pp_group_sync(F);
+        if (ok && k < w) {
             pp_update<T, STRUCT>(F, S, H);
             ok = pp_group_sync(F);
-            if (!ok && !leads) return;
         }
     }
+    if (!ok) {
+        pp_give_up(F);
+        return;
+    }
     if (F.C > 1) xn = F.xn;   // one CTA alone uses no mbarrier
-    if (!ok) return;
     if constexpr (GEN) pp_urows<T>(F, H, F.grank, F.gs);
     for (int64_t q = gt; q < (int64_t)w * w; q += GT) {
         const int i = (int)(q % w), j = (int)(q / w);

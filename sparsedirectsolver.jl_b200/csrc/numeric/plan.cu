@@ -1764,7 +1764,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         P->d_norms = dalloc<double>(P, 2 * P->max_nrhs * nb);
         if (cudaMallocHost(&P->h_norms, sizeof(double) * 2 * P->max_nrhs * nb) != cudaSuccess)
             throw BuildError(SDSB200_ALLOC_FAILED, "cudaMallocHost");
-        // info of every member, then the step tasks' status word
+        // info of every member, then the factorization's status word
         if (cudaMallocHost(&P->h_info_pinned, sizeof(int64_t) * (nb + 1)) != cudaSuccess)
             throw BuildError(SDSB200_ALLOC_FAILED, "cudaMallocHost");
         {

@@ -144,7 +144,8 @@ struct Plan {
     int64_t n_flow_tasks = 0;
     unsigned int* d_flow_cnt = nullptr; // their counters: per launch count2 + 1 at list2, zeroed per launch
     int64_t flow_cnt_len = 0;
-    int32_t* d_flow_status = nullptr;   // nonzero: a bounded wait of the step tasks gave up
+    int32_t* d_flow_status = nullptr;   // nonzero: a bounded wait of the factorization's kernels gave up
+    uint64_t wait_ns = 2000000000;      // longest wait of the pivot kernels' CTAs for one another
     int64_t* d_flow_trace = nullptr;    // profiling: 4 int64 per step task
     int64_t psplit_slots = 0, psplit_cnts = 0;   // split tiles: most partial slots and counters of a launch
     void* d_psplit = nullptr;           // their 64 x 64 partial products

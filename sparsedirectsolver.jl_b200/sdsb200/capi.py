@@ -20,7 +20,7 @@ EXPORTS = ("sdsb200_default_opts", "sdsb200_plan_create", "sdsb200_plan_destroy"
            "sdsb200_get_stats", "sdsb200_get_pivots", "sdsb200_get_factor", "sdsb200_set_members",
            "sdsb200_set_interrupt", "sdsb200_set_graphs", "sdsb200_set_persistent", "sdsb200_set_profiling", "sdsb200_get_trace", "sdsb200_plan_stat", "sdsb200_last_error",
            "sdsb200_solve_noalloc", "sdsb200_sampled_outer", "sdsb200_residual", "sdsb200_solve_phase",
-           "sdsb200_schur_matrix")
+           "sdsb200_schur_matrix", "sdsb200_set_wait_limit")
 
 # solve sub-phases of sdsb200_solve_phase
 PHASE = {"fwd_perm": 1, "fwd": 2, "diag": 3, "bwd": 4, "bwd_perm": 5, "load": 6, "store": 7}
@@ -70,6 +70,7 @@ def bind(lib):
         "sdsb200_set_members": (C.c_int, [P, P, C.c_int32]),
         "sdsb200_set_interrupt": (C.c_int, [P, P]),
         "sdsb200_set_profiling": (C.c_int, [P, C.c_int32]),
+        "sdsb200_set_wait_limit": (C.c_int, [P, C.c_int64]),
         "sdsb200_set_graphs": (C.c_int, [P, C.c_int32]),
         "sdsb200_set_persistent": (C.c_int, [P, C.c_int32]),
         "sdsb200_plan_stat": (C.c_double, [P, C.c_char_p]),

@@ -9,6 +9,7 @@
 // pair, a result that differs in one bit from the serial steps: each is an error.
 //
 //   pivot_panel_check <seed> <cases>        random small fronts
+//   pivot_panel_check <seed> <cases> giveup  a wait gives up at a random moment: every thread must come to its end
 //   pivot_panel_check <seed> wide           clusters of 8 and 16 CTAs, blocks with and without the row copies
 #include <cuda_runtime.h>
 
@@ -58,6 +59,9 @@ struct Fiber {
     long target = 0;
     const struct Mbar* mbar = nullptr;
     int parity = 0;
+    const int* gate = nullptr;               // a gate's word that reaches `target`, or is closed
+    bool limited = false, expired = false;   // the wait has a limit; it has run out
+    bool lingers = false;                    // until no store is on its way
     inline bool blocked() const;
 };
 struct Store {                                // a remote store on its way
@@ -73,16 +77,20 @@ struct Mbar {
     inline void check();
 };
 static_assert(sizeof(Mbar) == 8, "an mbarrier is 8 bytes");
-inline bool Fiber::blocked() const { return (count && *count < target) || (mbar && mbar->phase == parity); }
-
 Fiber* cur;
 void* scheduler_sp;
 std::vector<Fiber*> fibers;
 std::vector<Store> flight;
+inline bool Fiber::blocked() const {
+    return !expired && ((count && *count < target) || (mbar && mbar->phase == parity) || (gate && *gate < target) ||
+                        (lingers && !flight.empty()));
+}
 std::vector<char> slow;                       // per link (source, destination): held back until all else waits
 long progress = 0;
 std::mt19937 rng(1);
 int threads_per_cta = 0;
+long first_expiry = -1;                       // the progress at which a wait runs out, whatever it waits for (-1: never)
+bool given_up = false;                        // ... and then the others, one after another
 
 [[noreturn]] void die(const char* what) {
     printf("%s (CTA %d thread %u)\n", what, cur ? cur->cta->bid : -1, cur ? cur->tid.x : 0u);
@@ -111,11 +119,12 @@ emu_switch:
     ret
 )");
 void yield() { emu_switch(&cur->sp, scheduler_sp); }
-void wait_count(const long* count, long target) {
+void wait_count(const long* count, long target, bool limited = false) {
     cur->count = count;
     cur->target = target;
+    cur->limited = limited;
     while (cur->blocked()) yield();
-    cur->count = nullptr;
+    if (!limited) cur->count = nullptr;
 }
 
 unsigned long long* warp_sync(unsigned long long v) {
@@ -187,11 +196,22 @@ void run() {
         for (size_t i = flight.size(); i-- > 0;)
             if (!slow[flight[i].link] && rng() % 2) deliver(i);
         if (!any) break;
+        if (first_expiry >= 0 && (given_up ? rng() % 4 == 0 : progress >= first_expiry)) {
+            // a wait runs out: one at first, then some of those that wait and look at the status word
+            std::vector<Fiber*> waiting;
+            for (Fiber* f : fibers)
+                if (!f->done && f->limited && f->blocked()) waiting.push_back(f);
+            if (!waiting.empty()) {
+                for (size_t n = given_up ? 1 + rng() % waiting.size() : 1; n-- > 0;) waiting[rng() % waiting.size()]->expired = true;
+                given_up = true;
+                progress++;
+            }
+        }
         if (progress != before) {
             idle = 0;
-        } else if (++idle > 1 && flight.empty()) {
+        } else if (++idle > 40 && flight.empty()) {
             die("every thread waits");
-        } else if (idle > 1) {   // what is held back, a part of it
+        } else if (idle > 1 && !flight.empty()) {   // what is held back, a part of it
             for (size_t n = 1 + rng() % flight.size(); n-- > 0;) deliver(rng() % flight.size());
         }
     }
@@ -227,6 +247,8 @@ static unsigned __reduce_min_sync(unsigned, unsigned x) {
     for (int i = 0; i < 32; ++i) r = min(r, (unsigned)v[i]);
     return r;
 }
+static bool __any_sync(unsigned m, int p) { return __ballot_sync(m, p) != 0; }
+static bool __all_sync(unsigned m, int p) { return __ballot_sync(m, p) == 0xffffffffu; }
 template <class X>
 static X emu_from_lane(X x, int lane) {
     unsigned long long b = 0;
@@ -291,12 +313,28 @@ static void pp_x_arm(unsigned long long* mbar, int bytes) {
     m->check();
     emu::progress++;
 }
-static void pp_x_wait(unsigned long long* mbar, int parity, int32_t*) {
+struct PanelLimit {
+    int32_t* status;
+    uint64_t ns;
+};
+// the end of a wait with a limit: true, what it waited for has come
+static bool emu_end(int32_t* status, bool come) {
+    emu::Fiber* f = emu::cur;
+    f->limited = false;
+    f->count = nullptr;
+    f->mbar = nullptr;
+    const bool gave_up = f->expired && !come;
+    f->expired = false;
+    if (gave_up) *status = 1;
+    return !gave_up;
+}
+static bool pp_x_wait(unsigned long long* mbar, int parity, const PanelLimit& limit) {
     emu::Fiber* f = emu::cur;
     f->mbar = emu_mbar(mbar);
     f->parity = parity;
+    f->limited = true;
     while (f->blocked()) emu::yield();
-    f->mbar = nullptr;
+    return emu_end(limit.status, f->mbar->phase != parity);
 }
 // the first n threads of the CTA
 static void pp_warps_barrier(int n) {
@@ -327,15 +365,34 @@ static void pp_cluster_barrier() {
     emu::wait_count(&c->arrived, (long)c->ctas.size() * emu::threads_per_cta * (op + 1));
 }
 static long emu_group_arrived;
-static void pp_group_barrier(unsigned*, unsigned& epoch, int gs, int32_t*, int*) {
+static void pp_group_barrier(unsigned*, unsigned& epoch, int gs, const PanelLimit& limit, int* ok) {
     emu::cta_sync();
     if (emu::cur->tid.x == 0) {
         epoch += gs;
         emu_group_arrived++;
         emu::progress++;
-        emu::wait_count(&emu_group_arrived, epoch);
+        emu::wait_count(&emu_group_arrived, epoch, true);
+        if (!emu_end(limit.status, emu_group_arrived >= (long)epoch)) *ok = 0;
     }
     emu::cta_sync();
+}
+static bool pp_gate(int* gate, int n, const PanelLimit& limit) {
+    constexpr int CLOSED = 1 << 30;
+    if (*gate & CLOSED) return false;
+    ++*gate;
+    emu::progress++;
+    emu::cur->limited = true;
+    emu::cur->gate = gate;
+    emu::cur->target = n;
+    while (emu::cur->blocked()) emu::yield();
+    emu::cur->gate = nullptr;
+    if (!emu_end(limit.status, *gate >= n)) *gate |= CLOSED;   // (an n that was reached stays)
+    return *gate == n;
+}
+static void pp_remote_set(int* p, int q, int v) {
+    emu::Cta* d = emu::cur->cta->cluster->ctas[q];
+    if (d->left == 0) emu::die("a store into the shared memory of a CTA that has left");
+    *reinterpret_cast<int*>(d->smem + emu::offset_of(p, sizeof(int))) = v;
 }
 
 }  // namespace sds
@@ -500,7 +557,7 @@ static void thread_start() {
 }
 
 template <typename T, int STRUCT>
-static bool check(int f, int w, int C, int nclusters, int values, const Options& o, unsigned seed) {
+static bool check(int f, int w, int C, int nclusters, int values, const Options& o, unsigned seed, bool give_up) {
     constexpr bool GEN = STRUCT == STRUCT_G;
     std::mt19937 g(seed);
     std::normal_distribution<double> normal;
@@ -581,16 +638,21 @@ static bool check(int f, int w, int C, int nclusters, int values, const Options&
         c.cluster->ctas.push_back(&c);
         auto* S = reinterpret_cast<PanelSmem<T>*>(c.smem);
         S->mbar[0] = S->mbar[1] = 0;
+        S->dead = 0;
         if (C == 1) jobs[b] = {b == 0 ? PANEL_SINGLE : PANEL_IDLE, 0, 0, 1};
         else jobs[b] = {b < C ? PANEL_LEAD : PANEL_HELP, 0, b, ncta};
     }
     thread_body = [&] {
         emu::Cta* c = emu::cur->cta;
         const PanelJob job = jobs[c->bid];
+        const PanelGroups G{jobs.data(), nullptr, &bar, &status, 0, C};
+        PanelSmem<T>& S = *reinterpret_cast<PanelSmem<T>*>(c->smem);
         unsigned xn = 0;
-        if (job.role != PANEL_IDLE)
-            pp_front<T, STRUCT>(A, job, *reinterpret_cast<PanelSmem<T>*>(c->smem), C, &bar, &status, xn);
+        if (job.role != PANEL_IDLE) pp_front<T, STRUCT>(A, job, S, G, xn);
         pp_cluster_barrier();
+        emu::cur->lingers = S.dead != 0;
+        while (emu::cur->blocked()) emu::yield();
+        emu::cur->lingers = false;
     };
     for (auto* x : emu::fibers) delete x;
     emu::fibers.clear();
@@ -608,6 +670,8 @@ static bool check(int f, int w, int C, int nclusters, int values, const Options&
             emu::fibers.push_back(x);
         }
     emu_group_arrived = 0;
+    emu::given_up = false;
+    emu::first_expiry = give_up ? emu::progress + (long)(g() % (60000 + 100 * w * ncta)) : -1;
     emu::run();
 
     bool ok = true;
@@ -615,6 +679,18 @@ static bool check(int f, int w, int C, int nclusters, int values, const Options&
         if (ok) printf("%s differs at %ld: ", what, (long)at);
         ok = false;
     };
+    if (give_up && status) {   // the panels are what they are; nothing around them has changed
+        for (int64_t q = 0; q < GUARD; ++q)
+            for (auto* v : {&P2, &U2})
+                if ((*v)[q] != T(777) || (*v)[len + GUARD + q] != T(777)) fail("a guard", q);
+        for (int i = 0; i < PAD; ++i)
+            if (scratch[i] != 777.0 || scratch[scratch.size() - 1 - i] != 777.0) fail("the scratch's guard", i);
+        printf("%s %s FP%zu f %d w %d, %d clusters of %d: given up\n", ok ? "ok" : "FAIL", GEN ? "LU" : "LDLT", 8 * sizeof(T), f, w,
+               nclusters, C);
+        fflush(stdout);
+        return ok;
+    }
+    if (status) fail("the status word", 0);
     for (int64_t q = 0; q < len + 2 * GUARD; ++q) {
         if (!same(P1[q], P2[q])) fail("the panel", q - GUARD);
         if (GEN && !same(U1[q], U2[q])) fail("the U^T panel", q - GUARD);
@@ -637,15 +713,17 @@ static bool check(int f, int w, int C, int nclusters, int values, const Options&
     return ok;
 }
 
-static bool check_any(bool gen, bool fp32, int f, int w, int C, int nclusters, int values, const Options& o, unsigned seed) {
-    if (gen) return fp32 ? check<float, STRUCT_G>(f, w, C, nclusters, values, o, seed)
-                         : check<double, STRUCT_G>(f, w, C, nclusters, values, o, seed);
-    return fp32 ? check<float, STRUCT_S>(f, w, C, nclusters, values, o, seed)
-                : check<double, STRUCT_S>(f, w, C, nclusters, values, o, seed);
+static bool check_any(bool gen, bool fp32, int f, int w, int C, int nclusters, int values, const Options& o, unsigned seed,
+                      bool give_up = false) {
+    if (gen) return fp32 ? check<float, STRUCT_G>(f, w, C, nclusters, values, o, seed, give_up)
+                         : check<double, STRUCT_G>(f, w, C, nclusters, values, o, seed, give_up);
+    return fp32 ? check<float, STRUCT_S>(f, w, C, nclusters, values, o, seed, give_up)
+                : check<double, STRUCT_S>(f, w, C, nclusters, values, o, seed, give_up);
 }
 
 int main(int argc, char** argv) {
     const unsigned seed = argc > 1 ? atoi(argv[1]) : 1;
+    const bool give_up = argc > 3 && !strcmp(argv[3], "giveup");
     std::mt19937 g(seed);
     emu::rng.seed(seed);
     auto pick = [&](std::initializer_list<double> v) { return v.begin()[g() % v.size()]; };
@@ -662,14 +740,14 @@ int main(int argc, char** argv) {
     } else {
         for (int n = argc > 2 ? atoi(argv[2]) : 20, q = 0; q < n; ++q) {
             const int w = 1 + g() % (q % 3 == 0 ? 40 : 110), f = w + (g() % 4 == 0 ? 0 : g() % 200);
-            const int C = (int)pick({1, 2, 4, 8}), nclusters = C == 1 || C == 8 ? 1 : 1 + g() % 2;
+            const int C = give_up ? (int)pick({2, 4, 8}) : (int)pick({1, 2, 4, 8}), nclusters = C == 1 || C == 8 ? 1 : 1 + g() % 2;
             Options o;
             o.u = pick({0.01, 0.1, 0.5, 0.9, 1.0});
             o.eps = pick({1e-13, 1e-13, 0.0, 0.5});
             const bool gen = g() % 3 == 0;
             if (!gen) o.pivot = (int)pick({(double)PIVOT_BK, (double)PIVOT_BK, (double)PIVOT_BK, (double)PIVOT_NONE, (double)PIVOT_DIAGONAL});
             else o.lu_pivot = g() % 4 != 0;
-            ok &= check_any(gen, g() % 3 == 0, f, w, C, nclusters, g() % NVALUES, o, g());
+            ok &= check_any(gen, g() % 3 == 0, f, w, C, nclusters, g() % NVALUES, o, g(), give_up);
         }
     }
     printf(ok ? "all ok\n" : "FAILED\n");
