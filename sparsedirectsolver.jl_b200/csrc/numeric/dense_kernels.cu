@@ -331,6 +331,7 @@ struct CholStepSmem {
     T LT[CS_H][CS_H];                 // the half's columns below the diagonal: LT[j][e] = L(j + 1 + e, j)
     T rdiag[CS_H];
     int status;
+    int failed;                       // an earlier step of this front failed
 };
 
 template <typename T>
@@ -443,6 +444,8 @@ __global__ void __launch_bounds__(CS_THREADS) chol_step_kernel(CholStepArgs<T> A
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = r1 + max(task.tile, 0) * TR;
     const int rows = task.tile >= 0 ? min(TR, f - row0) : 0;
+    // read once for the whole CTA: the step's head may be writing it
+    if (tid == 0) S.failed = finfo[s];
     // the block (beyond its columns: the identity) and the tile (zeros), every load before the first store
     {
         constexpr int U = NB * NB / CS_THREADS;
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(CS_THREADS) chol_step_kernel(CholStepArgs<T> A
         }
     }
     __syncthreads();
-    if (finfo[s] != 0) return;   // an earlier step of this front failed
+    if (S.failed != 0) return;
     const T eps = (T)A.eps;
     int status = 0;
     for (int h = 0; h < nbb; h += CS_H) {
