@@ -369,8 +369,17 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         for (const DFront& F : P->fronts)
             if (F.f > FSMALL_DEFAULT && F.f <= FSMALL_MANY) level_many[F.level] += P->nbatch;
         const bool spd = P->structure == STRUCT_SPD;
+        // the shared-memory kernel takes a child's rows in any order, the large-front assembly increasing ones only
+        // (as the analysis gives them): a plan made by hand keeps its fronts there while they fit
+        std::vector<char> unordered(ns, 0);
+        for (const DFront& C : P->fronts)
+            for (int t = 1; C.parent >= 0 && t < C.f - C.w; ++t)
+                if (relind[C.ri_begin + t] <= relind[C.ri_begin + t - 1]) {
+                    unordered[C.parent] = 1;
+                    break;
+                }
         auto fsmall_of = [&](const DFront& F) {
-            if (tune_fsmall || (!spd && P->nbatch > 1)) return classes.back();
+            if (tune_fsmall || (!spd && P->nbatch > 1) || unordered[&F - P->fronts.data()]) return classes.back();
             return spd && level_many[F.level] >= FSMALL_MANY_FRONTS ? FSMALL_MANY : FSMALL_DEFAULT;
         };
         // 0: a large front
