@@ -7,20 +7,24 @@
 // at once: the block's rows are solved against its unit triangle (T1), then every entry takes the block's
 // products one after another (T2), by the leader and the front's helper CTAs.
 //
-// What bounds it: the chain of pivot steps, 1.8 us a column with everything (lap3d 40^3 "S": 9.6 ms over the
-// 5477 columns of the tree's wide fronts, level by level; 40^3 LU 11.2 ms; with every pivot row sent by the CTA
-// that holds it 10.8 and 12.3 ms; with the statistics in every thread and D written inside the chain as well
-// 12.2 ms "S"; with plain remote stores and a cluster barrier per step 14.4 and
-// 14.1 ms; the cooperative kernel's two group barriers a column in global memory 58.8 and 71.3 ms). The
+// What bounds it: the chain of pivot steps, 1.6 us a column with everything (lap3d 40^3 "S": 8.9 ms over the
+// 5477 columns of the tree's wide fronts, level by level; 40^3 LU 10.4 ms; with the loop's short loops unrolled 9.7
+// and 11.0 ms; with every pivot row sent by the CTA that holds it as well 10.8 and 12.3 ms; with the statistics in
+// every thread and D written inside the chain as well 12.2 ms "S"; with plain remote stores and a cluster barrier per
+// step 14.4 and 14.1 ms; the cooperative kernel's two group barriers a column in global memory 58.8 and 71.3 ms). The
 // updates run at a few percent of the FP64 rate; T2's tiles double-buffered cost LU 14.7 ms (registers).
 //
 // Every entry receives the products of ldlt_front_steps / lu_front_steps (front_factor.cuh) in the same
 // order, each product and difference rounded on its own, and every pivot decision sees the same values, so
 // pivots, D and panels are those of the one-CTA kernel bit for bit.
 //
-// A pivot that needs a column outside the block (a Bunch-Kaufman partner, or the search over all diagonals
-// after a rejected choice) is taken only as a block's first one, where the whole front is up to date: a
-// later one ends the block early.
+// A Bunch-Kaufman partner may lie outside the block. Its column is then brought up to date by itself: the block's
+// eliminated rows are solved against their triangle in that column, and every row takes their products (pp_bring).
+// If it becomes a pivot, it takes the place of the block's column, whose values from before the block go where it
+// was, for the block's later products. (Ending the block at every such pivot made a dense random front of 2400
+// columns 48.7 ms and one whose partners are all far 39.9 ms, against 35.9 and 31.7 ms of the cooperative kernel.)
+// The search over all diagonals after a rejected choice needs the whole front up to date: it ends the block, unless
+// the rejected one is its first.
 #pragma once
 #include <stdint.h>
 
@@ -58,7 +62,8 @@ struct PanelSmem {
     int st[NSTAT];                                         // the statistics (thread 0 of the leader's first CTA)
     double red[PP_WARPS];
     int redi[PP_WARPS];
-    PanelHdr<T> hdr;                                       // T1 / T2: the block's header
+    PanelHdr<T> hdr;                                       // T1 / T2: the block's header; "S", between them: the pivot rows'
+                                                           // multipliers and first places that pp_bring needs
     union {
         T L[PP_NB][PP_THREADS];                            // the block: the rows' multipliers
         struct {
@@ -190,8 +195,8 @@ struct PanelX {
     const int C, rank, nw;
     int b;
     unsigned xn;
-    __device__ PanelX(const PanelFront<T, GEN>& F, PanelSmem<T>& S_, int nw_)
-        : S(S_), C(F.C), rank(F.rank), nw(nw_), b(0), xn(F.xn) {}
+    __device__ PanelX(PanelSmem<T>& S_, int C_, int rank_, int nw_, unsigned xn_)
+        : S(S_), C(C_), rank(rank_), nw(nw_), b(0), xn(xn_) {}
     // opens the next exchange, of `bytes` bytes into each CTA
     __device__ __forceinline__ void open(int bytes) {
         b = xn & 1;
@@ -259,6 +264,7 @@ struct PanelX {
         __syncwarp();
         if (C > 1) {
             const int lane = threadIdx.x & 31, per = 32 / C, q = lane / per, ch = (left + 2) / 2;
+#pragma unroll 1
             for (int c = lane % per; c < ch; c += per) pp_x_store2(row + 2 * c, q, row[2 * c], row[2 * c + 1], &S.mbar[b]);
         }
     }
@@ -275,6 +281,7 @@ struct PanelTeam {
         if ((rank & 31) == 0) red[rank >> 5] = v;
         pp_warps_barrier(size);
         double r = red[0];
+#pragma unroll 1
         for (int w = 1; w < (size >> 5); ++w) r = jmax(r, red[w]);
         return r;
     }
@@ -288,6 +295,7 @@ struct PanelTeam {
         pp_warps_barrier(size);
         v = red[0];
         idx = redi[0];
+#pragma unroll 1
         for (int w = 1; w < (size >> 5); ++w)
             if (red[w] > v || (red[w] == v && redi[w] >= 0 && (idx < 0 || redi[w] < idx))) {
                 v = red[w];
@@ -308,6 +316,7 @@ __device__ void pp_search(const PanelFront<T, GEN>& F, PanelSmem<T>& S, int nw, 
     while (true) {
         double a = -1.0;
         int j = -1;
+#pragma unroll 1
         for (int i = k + tm.rank; i < F.w; i += tm.size) {
             const double x = fabs(F.get(i, i));
             if (!(x >= eps)) continue;
@@ -324,6 +333,7 @@ __device__ void pp_search(const PanelFront<T, GEN>& F, PanelSmem<T>& S, int nw, 
         const double a0 = fabs(F.get(k, k));
         double a = -1.0;
         int j = -1;
+#pragma unroll 1
         for (int i = k + 1 + tm.rank; i < F.w; i += tm.size) {
             const double x = fabs(F.get(i, i));
             if (x > a) { a = x; j = i; }
@@ -337,6 +347,51 @@ __device__ void pp_search(const PanelFront<T, GEN>& F, PanelSmem<T>& S, int nw, 
     c_out = bc;
 }
 
+// The row's up-to-date entry of column r, outside the block, behind the block's first j steps (of which `firsts` begin
+// a 2x2 pair); 0 for finished rows. Pivot rows sent .. j - 1 send their multipliers first (exchange xn). Every warp
+// solves the column's entries of the pivot rows for itself, row t by lane t, while its rows take the products. A
+// call, so that the step's loop stays small.
+template <typename T>
+struct PanelEntry {
+    T v;
+    int ok;   // 0: a wait gave up
+};
+template <typename T>
+__device__ __noinline__ PanelEntry<T> pp_bring(PanelSmem<T>& S, const T* column, int C, int rank, int nw, unsigned xn, int k0, int j,
+                                               int sent, unsigned firsts, int rp, int src, int spare) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    T v = rp >= k0 + j ? __ldcg(column + src) : T(0);
+    if (j == 0) return {v, 1};
+    if (sent < j) {
+        PanelX<T, false> X(S, C, rank, nw, xn);
+        X.open(X.join_bytes() + (j - sent) * 4 + (j * (j - 1) - sent * (sent - 1)) / 2 * (int)sizeof(T));
+        X.join();
+        for (int t = sent; t < j; ++t) {
+            const unsigned own = __ballot_sync(0xffffffffu, rp == k0 + t && !spare);
+            if (own == 0) continue;
+            const int o = __ffs(own) - 1, at = __shfl_sync(0xffffffffu, src, o);
+            if (lane < C) X.put(&S.hdr.rowmap[t], lane, at);
+            for (int i = lane; i < C * t; i += 32) X.put(&S.hdr.lt[i % t][t], i / t, S.L[i % t][tid - lane + o]);
+        }
+        if (!X.close()) return {T(0), 0};
+    }
+    T g = lane < j ? __ldcg(column + S.hdr.rowmap[lane]) : T(0);
+    for (int s = 0; s < j;) {
+        const T u = __shfl_sync(0xffffffffu, g, s);
+        if (firsts >> s & 1) {
+            const T u1 = __shfl_sync(0xffffffffu, g, s + 1);
+            if (lane > s + 1) g -= S.hdr.lt[s][lane] * u + S.hdr.lt[s + 1][lane] * u1;
+            if (rp >= k0 + j) v -= S.L[s][tid] * u + S.L[s + 1][tid] * u1;
+            s += 2;
+        } else {
+            if (lane > s) g -= S.hdr.lt[s][lane] * u;
+            if (rp >= k0 + j) v -= S.L[s][tid] * u;
+            s += 1;
+        }
+    }
+    return {v, 1};
+}
+
 struct PanelPivot {
     int pivot, lu_pivot;
     double u, eps;
@@ -348,7 +403,9 @@ struct PanelPivot {
 // that is left, or -1 (the whole CTA) after a wait that gave up.
 //
 // A step is a chain of latencies, not of work: the maxima to the other CTAs, the decision,
-// a division, the update of up to 31 columns.
+// a division, the update of up to 31 columns. The loop over the steps has to stay small for the instruction caches:
+// short loops in it are not unrolled (pivot launches 9.7 -> 8.9 ms lap3d 40^3 "S", 16.6 -> 15.6 KKT 80 x 75, 11.0 ->
+// 10.4 40^3 LU).
 template <typename T, int STRUCT>
 __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, const PanelPivot& pv, int k0) {
     constexpr bool GEN = STRUCT == STRUCT_G;
@@ -368,21 +425,21 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
     int rp = src;                       // the row's place; a finished row keeps its own (<= k)
     T a[PP_NB];                         // the row's entries of columns k, k + 1, ...: the columns move down by one
                                         // with every eliminated one, so that no index depends on k
-    int mylp = 0;
     const double alpha = (1.0 + sqrt(17.0)) / 8.0;
-    auto load = [&]() {
 #pragma unroll
-        for (int e = 0; e < PP_NB; ++e) a[e] = (src >= 0 && e < nb) ? F.at(src, k0 + e) : T(0);
-        mylp = (orig >= 0 && orig < w) ? F.lp[orig] : 0;
-    };
-    load();
+    for (int e = 0; e < PP_NB; ++e) a[e] = (src >= 0 && e < nb) ? F.at(src, k0 + e) : T(0);
+    const int mylp = (orig >= 0 && orig < w) ? F.lp[orig] : 0;
     // the next block's counters: the last one's, which every CTA has read, and the meetings of the group behind this
     // block come before anyone counts in them
     if (rank == 0 && tid == 0) F.hdr->ndisp[F.par ^ 1] = F.hdr->moved[F.par ^ 1] = 0;
     if (warp < nw) {
-        PanelX<T, GEN> X(F, S, nw);
+        PanelX<T, GEN> X(S, C, rank, nw, F.xn);
         int j = 0;
         bool gave_up = false;
+        // "S", lane e: where in the block column k0 + e was when it began; step e begins a 2x2 pair; every CTA has
+        // pivot row e's multipliers (for pp_bring: in one register, of which the steps without it need none)
+        constexpr int FIRST = PP_NB, SENT = 2 * PP_NB;
+        int from = lane;
         while (j < nb) {
             const int k = k0 + j, left = nb - j;   // columns k .. kend - 1
             // a bound of the column below row k, and row k itself, to every leader CTA
@@ -393,6 +450,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
             if (!copies) X.row(a, rp, k, j, left);
             // (no entry's part is all ones: its sign is cleared)
             h = X.close_lane() ? 0u : 0xffffffffu;
+#pragma unroll 1
             for (int i = lane; i < nparts; i += 32) h = max(h, S.hi[X.b][i]);
             h = __reduce_max_sync(0xffffffffu, h);
             if (h == 0xffffffffu) { gave_up = true; break; }
@@ -405,6 +463,8 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
             else if (pv.pivot == PIVOT_NONE) fast = true;
             else fast = akk >= pv.eps && akk >= pv.u * bound && (pv.pivot == PIVOT_DIAGONAL || akk >= alpha * bound);
             int c = k, r2 = -1;
+            bool searched = false;
+            T v;                                         // "S": the row's entry of the partner's column
             if (!fast) {
                 const unsigned long long key = rp > k ? pp_key(a[0]) : 0ull;
                 const unsigned long long mkey = pp_warp_max<T>(key);
@@ -421,6 +481,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                 if (!X.close()) { gave_up = true; break; }
                 unsigned long long lk = 0, mk = 0;
                 int r = 0x7fffffff;
+#pragma unroll 1
                 for (int i = lane; i < nparts; i += 32) {
                     const unsigned long long l = S.lam[i], m = S.mx[i];
                     const int x = S.ridx[i];
@@ -434,13 +495,22 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                 } else {
                     bool acc;
                     int bc = k, br = -1;
+                    v = T(0);
                     if (pv.pivot == PIVOT_DIAGONAL || r < 0 || akk >= alpha * lambda) {
                         acc = akk >= pv.eps && akk >= pv.u * mall;
                     } else {
-                        if (r >= kend && j > 0) break;   // the partner's column is not up to date
                         // column r: its maxima, those of column k without row r, and the corner entries
-                        T v = T(0);
-                        if (rp >= k) v = r < kend ? pp_pick(a, r - k) : F.at(src, r);
+                        if (r >= kend) {
+                            const unsigned firsts = __ballot_sync(0xffffffffu, from & FIRST);
+                            const int sent = __popc(__ballot_sync(0xffffffffu, from & SENT));
+                            const PanelEntry<T> e = pp_bring<T>(S, &F.at(0, r), C, rank, nw, X.xn, k0, j, sent, firsts, rp, src, spare);
+                            X.xn += sent < j;
+                            if (lane < j) from |= SENT;
+                            if (!e.ok) { gave_up = true; break; }
+                            v = e.v;
+                        } else if (rp >= k) {
+                            v = pp_pick(a, r - k);
+                        }
                         const unsigned long long kv = rp >= k && rp != r ? pp_key(v) : 0ull;
                         unsigned long long s1 = pp_warp_max<T>(rp < w ? kv : 0ull);
                         unsigned long long s2 = pp_warp_max<T>(rp != k ? kv : 0ull);
@@ -453,14 +523,17 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                             X.put(&S.m1[at], lane, s3);
                         }
                         if (rp == r && !spare)
+#pragma unroll 1
                             for (int q = 0; q < C; ++q) {
                                 X.put(&S.sc[0], q, v);
                                 X.put(&S.sc[2], q, a[0]);
                             }
                         if (rp == k && !spare)
+#pragma unroll 1
                             for (int q = 0; q < C; ++q) X.put(&S.sc[1], q, v);
                         if (!X.close()) { gave_up = true; break; }
                         s1 = s2 = s3 = 0;
+#pragma unroll 1
                         for (int i = lane; i < nparts; i += 32) {
                             if (S.sg[i] > s1) s1 = S.sg[i];
                             if (S.m2[i] > s2) s2 = S.m2[i];
@@ -488,7 +561,9 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                     }
                     c = bc;
                     r2 = br;
+                    if (acc && br >= 0 && left < 2) break;   // a pair needs two of the block's columns
                     if (!acc) {
+                        searched = true;
                         if (j > 0) break;                // the search needs the whole front up to date
                         X.open(X.join_bytes() + 8);
                         if (rank == 0) {
@@ -499,6 +574,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                             int cs = k, rs = -1;
                             pp_search(F, S, nw, k, pv.pivot, pv.u, pv.eps, bc, br, cs, rs);
                             if (tid == 0)
+#pragma unroll 1
                                 for (int q = 0; q < C; ++q) {
                                     X.put(&S.sel[0], q, cs);
                                     X.put(&S.sel[1], q, rs);
@@ -525,36 +601,28 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         }
                         if (rp == p) rp = q;
                         else if (rp == q) rp = p;
+                        if (!GEN) {
+                            const int fp = __shfl_sync(0xffffffffu, from, p - k0), fq = __shfl_sync(0xffffffffu, from, q - k0);
+                            if (lane == p - k0) from = fq;   // (neither is eliminated: no other bits)
+                            else if (lane == q - k0) from = fp;
+                        }
                     } else if (p != q && GEN) {          // row interchange: rows change places, their data stay
                         if (rp == p) rp = q;
                         else if (rp == q) rp = p;
-                    } else if (p != q) {                 // outside it (j = 0): the interchange in memory
-                        const int gt = rank * nw * 32 + tid, GT = C * nw * 32;
-                        for (int i = gt; i < f; i += GT) {
-                            if (i == p || i == q) continue;
-                            const T t = F.at(i, p);
-                            F.at(i, p) = F.at(i, q);
-                            F.at(i, q) = t;
+                    } else if (p != q) {                 // outside it: v, and the old column's first values for later
+                        if (searched) {                  // (j = 0: every column is up to date)
+                            v = rp >= k ? F.at(src, q) : T(0);
+                            if (!X.meet()) { gave_up = true; break; }
                         }
-                        for (int i = gt; i < w; i += GT) {
-                            if (i == p || i == q) continue;
-                            const T t = F.at(p, i);
-                            F.at(p, i) = F.at(q, i);
-                            F.at(q, i) = t;
+                        if (rp >= k) {
+                            if (p == k) a[0] = v;
+                            else a[1] = v;
                         }
-                        if (gt == 0) {
-                            T t = F.at(p, p);
-                            F.at(p, p) = F.at(q, q);
-                            F.at(q, q) = t;
-                            t = F.at(p, q);
-                            F.at(p, q) = F.at(q, p);
-                            F.at(q, p) = t;
-                            const int tl = F.lp[p];
-                            F.lp[p] = F.lp[q];
-                            F.lp[q] = tl;
-                        }
-                        if (!X.meet()) { gave_up = true; break; }
-                        load();
+                        if (rp == p) rp = q;
+                        else if (rp == q) rp = p;
+                        const int m = __shfl_sync(0xffffffffu, from, p - k0);
+                        if (orig >= 0) F.at(orig, q) = F.at(orig, k0 + m);
+                        __threadfence();                 // (pp_bring reads past the first-level cache)
                     }
                     X.open(X.join_bytes() + (r2 >= 0 ? 2 : 1) * X.row_bytes(left));
                     X.join();
@@ -573,6 +641,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         X.open(X.join_bytes() + 4);
                         X.join();
                         if (rp == k && !spare)
+#pragma unroll 1
                             for (int q = 0; q < C; ++q) X.put(&S.plp, q, mylp);
                         if (!X.close()) { gave_up = true; break; }
                         lpk = S.plp;
@@ -611,6 +680,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                 }
                 j += 1;
             } else {
+                if (lane == j) from |= FIRST;
                 const double fa = (double)S.prow[j][1], fb = (double)S.prow[j + 1][1], fc = (double)S.prow[j + 1][2];
                 const double det = fa * fc - fb * fb;
                 const double e11 = fc / det, e12 = -fb / det, e21 = -fb / det, e22 = fa / det;

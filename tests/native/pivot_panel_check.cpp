@@ -220,6 +220,9 @@ void run() {
 
 }  // namespace emu
 
+#undef __noinline__
+#define __noinline__
+
 // --- what the kernel's code calls ----------------------------------------------------------------------------------
 static uint3 emu_thread() { return emu::cur->tid; }
 #define threadIdx emu_thread()
@@ -234,6 +237,11 @@ static unsigned __ballot_sync(unsigned, int p) {
     for (int i = 0; i < 32; ++i) r |= v[i] ? 1u << i : 0u;
     return r;
 }
+template <class X>
+static X __ldcg(const X* p) {
+    return *p;
+}
+static int __ffs(unsigned x) { return __builtin_ffs((int)x); }
 static int __popc(unsigned x) { return __builtin_popcount(x); }
 static unsigned __reduce_max_sync(unsigned, unsigned x) {
     const unsigned long long* v = emu::warp_sync(x);
