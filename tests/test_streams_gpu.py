@@ -1,0 +1,46 @@
+"""One plan called on two streams in turn, with no wait between the calls: they share the plan's working vectors, so
+each must wait for the last, whether its launches go out directly (the one-launch solve, a first factorization) or
+as a recorded graph (the per-level solve, a repeated factorization)."""
+import numpy as np
+import pytest
+
+from sdsb200 import matrices as M
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ir", [0, 1])
+@pytest.mark.parametrize("structure", ["SPD", "G"])
+def test_solves_on_two_streams(structure, ir):
+    import torch
+
+    from sdsb200._native import numeric_lib
+    from sdsb200.solver import DirectSolver
+
+    A = M.lap3d(24, 24, 24, seed=6) if structure == "SPD" else M.convection_diffusion3d(18, 18, 18, seed=6)
+    n, nrhs = A.shape[0], 8
+    ds = DirectSolver(A, structure, reordering_alg="nd", max_nrhs=nrhs, ir_n_steps=ir)
+    ds.execute("analysis")
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    b = [torch.from_numpy(np.random.default_rng(q).uniform(-1, 1, (n, nrhs))).cuda() for q in range(2)]
+    torch.cuda.synchronize()
+    lib = numeric_lib()
+    want = {}
+    for mode in (1, 0):
+        lib.sdsb200_set_persistent(ds._plan, mode)
+        assert ds.execute("factorization") == 0
+        for q in range(2):
+            want[mode, q] = ds.execute("solve", None, b[q]).clone()
+            torch.cuda.synchronize()
+    got = []
+    for rep in range(12):
+        for q, mode in ((0, 1), (1, 1), (0, 0), (1, 1), (0, 1), (1, 0)):
+            lib.sdsb200_set_persistent(ds._plan, mode)
+            with torch.cuda.stream(streams[q]):
+                got.append((mode, q, ds.execute("solve", None, b[q])))
+                got[-1][2].record_stream(streams[q])
+        with torch.cuda.stream(streams[rep % 2]):
+            assert ds.execute("refactorization") == 0   # the same values, the same factor
+    torch.cuda.synchronize()
+    for mode, q, x in got:
+        assert torch.equal(x, want[mode, q]), (mode, q)
