@@ -205,18 +205,20 @@ int sdsb200_get_factor(sdsb200_plan* plan, int32_t member, double* h_factor, dou
 /* ubatch_index / ubatch_mask: restrict later calls to h_members (0-based), nact of them; nact < 0 = all. */
 int sdsb200_set_members(sdsb200_plan* plan, const int32_t* h_members, int32_t nact);
 
-/* user_host_interrupt: a host flag polled between launch groups (factorization) and refinement steps. */
+/* user_host_interrupt: a host flag polled before a factorization and each refinement step, and between the launch
+ * groups of a factorization that is not a graph's replay or recording (sdsb200_set_graphs). */
 int sdsb200_set_interrupt(sdsb200_plan* plan, const volatile int32_t* h_flag);
 
-/* CUDA graphs (on by default): the launch program of sdsb200_factor and of the solve / refinement
- * steps is captured once per set of buffers and options and replayed. The user_host_interrupt flag is
- * then polled before a factorization and before each refinement step, not between launch groups. */
+/* CUDA graphs (on by default): sdsb200_factor launches directly in the first call with a set of buffers and
+ * options, records its launch program into a graph in the second in a row and replays it from then on; the per-level
+ * solve and its refinement steps are recorded in the first call. The one-launch solve needs no graph. The
+ * user_host_interrupt flag is polled between launch groups in calls that launch directly only. */
 int sdsb200_set_graphs(sdsb200_plan* plan, int32_t on);
 
-/* Solve engine. Nonzero (default): the dataflow solve, one cooperative persistent launch per group of
- * 8 right-hand sides with no grid barrier (tasks in a topological order of the elimination tree,
- * synchronised by per-front counters and per-block flags; a uniform batch runs every active member's
- * tasks in the same launch); 0: one launch per level and sweep (the engine of the solve sub-phases). */
+/* Solve engine. Nonzero (default): the dataflow solve, one cooperative persistent launch per 32
+ * right-hand sides of a single system or 8 of a uniform batch, with no grid barrier (tasks in a topological
+ * order of the elimination tree, synchronised by per-front counters and per-block flags; groups of 8
+ * right-hand sides, or every active member of a batch, run their tasks in the same launch); 0: one launch per level and sweep (the engine of the solve sub-phases). */
 int sdsb200_set_persistent(sdsb200_plan* plan, int32_t on);
 
 /* Longest wait, in ns, of the CTAs of a wide LDLT / LU front for one another (2e9 by default). A factorization in
@@ -265,13 +267,13 @@ int sdsb200_sampled_outer(int64_t n, int64_t nnz, const void* rowptr, const void
                           void* stream);
 
 /* Solve without allocating (no counterpart in the reference): op(A) X = B for one active batch member,
- * no refinement, as two small memsets (the status word; the plan's flag and counter buffer, which is
+ * no refinement, as small memsets (the status word; the plan's flag and counter buffer, which is
  * plan memory allocated at plan creation and shared by every solve on the plan) and one cooperative
- * kernel launch per group of 8 right-hand sides. On a plan with an FP32 factor it returns the
+ * kernel launch per 32 right-hand sides. On a plan with an FP32 factor it returns the
  * unrefined solution through that factor (FP32 accuracy); refine it with sdsb200_residual and further
  * calls when FP64 accuracy is needed. sdsb200_solve keeps its
- * working vectors in the plan and records its launches into a CUDA graph per set of buffers, and
- * building that graph makes the driver allocate device memory on the first call with new buffers.
+ * working vectors in the plan and, with the per-level engine, records its launches into a CUDA graph per set of
+ * buffers, which makes the driver allocate device memory on the first call with new buffers.
  * Callers that may not allocate once set-up is over (a framework whose pool allocator owns all device
  * memory, a real-time loop that forbids allocation after start-up) call this entry point instead:
  * the working vectors Y and xtmp (n * nrhs doubles each) and the update vectors (the plan's ulen

@@ -283,7 +283,7 @@ int run_factor(Plan* P, const double* nzval, double eps, double u, int pivot, in
                 a.copy_src = static_cast<const T*>(P->d_inv);
                 a.copy_stride = P->inv_len;
                 a.exact = sizeof(T) == 8 ? L.exact : 0;
-                // FP32: the panel steps' rank-32 updates (C in the factor) on the SIMT pipes; the
+                // FP32: the panel steps' rank-64 updates (C in the factor) on the SIMT pipes; the
                 // contribution-block (Schur complement) updates on the tensor cores
                 a.simt = (sizeof(T) == 4 && L.cbuf == BUF_FACTOR) ? 1 : 0;
                 e = launch_gemm<T>(a, nm, st);
@@ -545,8 +545,8 @@ int run_sweeps(Plan* P, int nrhs, bool transpose, cudaStream_t st, int which) {
     return SDSB200_OK;
 }
 
-// the whole solve as dataflow tasks in one persistent launch per group of up to DF_MAX_NRHS
-// right-hand sides (solve_dataflow.cu)
+// the whole solve as dataflow tasks in one persistent launch (solve_dataflow.cu), of up to DF_MAX_GROUPS groups of
+// DF_MAX_NRHS right-hand sides of one system, or of one group for every active member of a batch
 template <typename T>
 int run_dataflow(Plan* P, int nrhs, bool transpose, const double* in, int64_t ldin, double* out, int64_t ldout,
                  int mode, cudaStream_t st) {

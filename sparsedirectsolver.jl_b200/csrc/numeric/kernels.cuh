@@ -62,11 +62,6 @@ struct StatsArgs {
     int32_t ns;
 };
 
-// Large Cholesky column-block panel: diagonal block + trsm of the rows below.
-
-
-// Diagonal block of a large Cholesky front: factor in place and write its inverse (ld 64) to scratch.
-
 // One task of a large-Cholesky step: a 64-row tile of the rows below the diagonal block of front
 // `front` (tile >= 0), or the diagonal block alone when no rows are below it (tile = -1). The task
 // with tile <= 0 is the step's head: it records the statistics and puts L11 at `scr` of the scratch
@@ -162,7 +157,7 @@ struct GemmArgs {
     int64_t copy_stride;   // per-member stride of copy_src
     int32_t exact;     // FP64 mode-0 tiles summed in the oracle's order, every product and sum rounded:
                        // 1 (LDLT) c = c - a_k b_k for k = 0, 1, ...; 2 (LU) c = c - (a_0 b_0 + a_1 b_1 + ...)
-    int32_t simt;      // FP32: the SIMT kernel (the panel steps' rank-32 updates) instead of tcgen05
+    int32_t simt;      // FP32: the SIMT kernel (the panel steps' rank-64 updates) instead of tcgen05
 };
 
 // FP32 grouped GEMM on the tensor cores (tcgen05, 3xTF32); tc_kernels.cu
@@ -281,7 +276,7 @@ constexpr int CHOL_NB = 64;   // column block of the large-front Cholesky steps
 constexpr int FLOW_NB = 32;   // column block of the dataflow steps (CholFlowArgs)
 cudaError_t prepare_factor_kernels(int max_smem);
 cudaError_t prepare_dense_kernels(int max_smem);
-cudaError_t prepare_solve_kernels(int max_smem);   // column block of the large-front Cholesky
+cudaError_t prepare_solve_kernels(int max_smem);
 template <typename T>
 cudaError_t launch_large_pivot(int structure, const LargePivotArgs<T>& a, int nmembers, cudaStream_t st);
 template <typename T>

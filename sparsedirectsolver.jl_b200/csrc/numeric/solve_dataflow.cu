@@ -490,19 +490,25 @@ __device__ __noinline__ void df_narrow_backward(const DataflowArgs<T>& A, int s,
 template <typename T, int NR>
 __device__ __forceinline__ void df_warp_front(const DataflowArgs<T>& A, int s, bool forward, double* z, int64_t* stamp) {
     const int f = A.fronts[s].f, w = A.fronts[s].w;
-    if (NR <= 4 && w <= 8 && f <= 32) {
-        if (forward) df_warp_forward<T, NR, 8, 1>(A, s, z, stamp);
-        else df_narrow_backward<T, NR, 1>(A, s, z, stamp);
-    } else if (NR <= 4 && w <= 8 && f <= 64) {
-        if (forward) df_warp_forward<T, NR, 8, 2>(A, s, z, stamp);
-        else df_narrow_backward<T, NR, 2>(A, s, z, stamp);
-    } else if (NR <= 4 && w <= 16 && f <= 64) {
-        if (forward) df_warp_forward<T, NR, 16, 2>(A, s, z, stamp);
-        else df_warp_backward<T, NR, 16, 2>(A, s, z, stamp);
-    } else {
-        if (forward) df_warp_forward<T, NR, DF_WARP_W, 4>(A, s, z, stamp);
-        else df_warp_backward<T, NR, DF_WARP_W, 4>(A, s, z, stamp);
+    if constexpr (NR <= 4) {
+        if (w <= 8 && f <= 32) {
+            if (forward) df_warp_forward<T, NR, 8, 1>(A, s, z, stamp);
+            else df_narrow_backward<T, NR, 1>(A, s, z, stamp);
+            return;
+        }
+        if (w <= 8 && f <= 64) {
+            if (forward) df_warp_forward<T, NR, 8, 2>(A, s, z, stamp);
+            else df_narrow_backward<T, NR, 2>(A, s, z, stamp);
+            return;
+        }
+        if (w <= 16 && f <= 64) {
+            if (forward) df_warp_forward<T, NR, 16, 2>(A, s, z, stamp);
+            else df_warp_backward<T, NR, 16, 2>(A, s, z, stamp);
+            return;
+        }
     }
+    if (forward) df_warp_forward<T, NR, DF_WARP_W, 4>(A, s, z, stamp);
+    else df_warp_backward<T, NR, DF_WARP_W, 4>(A, s, z, stamp);
 }
 
 // ---------------------------------------------------------------------------------------------------

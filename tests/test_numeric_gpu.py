@@ -175,8 +175,8 @@ def test_lu_convection_diffusion(torch_cuda, g):
 @pytest.mark.parametrize("case", ["kkt_ldlt", "cd_lu", "kkt_lu"])
 def test_wide_fronts_many_chunks(torch_cuda, case):
     # fronts of more than two 256-row chunks, and (kkt_ldlt, cd_lu) of more than one 32-column group:
-    # the chunked large-front assembly, and the cooperative kernel's per-chunk column maxima, update
-    # items and deferred multiplier writes; kkt_lu also interchanges hundreds of rows
+    # the chunked large-front assembly, and the panel kernel's blocks, column maxima and update tiles over
+    # clusters of CTAs; kkt_lu also interchanges hundreds of rows
     if case == "kkt_ldlt":
         A, st, kw = small_kkt(40, 40, 600, seed=3), "S", {}
     elif case == "cd_lu":

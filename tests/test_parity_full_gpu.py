@@ -100,7 +100,7 @@ def _berr(ds, A, b, transpose=False):
 
 
 def test_mixed_spd_factor_wide_fronts(torch_cuda):
-    # lap3d 24^3 with ND: fronts wider than 32 columns run the FP32 32-column steps and the 3xTF32
+    # lap3d 24^3 with ND: fronts wider than 32 columns run the FP32 64-column steps and the 3xTF32
     # tensor-core Schur updates; the small fronts run the FP32 shared-memory kernel
     A = M.lap3d(24, 24, 24, seed=5)
     d32 = _solver(A, "SPD", reordering_alg="nd", factor_precision="fp32", ir_n_steps=10, ir_tol=1e-14)
@@ -120,7 +120,7 @@ def test_mixed_spd_factor_wide_fronts(torch_cuda):
 @pytest.mark.parametrize("case", ["kkt20", "kkt40_coop"])
 def test_mixed_ldlt_inertia(torch_cuda, case):
     # Bunch-Kaufman LDL^T with an FP32 factor: the inertia must equal the FP64 oracle's. kkt40_coop
-    # has fronts above 512 rows and 32 columns (the cooperative wide-front kernel).
+    # has fronts above 512 rows and 32 columns (the panel kernel on clusters of CTAs).
     A = small_kkt(20, 20, 150, seed=2) if case == "kkt20" else small_kkt(40, 40, 600, seed=3)
     nh = 400 if case == "kkt20" else 1600
     nj = A.shape[0] - nh
