@@ -103,7 +103,7 @@ typedef struct sdsb200_plan_options {
 /* Plan tuning (the shapes an autotuner chooses; no counterpart in the reference):
  * fsmall = the largest front order handled by the shared-memory small-front kernel (one of 32, 64,
  * 96, 128, 160, and 224 for FP32; 0 = by the plan: 64 rows, 96 for Cholesky levels with many such
- * fronts, the largest class for LDLT and LU batches); wide = the tallest front (at most 32
+ * fronts, 128 for LDLT plans of one or two fronts, the largest class for LDLT and LU batches); wide = the tallest front (at most 32
  * columns) that the dataflow solve gives to one warp, larger fronts going to tile tasks (16..128,
  * 0 = 128); chains = how the dataflow solve treats those tiled fronts: 0, through their inverse
  * panels [L11^-1; L21 L11^-1] (f x w each, built after every factorization of a single-system plan),

@@ -622,7 +622,7 @@ __device__ int pp_block(PanelFront<T, STRUCT == STRUCT_G>& F, PanelSmem<T>& S, c
                         else if (rp == q) rp = p;
                         const int m = __shfl_sync(0xffffffffu, from, p - k0);
                         if (orig >= 0) F.at(orig, q) = F.at(orig, k0 + m);
-                        __threadfence();                 // (pp_bring reads past the first-level cache)
+                        if (C > 1) __threadfence();      // (pp_bring reads past the first-level cache)
                     }
                     X.open(X.join_bytes() + (r2 >= 0 ? 2 : 1) * X.row_bytes(left));
                     X.join();

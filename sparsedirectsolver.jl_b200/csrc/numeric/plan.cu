@@ -364,7 +364,12 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
         // launch has a CTA's front for every SM: 256 uneven systems 1681 / 1679 / 1766 / 1875, uniform batch
         // 96^2 x 256 7094 / 5642 / 5717 / 6332. LDLT and LU batches keep every front that fits: their large
         // fronts run on one CTA each.
-        constexpr int FSMALL_DEFAULT = 64, FSMALL_MANY = 96, FSMALL_MANY_FRONTS = 148;
+        // An LDLT plan of one or two fronts (a dense matrix) keeps those of up to 128 rows as well: there every pivot may
+        // be an interchange with a far column, which the panel kernel pays more for, and nothing else runs beside
+        // the front. Factorization of one dense front, shared memory / panel kernel, us: random values, 66 rows 209 / 282,
+        // 100 rows 312 / 437, 130 rows 472 / 580; diagonally dominant 209 / 171, 320 / 228, 480 / 309. (Sparse indefinite
+        // problems, fronts of up to 64 / up to 160 rows there: lap3d 24^3 - 2 I 5824 / 7626, lap2d 120^2 - 3 I 3710 / 5467.)
+        constexpr int FSMALL_DEFAULT = 64, FSMALL_MANY = 96, FSMALL_MANY_FRONTS = 148, FSMALL_DENSE_S = 128;
         std::vector<int64_t> level_many(P->nlevels, 0);
         for (const DFront& F : P->fronts)
             if (F.f > FSMALL_DEFAULT && F.f <= FSMALL_MANY) level_many[F.level] += P->nbatch;
@@ -380,6 +385,7 @@ Plan* build_plan(const sdsb200_symbolic* sym, const sdsb200_plan_options* popts,
                 }
         auto fsmall_of = [&](const DFront& F) {
             if (tune_fsmall || (!spd && P->nbatch > 1) || unordered[&F - P->fronts.data()]) return classes.back();
+            if (P->structure == STRUCT_S && ns <= 2) return FSMALL_DENSE_S;
             return spd && level_many[F.level] >= FSMALL_MANY_FRONTS ? FSMALL_MANY : FSMALL_DEFAULT;
         };
         // 0: a large front
