@@ -456,17 +456,17 @@ __device__ __noinline__ void df_narrow_backward(const DataflowArgs<T>& A, int s,
         if (r < nrhs) {
 #pragma unroll
             for (int i = 0; i < 8 * K; ++i)
-                if (g + 4 * i < m) acc += (double)lv[i] * x2[g + 4 * i + r * m];
+                if (4 * i < m) {   // (the same for the warp: most fronts have a few rows)
+                    if (g + 4 * i < m) acc += (double)lv[i] * x2[g + 4 * i + r * m];
+                }
         }
         acc += __shfl_xor_sync(0xffffffffu, acc, 8);
         acc += __shfl_xor_sync(0xffffffffu, acc, 16);
         y[r] -= acc;                // lanes < 8: column lane
         x[r] = 0.0;
 #pragma unroll
-        for (int i = 0; i < W; ++i) {
-            const double yi = __shfl_sync(0xffffffffu, y[r], i);
-            if (i < w) x[r] += (double)iv[i] * yi;
-        }
+        for (int i = 0; i < W; ++i)
+            if (i < w) x[r] += (double)iv[i] * __shfl_sync(0xffffffffu, y[r], i);
     }
     if (lane < w) {
 #pragma unroll
