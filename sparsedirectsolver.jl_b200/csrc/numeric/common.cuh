@@ -49,8 +49,10 @@ struct SKid {
     int64_t cb;
     int32_t mc, sri;           // order of its contribution block; its rows' start, relative to the front's
 };
-constexpr int SF_KIDS = 64;    // kids and items that the kernel stages in shared memory (the rest from global)
-constexpr int SF_ITEMS = 768;
+// kids and items that the kernel stages in shared memory for a class of fronts of at most fmax rows (a front with
+// more reads them from global memory): few enough that they cost the small classes no resident CTAs
+__host__ __device__ constexpr int sf_kids(int fmax) { return fmax < 64 ? fmax : 64; }
+__host__ __device__ constexpr int sf_items(int fmax) { return fmax < 96 ? 8 * fmax : 768; }
 constexpr int SF_MAX_KIDS = 65535;   // an item packs p (8 bits), the kid (16) and t (8)
 
 // Rows of a front column that the large-front assembly builds at a time in shared memory (per warp)

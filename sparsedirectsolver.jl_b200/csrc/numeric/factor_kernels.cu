@@ -146,10 +146,11 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int at,
     const int ld = f | 1;
     T* F = reinterpret_cast<T*>(smem_raw);
     size_t off = ((size_t)ld * f * sizeof(T) + 15) & ~size_t(15);
-    SKid* skid = reinterpret_cast<SKid*>(smem_raw + off);    // SF_KIDS
-    uint32_t* sitem = reinterpret_cast<uint32_t*>(skid + SF_KIDS);   // SF_ITEMS
-    uint8_t* ssri = reinterpret_cast<uint8_t*>(sitem + SF_ITEMS);    // SF_ITEMS
-    double* dd = reinterpret_cast<double*>(ssri + SF_ITEMS); // w
+    const int max_kids = sf_kids(A.fmax), max_items = sf_items(A.fmax);
+    SKid* skid = reinterpret_cast<SKid*>(smem_raw + off);
+    uint32_t* sitem = reinterpret_cast<uint32_t*>(skid + max_kids);
+    uint8_t* ssri = reinterpret_cast<uint8_t*>(sitem + max_items);
+    double* dd = reinterpret_cast<double*>(ssri + max_items); // w
     double* ee = dd + w;                                     // w
     double* lvec = ee + w;                                   // 2 f (multipliers)
     int* lp = reinterpret_cast<int*>(lvec + 2 * f);          // w
@@ -170,7 +171,7 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int at,
         before = k > fd.am_begin ? A.maps.am_loc[k - 1] : 0;
         v0 = nz[A.maps.am_src[k]];
     }
-    const bool skids = fd.nkid <= SF_KIDS, sits = fd.nsri <= SF_ITEMS;
+    const bool skids = fd.nkid <= max_kids, sits = fd.nsri <= max_items;
     if (skids && tid < fd.nkid) skid[tid] = A.kids[fd.kid_begin + tid];
     if (sits)
         for (int q = tid; q < fd.nsri; q += nt) {
@@ -206,13 +207,17 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int at,
     int n[SF_U], q0[SF_U], p[SF_U];
     const T* col[SF_U];
     const uint8_t* ri[SF_U];
-    int g = warp, e = A.ep[fd.ep_begin + g], e1 = A.ep[fd.ep_begin + g + 1];
+    // (four warps have the items of two groups of columns each; fronts in registers have eight)
+    const bool two = RPL == 0 && nwarps < 8;
+    const int32_t* ep = A.ep + fd.ep_begin + warp;
+    const int e0 = ep[0], n0 = ep[1] - e0, e1 = two ? ep[4] : 0, nitems = n0 + (two ? ep[5] - e1 : 0);
+    int e = 0;
     auto load = [&]() {
 #pragma unroll
         for (int u = 0; u < SF_U; ++u) {
             n[u] = 0;
-            if (e + u >= e1) continue;
-            const uint32_t it = items[e + u];
+            if (e + u >= nitems) continue;
+            const uint32_t it = items[!two || e + u < n0 ? e0 + e + u : e1 + e + u - n0];
             const SKid kid = kids[(it >> 8) & 0xffffu];
             const int t = it & 0xffu;
             p[u] = it >> 24;
@@ -227,9 +232,9 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int at,
             }
         }
     };
-    load();
+    if (fd.nsri > 0) load();
     __syncthreads();
-    while (true) {
+    while (fd.nsri > 0) {
 #pragma unroll
         for (int u = 0; u < SF_U; ++u) {
             if (n[u] == 0) continue;
@@ -238,18 +243,22 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int at,
                 const int q = q0[u] + lane + 32 * x;
                 if (q < n[u]) F[ri[u][q] + p[u] * ld] += v[u][x];
             }
-            for (int q = q0[u] + lane + 64; q < n[u]; q += 32) F[ri[u][q] + p[u] * ld] += col[u][q];
+            constexpr int SF_T = RPL > 0 ? 1 : 4;   // (fronts in registers have at most 96 rows)
+            for (int q = q0[u] + lane + 64; q < n[u]; q += 32 * SF_T) {
+                T t[SF_T];
+#pragma unroll
+                for (int x = 0; x < SF_T; ++x) t[x] = q + 32 * x < n[u] ? col[u][q + 32 * x] : T(0);
+#pragma unroll
+                for (int x = 0; x < SF_T; ++x)
+                    if (q + 32 * x < n[u]) F[ri[u][q + 32 * x] + p[u] * ld] += t[x];
+            }
             __syncwarp();
         }
         e += SF_U;
-        while (e >= e1 && (g += nwarps) < 8) {
-            e = A.ep[fd.ep_begin + g];
-            e1 = A.ep[fd.ep_begin + g + 1];
-        }
-        if (e >= e1) break;
+        if (e >= nitems) break;
         load();
     }
-    __syncthreads();
+    if (fd.nsri > 0) __syncthreads();   // (not for the leaves)
     if constexpr (RPL > 0) {
         constexpr int CPW = 4 * RPL;
         T a[CPW][RPL];
@@ -386,8 +395,12 @@ __device__ __forceinline__ void small_front(const SmallArgs<T>& A, const int at,
     }
 }
 
+// CTAs of 256 threads that an SM must hold: levels and batches of small fronts need them more than the registers
+// (lap2d 300^2 a pass 2.02 ms, 2.08 with 82 and 85 registers where 64 and 80 fit; 128 systems of lap2d 48^2 "S" 2.20 ms,
+// 2.38 with 80).
+constexpr int small_front_ctas(int rpl) { return rpl == 1 ? 3 : rpl == 3 ? 2 : 4; }
 template <typename T, int STRUCT, int RPL>
-__global__ void __launch_bounds__(256) small_front_kernel(SmallArgs<T> A) {
+__global__ void __launch_bounds__(256, small_front_ctas(RPL)) small_front_kernel(SmallArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
     small_front<T, STRUCT, RPL>(A, blockIdx.x, member, smem_raw);
@@ -403,7 +416,7 @@ __global__ void __launch_bounds__(256) small_front_kernel(SmallArgs<T> A) {
 // src/numeric/subtree.jl:274-316, subtree_ldlt_kernel! src/numeric/ldlt.jl:1133-1228,
 // subtree_lu_kernel! src/numeric/lu.jl:424-493).
 template <typename T, int STRUCT, int RPL>
-__global__ void __launch_bounds__(256) subtree_kernel(SmallArgs<T> A) {
+__global__ void __launch_bounds__(256, small_front_ctas(RPL)) subtree_kernel(SmallArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int member = A.members ? A.members[blockIdx.y] : blockIdx.y;
     const int q0 = A.sub_ptr[blockIdx.x], q1 = A.sub_ptr[blockIdx.x + 1];
@@ -597,7 +610,7 @@ __global__ void __launch_bounds__(32 * WARP_FRONTS_PER_CTA) warp_front_kernel(Sm
 size_t small_front_smem(int fmax, int elsize) {
     size_t ld = fmax | 1;
     size_t b = (ld * fmax * elsize + 15) & ~size_t(15);
-    b += sizeof(SKid) * SF_KIDS + 5 * SF_ITEMS;   // the staged kids, items and rows
+    b += sizeof(SKid) * sf_kids(fmax) + 5 * sf_items(fmax);   // the staged kids, items and rows
     b += sizeof(double) * (2 * fmax + 2 * fmax);  // dd, ee (w <= f), lvec (2 f)
     b += sizeof(int) * (fmax + 16);               // lp, ctl
     b += fmax + 16;                               // kind
@@ -607,11 +620,12 @@ size_t small_front_smem(int fmax, int elsize) {
 template <typename T>
 cudaError_t launch_small(int structure, const SmallArgs<T>& a, int count, int nmembers, int fmax, cudaStream_t st) {
     const bool sub = a.sub_ptr != nullptr;
+    SmallArgs<T> b = a;
+    b.count = count;
+    b.fmax = fmax;
     if (structure == STRUCT_SPD && fmax <= WARP_FRONT_F && !sub &&
         (int64_t)count * nmembers >= WARP_FRONT_MIN_LAUNCH) {   // a warp per front
         const size_t wsmem = (size_t)WARP_FRONTS_PER_CTA * warp_front_bytes<T>();
-        SmallArgs<T> b = a;
-        b.count = count;
         dim3 wgrid((count + WARP_FRONTS_PER_CTA - 1) / WARP_FRONTS_PER_CTA, nmembers);
         warp_front_kernel<T><<<wgrid, 32 * WARP_FRONTS_PER_CTA, wsmem, st>>>(b);
         return cudaGetLastError();
@@ -621,8 +635,8 @@ cudaError_t launch_small(int structure, const SmallArgs<T>& a, int count, int nm
     int threads = regs || fmax > 48 ? 256 : 128;
     dim3 grid(count, nmembers);
     auto go = [&](auto kern, auto sub_kern) {
-        if (sub) sub_kern<<<grid, threads, smem, st>>>(a);
-        else kern<<<grid, threads, smem, st>>>(a);
+        if (sub) sub_kern<<<grid, threads, smem, st>>>(b);
+        else kern<<<grid, threads, smem, st>>>(b);
     };
     switch (structure) {
         case STRUCT_SPD:

@@ -11,6 +11,7 @@ template <typename T>
 struct SmallArgs {
     DeviceMaps maps;
     int32_t count;           // fronts of the launch (the warp-per-front kernel)
+    int32_t fmax;            // the launch's class: no front has more rows
     const SFront* sf;        // the launch's fronts, with their kids, rows and items
     const SKid* kids;
     const uint8_t* sri;
