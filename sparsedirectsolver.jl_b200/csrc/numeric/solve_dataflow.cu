@@ -449,25 +449,32 @@ __device__ __noinline__ void df_narrow_backward(const DataflowArgs<T>& A, int s,
                 if (r < nrhs) x2[lane + 32 * k + r * m] = A.Y[ridx[k] + r * n];
         }
     __syncwarp();
+    // the loops end at the front's last row and column, the same for the warp: most fronts have a few
     double x[NR];
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        double acc = 0.0;
-        if (r < nrhs) {
+    for (int r = 0; r < NR; ++r) x[r] = 0.0;
 #pragma unroll
-            for (int i = 0; i < 8 * K; ++i)
-                if (4 * i < m) {   // (the same for the warp: most fronts have a few rows)
-                    if (g + 4 * i < m) acc += (double)lv[i] * x2[g + 4 * i + r * m];
-                }
+    for (int i = 0; i < 8 * K; ++i)
+        if (4 * i < m) {
+            if (g + 4 * i < m) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+                    if (r < nrhs) x[r] += (double)lv[i] * x2[g + 4 * i + r * m];
+            }
         }
-        acc += __shfl_xor_sync(0xffffffffu, acc, 8);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-        y[r] -= acc;                // lanes < 8: column lane
-        x[r] = 0.0;
 #pragma unroll
-        for (int i = 0; i < W; ++i)
-            if (i < w) x[r] += (double)iv[i] * __shfl_sync(0xffffffffu, y[r], i);
+    for (int r = 0; r < NR; ++r) {
+        x[r] += __shfl_xor_sync(0xffffffffu, x[r], 8);
+        x[r] += __shfl_xor_sync(0xffffffffu, x[r], 16);
+        y[r] -= x[r];               // lanes < 8: column lane
+        x[r] = 0.0;
     }
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+        if (i < w) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) x[r] += (double)iv[i] * __shfl_sync(0xffffffffu, y[r], i);
+        }
     if (lane < w) {
 #pragma unroll
         for (int r = 0; r < NR; ++r)
