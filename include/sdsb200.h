@@ -211,7 +211,8 @@ int sdsb200_set_interrupt(sdsb200_plan* plan, const volatile int32_t* h_flag);
 
 /* CUDA graphs (on by default): sdsb200_factor launches directly in the first call with a set of buffers and
  * options, records its launch program into a graph in the second in a row and replays it from then on; the per-level
- * solve and its refinement steps are recorded in the first call. The one-launch solve needs no graph. The
+ * solve and its refinement steps are recorded in the first call, the one-launch solve in the 32nd in a row with the
+ * same buffers. Inside a caller's stream capture every call launches directly. The
  * user_host_interrupt flag is polled between launch groups in calls that launch directly only. */
 int sdsb200_set_graphs(sdsb200_plan* plan, int32_t on);
 
@@ -272,8 +273,8 @@ int sdsb200_sampled_outer(int64_t n, int64_t nnz, const void* rowptr, const void
  * kernel launch per 32 right-hand sides. On a plan with an FP32 factor it returns the
  * unrefined solution through that factor (FP32 accuracy); refine it with sdsb200_residual and further
  * calls when FP64 accuracy is needed. sdsb200_solve keeps its
- * working vectors in the plan and, with the per-level engine, records its launches into a CUDA graph per set of
- * buffers, which makes the driver allocate device memory on the first call with new buffers.
+ * working vectors in the plan and records its launches into a CUDA graph (sdsb200_set_graphs), which makes the driver
+ * allocate device memory.
  * Callers that may not allocate once set-up is over (a framework whose pool allocator owns all device
  * memory, a real-time loop that forbids allocation after start-up) call this entry point instead:
  * the working vectors Y and xtmp (n * nrhs doubles each) and the update vectors (the plan's ulen

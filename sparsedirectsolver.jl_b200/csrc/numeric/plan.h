@@ -182,7 +182,9 @@ struct Plan {
 
     // CUDA graphs: the static launch program captured once per key (buffers, options) and replayed
     struct CachedGraph {
-        std::vector<uint64_t> key;
+        std::vector<uint64_t> key;      // what the graph was recorded for
+        std::vector<uint64_t> last;     // the last call's key, and how many calls in a row before it had the same
+        int repeats = 0;
         cudaGraphExec_t exec = nullptr;
         int64_t launches = 0;
     };
@@ -200,8 +202,6 @@ struct Plan {
     std::vector<int32_t> fwaits;         // per launch wait lists (ProgLaunch::wait_begin / wait_count)
     cudaEvent_t fstream_fork = nullptr;  // the extra streams start after the caller's prior work
     CachedGraph g_factor, g_solve, g_resid, g_corr;
-    std::vector<uint64_t> factor_key;    // the last factorization's buffers and options: a graph is captured
-                                         // for the second call in a row with the same
 
     bool profile = false;
     ProfAcc prof[PK_COUNT];

@@ -44,3 +44,28 @@ def test_solves_on_two_streams(structure, ir):
     torch.cuda.synchronize()
     for mode, q, x in got:
         assert torch.equal(x, want[mode, q]), (mode, q)
+
+
+def test_repeated_solves_record_a_graph():
+    """The one-launch solve launches directly, then (32 calls in a row with the same buffers) as a graph; other buffers
+    in between, a refinement step and another stream change nothing."""
+    import torch
+
+    from sdsb200.solver import DirectSolver
+
+    A = M.lap3d(12, 12, 12, seed=6)
+    n = A.shape[0]
+    ds = DirectSolver(A, "SPD", reordering_alg="nd", max_nrhs=2, ir_n_steps=1)
+    ds.execute("analysis")
+    assert ds.execute("factorization") == 0
+    b = [torch.from_numpy(np.random.default_rng(q).uniform(-1, 1, (n, 2))).cuda() for q in range(2)]
+    x = [torch.empty_like(v) for v in b]
+    want = [ds.execute("solve", None, v).clone() for v in b]
+    other = torch.cuda.Stream()
+    for q in [0] * 40 + [1] * 5 + [0] * 3 + [1] * 40 + [0, 1] * 4:
+        x[q].fill_(7.0)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(other if q else torch.cuda.current_stream()):
+            ds.execute("solve", x[q], b[q])
+        torch.cuda.synchronize()
+        assert torch.equal(x[q], want[q])
